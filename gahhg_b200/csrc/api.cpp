@@ -372,8 +372,7 @@ gahhg_status gahhg_build(const gahhg_polygon* poly, const gahhg_build_opts* opts
     if (o.semantics == GAHHG_SEMANTICS_EXACT) {
         // the exact index alone: the hierarchy waits until something needs it
         const double t0 = now_seconds();
-        s = grid_alloc_common(g);
-        if (s == GAHHG_OK) s = lattice_build(g);
+        s = lattice_build(g);
         g->stats.lattice_s = now_seconds() - t0;
     } else {
         s = grid_build(g);

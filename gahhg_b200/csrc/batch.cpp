@@ -3,7 +3,7 @@
 //
 // No counterpart in the reference (one polygon per process,
 // source/GPISP.cu:15-70).  Builds run in groups of consecutive polygons
-// (lattice_build_group: every step once for all polygons of a group, so
+// (lattice_build.cu: every step once for all polygons of a group, so
 // launches and host round trips scale with levels, not polygons) on a pool of
 // host threads, each with its own non-blocking stream and look-back scan
 // state; device memory comes from the stream-ordered pool, so no build
@@ -27,7 +27,7 @@ struct gahhg_batch {
     int shape = 0;  // pass-1 launch shape (batch_shape_info)
     std::vector<Polygon*> polys;
     std::vector<Grid*> grids;
-    std::vector<GroupIndex*> groups;  // polygons built together, in order
+    std::vector<LatticeSet*> groups;  // polygons built together, in order
     std::vector<int> swords;  // summary words per polygon (chunk sizing)
     DevArray<uint8_t> views;
     WorkerPool pool;
@@ -55,7 +55,7 @@ struct gahhg_batch {
         g_counters.release();
         views.release();
         for (Grid* g : grids) delete g;
-        for (GroupIndex* G : groups) group_free(G);
+        for (LatticeSet* G : groups) lattice_free(G);
         pool.destroy();
         if (owner_stream) {
             cudaStreamSynchronize(owner_stream);
@@ -83,15 +83,8 @@ gahhg_status build_exact_grid(Polygon* P, int device, cudaStream_t s, void** sca
     g->stream = s;
     g->borrowed = true;
     g->scan_state = *scan;
-    GAHHG_TRY(pool_alloc((void**)&g->d_err, sizeof(DeviceErrors), device, s));
-    GAHHG_TRY(pool_alloc((void**)&g->d_counts, 64 * sizeof(int), device, s));
-    GAHHG_CUDA_TRY(cudaMemsetAsync(g->d_err, 0, sizeof(DeviceErrors), s));
     const gahhg_status st = lattice_build(g);
     *scan = g->scan_state;  // the build may have grown it
-    cudaFreeAsync(g->d_err, s);
-    cudaFreeAsync(g->d_counts, s);
-    g->d_err = nullptr;
-    g->d_counts = nullptr;
     g->classified = true;
     return st;
 }
@@ -99,22 +92,15 @@ gahhg_status build_exact_grid(Polygon* P, int device, cudaStream_t s, void** sca
 // Builds the exact indexes of polys[0 .. count) together on stream s (a
 // worker's context).
 gahhg_status build_group(Polygon* const* polys, int count, int device, cudaStream_t s, void** scan,
-                         const int* top, const int* leaf, GroupIndex** out)
+                         const int* top, const int* leaf, LatticeSet** out)
 {
     Grid g;
     g.device = device;
     g.stream = s;
     g.borrowed = true;
     g.scan_state = *scan;
-    GAHHG_TRY(pool_alloc((void**)&g.d_err, sizeof(DeviceErrors), device, s));
-    GAHHG_TRY(pool_alloc((void**)&g.d_counts, 64 * sizeof(int), device, s));
-    GAHHG_CUDA_TRY(cudaMemsetAsync(g.d_err, 0, sizeof(DeviceErrors), s));
     const gahhg_status st = lattice_build_group(&g, polys, count, top, leaf, out);
     *scan = g.scan_state;  // the build may have grown it
-    cudaFreeAsync(g.d_err, s);
-    cudaFreeAsync(g.d_counts, s);
-    g.d_err = nullptr;
-    g.d_counts = nullptr;
     return st;
 }
 
@@ -141,45 +127,6 @@ void WorkerPool::destroy()
     }
     streams.clear();
     scans.clear();
-}
-
-// Builds grids[i] for every polygon with the pool's workers, one host thread
-// per worker stream.  Returns the first failure (index in *failed).
-gahhg_status WorkerPool::build_all(const std::vector<Polygon*>& polys, const gahhg_build_opts& base,
-                                   const int* top, const int* leaf, std::vector<Grid*>& grids, int* failed)
-{
-    const int count = (int)polys.size();
-    grids.assign(count, nullptr);
-    std::atomic<int> next(0);
-    std::atomic<int> bad(-1);
-    std::mutex mu;
-    std::string first_error;
-    gahhg_status first_status = GAHHG_OK;
-    auto worker = [&](int w) {
-        cudaSetDevice(device);
-        for (;;) {
-            const int i = next.fetch_add(1);
-            if (i >= count || bad.load() >= 0) break;
-            const gahhg_status st = build_exact_grid(polys[i], device, streams[w], &scans[w], base,
-                                                     top ? top[i] : 0, leaf ? leaf[i] : 0, &grids[i]);
-            if (st != GAHHG_OK) {
-                std::lock_guard<std::mutex> lock(mu);
-                if (bad.load() < 0) {
-                    bad.store(i);
-                    first_status = st;
-                    first_error = last_error();
-                }
-            }
-        }
-        cudaStreamSynchronize(streams[w]);
-    };
-    std::vector<std::thread> th;
-    const int nw = std::min((int)streams.size(), std::max(count, 1));
-    for (int w = 0; w < nw; w++) th.emplace_back(worker, w);
-    for (auto& t : th) t.join();
-    *failed = bad.load();
-    if (*failed >= 0) set_error("polygon %d: %s", *failed, first_error.c_str());
-    return *failed >= 0 ? first_status : GAHHG_OK;
 }
 
 }  // namespace gahhg
@@ -292,10 +239,10 @@ gahhg_status gahhg_batch_build(const gahhg_polygon* const* polys, int count, con
     std::vector<uint8_t> host(vb * count);
     long long bytes = 0, edges = 0;
     for (int k = 0; k < ngroups; k++) {
-        bytes += group_bytes(B->groups[k]);
+        bytes += (long long)lattice_bytes(B->groups[k]);
         for (int i = gstart[k]; i < gstart[k + 1]; i++) {
-            group_view_write(B->groups[k], i - gstart[k], host.data() + vb * i);
-            const long long sw = group_summary_words(B->groups[k], i - gstart[k]);
+            lattice_view_write(B->groups[k], i - gstart[k], host.data() + vb * i);
+            const long long sw = lattice_summary_words(B->groups[k], i - gstart[k]);
             B->swords.push_back((int)sw);
             edges += B->polys[i]->pv_num;
             if (sw > 4096) {

@@ -18,7 +18,7 @@
 
 #ifdef __CUDACC__
 #define XHD __host__ __device__ __forceinline__
-#define XHDN __host__ __device__ __noinline__
+#define XHDN static __host__ __device__ __noinline__
 #else
 #define XHD inline
 #define XHDN inline

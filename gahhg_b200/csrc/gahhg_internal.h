@@ -111,6 +111,25 @@ template <class T> struct DevArray {
         stream = s;
         return GAHHG_OK;
     }
+    // Exactly n elements (at least one), contents undefined; for arrays that
+    // do not grow.
+    gahhg_status alloc(size_t n, cudaStream_t s)
+    {
+        if (n == 0) n = 1;
+        if (n <= cap) return GAHHG_OK;
+        release();
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (pool_alloc((void**)&ptr, n * sizeof(T), dev, s) != GAHHG_OK) {
+            cudaGetLastError();
+            ptr = nullptr;
+            set_error("device allocation of %zu bytes failed", n * sizeof(T));
+            return GAHHG_ERR_NOMEM;
+        }
+        cap = n;
+        stream = s;
+        return GAHHG_OK;
+    }
     void release()
     {
         if (ptr) cudaFreeAsync(ptr, stream);
@@ -160,7 +179,7 @@ gahhg_status write_points_sidecar(const char* csv_path, const Points& pts);
 void build_grid0(std::vector<D3>& V, std::vector<Border>& B, std::vector<Cell>& C);
 
 // --------------------------------------------------------------- the grid --
-struct Lattice;  // exact-semantics query index (lattice.cu)
+struct LatticeSet;  // exact-semantics query index (lattice.cuh)
 
 struct Grid {
     const Polygon* poly = nullptr;
@@ -188,7 +207,7 @@ struct Grid {
 
     // query-layout copies (FP64 reference-semantics query)
     void* qlayout = nullptr;
-    Lattice* lattice = nullptr;
+    LatticeSet* lattice = nullptr;
 
     gahhg_stats stats{};
     bool classified = false;
@@ -201,7 +220,6 @@ struct Grid {
     ~Grid();
 };
 
-gahhg_status grid_alloc_common(Grid* g);  // device error word and count buffers
 gahhg_status grid_build(Grid* g);
 gahhg_status grid_classify(Grid* g);
 gahhg_status grid_query_ref(Grid* g, const double* d_lonlat, size_t n, uint8_t* d_labels, cudaStream_t s,
@@ -212,25 +230,21 @@ gahhg_status check_device_errors(Grid* g, const char* phase);
 // exact engine
 gahhg_status lattice_build(Grid* g);
 // Exact indexes of several polygons built together (shared launches); g
-// lends the device, stream, scratch counts, error word and scan state.
-struct GroupIndex;
+// lends the device, stream and scan state.
 gahhg_status lattice_build_group(Grid* g, Polygon* const* polys, int count, const int* top_cells,
-                                 const int* leaf_edges, GroupIndex** out);
-void group_free(GroupIndex* G);
-void group_view_write(const GroupIndex* G, int i, void* dst);
-long long group_summary_words(const GroupIndex* G, int i);
-long long group_bytes(const GroupIndex* G);
+                                 const int* leaf_edges, LatticeSet** out);
+// Polygon i's query view and summary size in a set.
+void lattice_view_write(const LatticeSet* L, int i, void* dst);
+long long lattice_summary_words(const LatticeSet* L, int i);
 gahhg_status lattice_query(Grid* g, const double* d_lonlat, size_t n, uint8_t* d_labels, int precision,
                            cudaStream_t s, uint64_t* d_counters);
 gahhg_status lattice_query_noalloc(Grid* g, const double* d_lonlat, size_t n, uint8_t* d_labels, int precision,
                                    cudaStream_t s);
 long long lattice_noalloc_max_points();
-void lattice_free(Lattice* L);
+void lattice_free(LatticeSet* L);
 // batches (lattice.cu)
 size_t lattice_view_bytes();
 size_t batch_chunk_bytes();
-void lattice_view_write(const Grid* g, void* dst);
-long long lattice_summary_words(const Grid* g);
 // Locate blocks on `device` whose summary copy ran out of time (plain loads instead).
 gahhg_status lattice_staging_fallbacks(int device, unsigned long long* out);
 // Chunks over segments of points stored segment after segment; segment p's
@@ -251,8 +265,9 @@ gahhg_status batch_query_launch(const void* d_views, const void* d_chunks, int n
                                 bool zero_counters = true, int shape = 0);
 int batch_shape_count();
 bool batch_shape_info(int shape, int* points_per_thread, int* blocks_per_sm);
-size_t lattice_bytes(const Lattice* L);
-size_t lattice_device_bytes(const Lattice* L);  // capacity held on the device
+size_t lattice_bytes(const LatticeSet* L);
+size_t lattice_device_bytes(const LatticeSet* L);   // capacity held on the device
+long long lattice_scratch_bytes(const LatticeSet* L);  // held beside the index at the end of its build
 
 // scans (scan.cu)
 size_t scan_state_bytes(size_t n);
@@ -271,8 +286,6 @@ struct WorkerPool {
     std::vector<void*> scans;
     gahhg_status create(int device, int n, int priority = 0);
     void destroy();
-    gahhg_status build_all(const std::vector<Polygon*>& polys, const gahhg_build_opts& base, const int* top,
-                           const int* leaf, std::vector<Grid*>& grids, int* failed);
 };
 gahhg_status build_exact_grid(Polygon* P, int device, cudaStream_t s, void** scan, const gahhg_build_opts& base,
                               int top, int leaf, Grid** out);

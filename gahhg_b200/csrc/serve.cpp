@@ -27,8 +27,8 @@
 // Builds.  Build workers (low-priority streams) take queued builds in order
 // once their estimated footprint fits in the HBM budget, evicting least
 // recently queried unpinned polygons first when asked to.  The estimate
-// (bytes per edge, learnt from finished builds, with a margin) is replaced by
-// the measured footprint when the build finishes.  Queries to a polygon that
+// (index bytes per edge with a margin and the build's own working memory, both
+// learnt from finished builds) is replaced by the measured footprint when the build finishes.  Queries to a polygon that
 // is still building are held and released when it is ready.
 //
 // A polygon's reference count covers its submitted but unfinished queries,
@@ -149,6 +149,7 @@ struct gahhg_server {
     int builds_running = 0;
     long long committed = 0;         // resident bytes + estimates of running builds
     double bytes_per_edge = 1024.0;  // learnt estimate
+    double scratch_per_edge = 0.0;   // learnt likewise, from the first build on
     long long resident_bytes = 0;
     int resident = 0;
 
@@ -260,8 +261,10 @@ struct gahhg_server {
 
     long long estimate(long long edges) const
     {
-        // lattice + polygon copy (24 B vertex + 8 B edge), 256 KB floor, 1.5x margin
-        return std::max<long long>(256 << 10, (long long)(1.5 * bytes_per_edge * (double)edges)) + edges * 32;
+        // lattice (256 KB floor, 1.5x margin) + polygon copy (24 B vertex + 8 B
+        // edge) + what a build holds beside its index while it runs
+        return std::max<long long>(256 << 10, (long long)(1.5 * bytes_per_edge * (double)edges)) + edges * 32 +
+               (long long)(scratch_per_edge * (double)edges);
     }
 
     // ------------------------------------------------------------- queries --
@@ -553,7 +556,7 @@ struct gahhg_server {
             long long bytes = 0;
             std::string msg;
             if (st == GAHHG_OK) {
-                sw = (int)lattice_summary_words(g);
+                sw = (int)lattice_summary_words(g->lattice, 0);
                 if (sw > MAX_SUMMARY_WORDS) {
                     set_error("the index's coarse summary (%d words) exceeds the batch kernel's %d", sw,
                               MAX_SUMMARY_WORDS);
@@ -562,7 +565,7 @@ struct gahhg_server {
             }
             if (st == GAHHG_OK) {
                 std::vector<uint8_t> v(view_bytes);
-                lattice_view_write(g, v.data());
+                lattice_view_write(g->lattice, 0, v.data());
                 cudaStream_t ws = workers.streams[w];
                 const double tv = now_seconds();
                 if (cudaMemcpyAsync(d_views + (size_t)id * view_bytes, v.data(), view_bytes, cudaMemcpyHostToDevice,
@@ -598,6 +601,8 @@ struct gahhg_server {
                     const double bpe = (double)(bytes - (long long)poly->pv_num * 32) / (double)poly->pv_num;
                     // never below the newest observation; decays slowly from larger ones
                     bytes_per_edge = std::max(bpe, 0.9 * bytes_per_edge + 0.1 * bpe);
+                    const double spe = (double)lattice_scratch_bytes(g->lattice) / (double)poly->pv_num;
+                    scratch_per_edge = std::max(spe, 0.9 * scratch_per_edge + 0.1 * spe);
                 }
                 for (Req* r : P.held) pending.push_back(r);
                 if (!P.held.empty()) cv_dispatch.notify_one();
