@@ -348,7 +348,7 @@ gahhg_status gahhg_batch_query_device(gahhg_batch* b, const double* d_lonlat, co
     uint64_t* d_stats = nullptr;
     GAHHG_TRY(pool_alloc(&d_chunks, std::max<size_t>(chunks.size(), 16), b->device, s));
     const long long qcap = std::max<long long>(total, 1);
-    GAHHG_TRY(pool_alloc((void**)&queue, sizeof(uint32_t) * batch_queue_words(qcap), b->device, s));
+    GAHHG_TRY(pool_alloc((void**)&queue, sizeof(uint32_t) * batch_queue_words(qcap, nchunks), b->device, s));
     GAHHG_TRY(pool_alloc((void**)&counters, 8 * sizeof(unsigned int), b->device, s));
     if (!chunks.empty())
         GAHHG_CUDA_TRY(cudaMemcpyAsync(d_chunks, chunks.data(), chunks.size(), cudaMemcpyHostToDevice, s));
@@ -420,7 +420,7 @@ gahhg_status gahhg_batch_query_graph(gahhg_batch* b, const double* d_lonlat, con
                           &b->g_nchunks);
         GAHHG_TRY(b->g_chunks.reserve(std::max<size_t>(chunks.size(), 16), ws, false));
         b->g_qcap = std::max<long long>(total, 1);
-        GAHHG_TRY(b->g_queue.reserve(batch_queue_words(b->g_qcap), ws, false));
+        GAHHG_TRY(b->g_queue.alloc(batch_queue_words(b->g_qcap, b->g_nchunks), ws));
         GAHHG_TRY(b->g_counters.reserve(8, ws, false));
         if (!chunks.empty())
             GAHHG_CUDA_TRY(cudaMemcpyAsync(b->g_chunks.ptr, chunks.data(), chunks.size(), cudaMemcpyHostToDevice, ws));

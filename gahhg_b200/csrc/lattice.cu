@@ -4,7 +4,8 @@
 // level-0 cells (kernel_PISP, source/GPISPAHHG.cu:1422-1504): about ten
 // dependent levels of plane tests per point.  Here the same question is
 // answered from a lattice over longitude/latitude that is indexed directly
-// from the input coordinates // (the lattice itself, and how it is built: lattice_build.cu.)
+// from the input coordinates (the lattice itself, and how it is built:
+// lattice_build.cu).
 //
 // A query reads lon/lat (16 B), computes the top cell with two FP64
 // multiply-adds, follows inner nodes by exact power-of-two scaling, and
@@ -40,102 +41,63 @@ inline int blocks_for(long long n) { return (int)std::max(1LL, (n + TPB - 1) / T
 
 // ------------------------------------------------------------- query ----
 
+// A query point: input longitude and FakeLL latitude (what the canonical XYZ is made from).
 struct PointCtx {
-    double lon, lat;      // input longitude and FakeLL latitude (canonical XYZ)
-    double lon_r, lat_r;  // the same point with lon in [-180, 180], lat in [-90, 90]
-    bool have64;
-    double q[3];
-    __device__ void need64()
-    {
-        if (!have64) {
-            gahhg_canon_vertex_xyz(lon, lat, q);
-            have64 = true;
-        }
-    }
+    double lon, lat;
 };
 
-// exact sign of orient(x, y, z) given a failed FP32 stage; `code` reports a
-// decided label (vertex rule / coincident center) through *early.
-__device__ __forceinline__ int sign_escalate(const double* x, const double* y, const double* z,
-                                             unsigned long long* cnt64, unsigned long long* cntx)
+__device__ __forceinline__ int sign_exactly(const double* x, const double* y, const double* z)
 {
-    int s = exact::orient_fp64(x, y, z);
-    if (cnt64) atomicAdd(cnt64, 1ull);
-    if (s != 0) return s;
-    if (cntx) atomicAdd(cntx, 1ull);
-    return exact::orient_exact(x, y, z);
+    const int s = exact::orient_fp64(x, y, z);
+    return s != 0 ? s : exact::orient_exact(x, y, z);
 }
 
-__device__ uint8_t leaf_label(const QueryView& Q, uint32_t leaf, PointCtx& P, bool fp32, unsigned long long* ctr)
+__device__ __forceinline__ void load_ends(const QueryView& Q, uint32_t e, double* A, double* B)
 {
-    const LeafRec L = Q.leaves[leaf];
-    double LR[3];
-    gahhg_canon_vertex_xyz(L.lon, L.lat, LR);
-    local_frame::Frame f;
-    local_frame::Tests ft;
-    if (fp32) fp32 = fabs(P.lon) <= 540.0 && local_frame::frame_at(P.lon, P.lat, L.lon, L.lat, L.sb, L.cb, f);
-    if (fp32) local_frame::tests_of(f, ft);
-    if (!fp32) P.need64();
-    unsigned long long* c64 = ctr ? ctr + 0 : nullptr;
-    unsigned long long* cx = ctr ? ctr + 1 : nullptr;
-    int par = 0;
-    for (int k = 0; k < L.cnt; k++) {
-        const uint32_t es = __ldg(Q.eids + L.off + k);
-        const int e = (int)(es & 0x7fffffffu);
-        const int s1 = (es >> 31) ? 1 : -1;
-        // the record holds (A, B) when s1 = +1, else (B, A): see local_frame.cuh
-        int s2 = 0, ea = 0, eb = 0;
-        if (fp32) {
-            const float4 r = __ldg(Q.recs + L.off + k);
-            s2 = s1 * local_frame::sign_edge(ft, r.x, r.y, r.z, r.w);
-            const float x1 = s1 > 0 ? r.x : r.z, x2 = s1 > 0 ? r.y : r.w;
-            const float y1 = s1 > 0 ? r.z : r.x, y2 = s1 > 0 ? r.w : r.y;
-            ea = local_frame::sign_end(ft, x1, x2);
-            eb = local_frame::sign_end(ft, y1, y2);
+    const double2* p = Q.ends + 3 * (size_t)e;
+    const double2 u = __ldg(p), v = __ldg(p + 1), w = __ldg(p + 2);
+    A[0] = u.x;
+    A[1] = u.y;
+    A[2] = v.x;
+    B[0] = v.y;
+    B[1] = w.x;
+    B[2] = w.y;
+}
+
+// The complete crossing test of a point in a leaf: FP64 filter, then exact
+// expansions with simulation of simplicity.  A call, not inlined: the few
+// points that need it must not cost the others registers.
+__device__ __noinline__ uint8_t leaf_label_exact(const QueryView* Qp, uint32_t leaf, double lon, double lat)
+{
+    const QueryView& Q = *Qp;
+    const LeafRec* Lp = Q.leaves + leaf;
+    const uint32_t off = Lp->off;
+    const int cnt = Lp->cnt;
+    const uint8_t label = Lp->label;
+    const double LR[3] = {Q.aux[leaf].R[0], Q.aux[leaf].R[1], Q.aux[leaf].R[2]};
+    double q[3];
+    gahhg_canon_vertex_xyz(lon, lat, q);
+    if (exact::same(q, LR)) {  // q is the center: its label, unless it is a vertex
+        for (int k = 0; k < cnt; k++) {
+            double A[3], B[3];
+            load_ends(Q, __ldg(Q.eids + off + k) & 0x7fffffffu, A, B);
+            if (exact::same(q, A) || exact::same(q, B)) return CELL_IN;
         }
-        double A[3], B[3];
-        bool haveAB = false;
-        auto needAB = [&]() {
-            if (!haveAB) {
-                const D3 a = Q.pv[Q.pe[2 * e]], b = Q.pv[Q.pe[2 * e + 1]];
-                A[0] = a.x;
-                A[1] = a.y;
-                A[2] = a.z;
-                B[0] = b.x;
-                B[1] = b.y;
-                B[2] = b.z;
-                haveAB = true;
-            }
-        };
-        if (s2 == 0) {
-            P.need64();
-            needAB();
-            if (exact::same(P.q, A) || exact::same(P.q, B)) return CELL_IN;  // vertex rule
-            if (exact::same(P.q, LR)) return L.label;                       // q is the center
-            s2 = sign_escalate(A, B, P.q, c64, cx);
-        }
-        if (s2 == s1) continue;
-        // s3 = orient(R, q, A); crossing needs s3 == s2
-        int s3 = ea;
-        if (s3 == 0) {
-            P.need64();
-            needAB();
-            if (exact::same(P.q, A) || exact::same(P.q, B)) return CELL_IN;
-            if (exact::same(P.q, LR)) return L.label;
-            s3 = sign_escalate(LR, P.q, A, c64, cx);
-        }
-        if (s3 != s2) continue;
-        int s4 = eb;
-        if (s4 == 0) {
-            P.need64();
-            needAB();
-            if (exact::same(P.q, A) || exact::same(P.q, B)) return CELL_IN;
-            if (exact::same(P.q, LR)) return L.label;
-            s4 = sign_escalate(LR, P.q, B, c64, cx);
-        }
-        if (s4 == -s2) par ^= 1;
+        return label;
     }
-    return (uint8_t)(par ? 3 - L.label : L.label);
+    int par = 0;
+    for (int k = 0; k < cnt; k++) {
+        const uint32_t es = __ldg(Q.eids + off + k);
+        const int s1 = (es >> 31) ? 1 : -1;
+        double A[3], B[3];
+        load_ends(Q, es & 0x7fffffffu, A, B);
+        if (exact::same(q, A) || exact::same(q, B)) return CELL_IN;  // vertex rule
+        const int s2 = sign_exactly(A, B, q);
+        if (s2 == s1) continue;
+        if (sign_exactly(LR, q, A) != s2) continue;  // a crossing needs orient(R, q, A) == s2
+        if (sign_exactly(LR, q, B) == -s2) par ^= 1;
+    }
+    return (uint8_t)(par ? 3 - label : label);
 }
 
 // Programmatic dependent launch (sm_90+): a kernel launched with
@@ -204,39 +166,69 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int li
     return false;
 }
 
+constexpr int SUMMARY_WORDS_MAX = 4096;  // 65,536 coarse cells of 2 bits: 16 KB
 __host__ __device__ __forceinline__ uint32_t summary_bytes(int swords) { return ((uint32_t)swords * 4u + 15u) & ~15u; }
 
 // ------------------------------------------------------ escalation tiers --
 //
-// The crossing tests of the queued points run in tiers, each its own launch
-// over the points the previous tier could not decide, so that no warp carries
-// the registers or waits on the branches of a rarer, costlier tier:
+// The crossing tests run in tiers, so that no warp carries the registers or
+// waits on the branches of a rarer, costlier tier:
 //   tier 1: every sign from the certified FP32 filter in the leaf's local
 //           frame (local_frame.cuh);
 //   tier 2: the canonical FP64 point, the vertex and center rules, and every
 //           sign from the FP64 filter on translated rows (orient_fp64_near);
-//   tier 3: the complete test (FP64 filter, then exact arithmetic with
-//           simulation of simplicity), leaf_label above.
+//   the complete test (leaf_label_exact) for what is left.
 // Every sign a tier returns is exact, so a label does not depend on the tier
 // that produced it.
 constexpr uint8_t LABEL_DEFER = 0xFF;
 
 // Tier 1 runs every edge of the leaf: a decided edge adds its crossing to
 // the parity, an undecided one is noted in `mask` (bit k for record k < 31)
-// and the FP64 tier evaluates only those, starting from the parity of the
-// decided ones (bit 31).  The label is exact either way: the crossing parity
-// is the XOR of independent per-edge tests.  MASK_ALL asks tier 2 for every
-// edge (a record beyond the 31st undecided, or the offset refused).
+// and the FP64 tier evaluates only those, starting from the label that the
+// decided ones give (bit 31: inside).  The label is exact either way: the
+// crossing parity is the XOR of independent per-edge tests.  MASK_ALL asks
+// tier 2 for every edge (a record beyond the 31st undecided, or the offset
+// refused).
 constexpr uint32_t MASK_ALL = 0xFFFFFFFFu;
 
-// Records whose loads tier 1 issues together (one group covers a leaf of
-// the default leaf size): the first group goes out before the offset's
-// arithmetic, so its latency hides behind the sines and cosines.
+// Records beyond the leaf's own two whose loads tier 1 issues together.
 constexpr int T1_GROUP = 4;
-// Blocks per SM of tier 1: five (48 registers, 20 bytes spilled) ran C2 at
-// 21.0-21.1 Gpts/s against 20.5 at four (56 registers); five with groups of
-// two (no spills) 20.5, six with groups of two (40 registers) 20.8.
-constexpr int T1_BLOCKS = 5;
+
+// A leaf as tier 1 reads it: four 16-byte loads of one line in flight.
+struct LeafLoad {
+    double lon, lat;
+    uint32_t off, cnt_label;
+    float sb, cb;
+    float4 r0, r1;
+    __device__ __forceinline__ int cnt() const { return (int)(cnt_label & 0xFFFFu); }
+    __device__ __forceinline__ uint32_t label() const { return (cnt_label >> 16) & 0xFFu; }
+};
+
+template <bool SHARED>
+__device__ __forceinline__ LeafLoad load_leaf(const LeafRec* p)
+{
+    const float4* f = reinterpret_cast<const float4*>(p);
+    float4 a, b;
+    LeafLoad L;
+    if constexpr (SHARED) {
+        a = f[0];
+        b = f[1];
+        L.r0 = f[2];
+        L.r1 = f[3];
+    } else {
+        a = __ldg(f);
+        b = __ldg(f + 1);
+        L.r0 = __ldg(f + 2);
+        L.r1 = __ldg(f + 3);
+    }
+    L.lon = __hiloint2double(__float_as_int(a.y), __float_as_int(a.x));
+    L.lat = __hiloint2double(__float_as_int(a.w), __float_as_int(a.z));
+    L.off = __float_as_uint(b.x);
+    L.cnt_label = __float_as_uint(b.y);
+    L.sb = b.z;
+    L.cb = b.w;
+    return L;
+}
 
 // A record of tier 1: from global memory through the read-only path, or
 // from a copy in shared memory (SHARED).
@@ -247,140 +239,130 @@ __device__ __forceinline__ float4 t1_record(const float4* p)
     else return __ldg(p);
 }
 
-// Tier 1 on the leaf L whose records start at rec (global memory, or the
-// staged copy in shared memory when SHARED).
+// Tier 1 on the leaf L whose third record and on are at rec + 2 ... (global
+// memory, or the staged copy in shared memory when SHARED).
 template <bool SHARED>
-__device__ __forceinline__ uint8_t leaf_label_fp32_at(const float4* rec, const LeafRec& L, const PointCtx& P,
-                                                    uint32_t& mask)
-{
-    const int cnt = L.cnt;
-    float4 r[T1_GROUP];
-#pragma unroll
-    for (int j = 0; j < T1_GROUP; j++) r[j] = j < cnt ? t1_record<SHARED>(rec + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-    local_frame::Frame f;
-    if (!(fabs(P.lon) <= 540.0) || !local_frame::frame_at(P.lon, P.lat, L.lon, L.lat, L.sb, L.cb, f)) {
-        mask = MASK_ALL;
-        return LABEL_DEFER;
-    }
-    local_frame::Tests t;
-    local_frame::tests_of(f, t);
-    int par = 0;
-    uint32_t und = 0;
-    bool all = false;
-    for (int k0 = 0; k0 < cnt; k0 += T1_GROUP) {
-        if (k0 > 0) {
-#pragma unroll
-            for (int j = 0; j < T1_GROUP; j++)
-                r[j] = k0 + j < cnt ? t1_record<SHARED>(rec + k0 + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int j = 0; j < T1_GROUP; j++) {
-            const int k = k0 + j;
-            if (k >= cnt) break;
-            const int x = local_frame::record_crossing(t, r[j].x, r[j].y, r[j].z, r[j].w);
-            if (x > 0) par ^= 1;
-            if (x < 0) {
-                if (k < 31)
-                    und |= 1u << k;
-                else
-                    all = true;
-            }
-        }
-    }
-    if (all) {
-        mask = MASK_ALL;
-        return LABEL_DEFER;
-    }
-    if (und) {
-        mask = und | ((uint32_t)par << 31);
-        return LABEL_DEFER;
-    }
-    return (uint8_t)(par ? 3 - L.label : L.label);
-}
-
-__device__ __forceinline__ uint8_t leaf_label_fp32(const QueryView& Q, const LeafRec& L, const PointCtx& P,
+__device__ __forceinline__ uint8_t leaf_label_fp32(const float4* rec, const LeafLoad& L, const PointCtx& P,
                                                  uint32_t& mask)
 {
-    return leaf_label_fp32_at<false>(Q.recs + L.off, L, P, mask);
+    const int cnt = L.cnt();
+    local_frame::Frame f;
+    mask = MASK_ALL;
+    if (!(fabs(P.lon) <= 540.0) || !local_frame::frame_at(P.lon, P.lat, L.lon, L.lat, L.sb, L.cb, f))
+        return LABEL_DEFER;
+    local_frame::Tests t;
+    local_frame::tests_of(f, t);
+    uint32_t par = L.label() == CELL_IN;
+    uint32_t und = 0;
+    bool all = false;
+    auto take = [&](const float4& r, int k) {
+        const int x = local_frame::record_crossing(t, r.x, r.y, r.z, r.w);
+        if (x > 0) par ^= 1u;
+        if (x < 0) {
+            if (k < 31) und |= 1u << k;
+            else all = true;
+        }
+    };
+    take(L.r0, 0);
+    if (cnt > 1) take(L.r1, 1);
+    for (int k0 = LEAF_INLINE; k0 < cnt; k0 += T1_GROUP) {
+        float4 r[T1_GROUP];
+#pragma unroll
+        for (int j = 0; j < T1_GROUP; j++) r[j] = t1_record<SHARED>(rec + min(k0 + j, cnt - 1));
+#pragma unroll
+        for (int j = 0; j < T1_GROUP; j++)
+            if (k0 + j < cnt) take(r[j], k0 + j);
+    }
+    if (all) return LABEL_DEFER;
+    if (und) {
+        mask = und | (par << 31);
+        return LABEL_DEFER;
+    }
+    return (uint8_t)(1u + par);
 }
 
-// Edges of a leaf whose FP64 endpoints the FP64 tier loads together: their
-// loads (edge id, then three 16-byte loads of the endpoints) are all in flight
-// before the first sign is evaluated, instead of one dependent chain per edge.
-constexpr int T2_GROUP = 4;
+// Records beyond the leaf's own two whose ends the FP64 tier loads together.
+constexpr int T2_GROUP = 2;
 
 // FP64 tier on the leaf's records selected by `mask` (MASK_ALL: every record,
-// parity from 0; else the records of bits 0..30, parity from bit 31).
-__device__ uint8_t leaf_label_fp64(const QueryView& Q, uint32_t leaf, PointCtx& P, uint32_t mask = MASK_ALL)
+// from the leaf's label; else the records of bits 0..30, from the label of
+// bit 31): the leaf's aux line, and edge words and ends beyond its two edges.
+__device__ __forceinline__ uint8_t leaf_label_fp64(const QueryView& Q, uint32_t leaf, const PointCtx& P, uint32_t mask)
 {
-    const LeafRec L = Q.leaves[leaf];
-    // the leaf's loads go out before the point's canonical XYZ is computed
-    const double LR[3] = {__ldg(Q.leafR + 3 * (size_t)leaf), __ldg(Q.leafR + 3 * (size_t)leaf + 1),
-                          __ldg(Q.leafR + 3 * (size_t)leaf + 2)};
-    const bool all = mask == MASK_ALL;
-    const int cnt = L.cnt;
-    int par = all ? 0 : (int)(mask >> 31);
-    uint32_t sel = all ? 0u : (mask & 0x7fffffffu);
-    int kk[T2_GROUP];
-    uint32_t es[T2_GROUP];
-    // the next T2_GROUP records (consecutive ones, or the next set bits of
-    // sel) and their edge words
-    auto next_group = [&](int k0) {
+    const LeafAux* X = Q.aux + leaf;
+    const uint4* xp = reinterpret_cast<const uint4*>(X);
+    const uint4 xa = __ldg(xp), xb = __ldg(xp + 1);
+    double2 e[T2_GROUP][3];
+    static_assert(T2_GROUP == LEAF_INLINE, "the line's edges are the first group");
+    // the line's ends go out with its header, the second edge's when it is asked for
 #pragma unroll
-        for (int j = 0; j < T2_GROUP; j++) {
-            if (all) {
-                kk[j] = k0 + j < cnt ? k0 + j : -1;
-            } else if (sel) {
-                kk[j] = __ffs(sel) - 1;
-                sel &= sel - 1u;
-            } else {
-                kk[j] = -1;
-            }
+    for (int j = 0; j < LEAF_INLINE; j++) {
+        const double2* p = reinterpret_cast<const double2*>(X->ends[j]);
+        if (mask >> j & 1u) {
+            e[j][0] = __ldg(p);
+            e[j][1] = __ldg(p + 1);
+            e[j][2] = __ldg(p + 2);
         }
-#pragma unroll
-        for (int j = 0; j < T2_GROUP; j++) es[j] = kk[j] >= 0 ? __ldg(Q.eids + L.off + kk[j]) : 0u;
-    };
-    // the first group's edge words are in flight while the point's canonical
-    // XYZ is computed
-    next_group(0);
-    P.need64();
-    for (int k0 = 0; kk[0] >= 0; k0 += T2_GROUP) {
-        double2 e[T2_GROUP][3];
+    }
+    const double LR[3] = {__hiloint2double((int)xa.y, (int)xa.x), __hiloint2double((int)xa.w, (int)xa.z),
+                          __hiloint2double((int)xb.y, (int)xb.x)};
+    const uint32_t off = xb.z;
+    uint32_t par = mask >> 31, sel = mask & 0x7fffffffu;
+    int left = 0;  // records after the selected ones (MASK_ALL on a long leaf)
+    if (mask == MASK_ALL) {
+        const int cnt = (int)(xb.w & 0xFFFFu);
+        par = ((xb.w >> 16) & 0xFFu) == CELL_IN;
+        left = max(0, cnt - 31);
+        sel = cnt >= 31 ? 0x7fffffffu : (1u << cnt) - 1u;
+    }
+    double q[3];
+    gahhg_canon_vertex_xyz(P.lon, P.lat, q);
+    // bits of the group's edges and of their signs (orient(A, B, R) > 0)
+    uint32_t group = sel & 3u, signs = xb.w >> 24, k0 = 0;
+    sel &= ~3u;
+    for (;;) {
 #pragma unroll
         for (int j = 0; j < T2_GROUP; j++) {
-            if (kk[j] >= 0) {
-                const double2* p = Q.ends + 3 * (size_t)(es[j] & 0x7fffffffu);
-                e[j][0] = __ldg(p);
-                e[j][1] = __ldg(p + 1);
-                e[j][2] = __ldg(p + 2);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < T2_GROUP; j++) {
-            if (kk[j] < 0) break;
-            const int s1 = (es[j] >> 31) ? 1 : -1;
+            if (!(group >> j & 1u)) continue;
+            const int s1 = (signs >> j & 1u) ? 1 : -1;
             const double A[3] = {e[j][0].x, e[j][0].y, e[j][1].x}, B[3] = {e[j][1].y, e[j][2].x, e[j][2].y};
-            if (exact::same(P.q, A) || exact::same(P.q, B)) return CELL_IN;  // vertex rule
-            if (exact::same(P.q, LR)) return L.label;                       // q is the center
-            // every row is within a cap of the first: translated rows keep the bound small
-            const int s2 = exact::orient_fp64_near(A, B, P.q);
+            if (exact::same(q, A) || exact::same(q, B)) return CELL_IN;  // vertex rule
+            if (exact::same(q, LR)) return LABEL_DEFER;                  // q is the center: the complete test
+            // every row is within a cell of the first: translated rows keep the bound small
+            const int s2 = exact::orient_fp64_near(A, B, q);
             if (s2 == 0) return LABEL_DEFER;
             if (s2 == s1) continue;
-            const int s3 = exact::orient_fp64_near(LR, P.q, A);
+            const int s3 = exact::orient_fp64_near(LR, q, A);
             if (s3 == 0) return LABEL_DEFER;
             if (s3 != s2) continue;
-            const int s4 = exact::orient_fp64_near(LR, P.q, B);
+            const int s4 = exact::orient_fp64_near(LR, q, B);
             if (s4 == 0) return LABEL_DEFER;
-            if (s4 == -s2) par ^= 1;
+            if (s4 == -s2) par ^= 1u;
         }
-        if (all ? k0 + T2_GROUP >= cnt : sel == 0u) break;
-        next_group(k0 + T2_GROUP);
+        if (!sel) {
+            if (left <= 0) break;
+            k0 += 31;
+            const int n = min(left, 31);
+            sel = n == 31 ? 0x7fffffffu : (1u << n) - 1u;
+            left -= n;
+        }
+        group = signs = 0;
+#pragma unroll
+        for (int j = 0; j < T2_GROUP; j++) {
+            if (!sel) break;
+            const uint32_t word = __ldg(Q.eids + off + k0 + __ffs(sel) - 1);
+            sel &= sel - 1u;
+            group |= 1u << j;
+            signs |= (word >> 31) << j;
+            const double2* p = Q.ends + 3 * (size_t)(word & 0x7fffffffu);
+            e[j][0] = __ldg(p);
+            e[j][1] = __ldg(p + 1);
+            e[j][2] = __ldg(p + 2);
+        }
     }
-    return (uint8_t)(par ? 3 - L.label : L.label);
+    return (uint8_t)(1u + par);
 }
 
-// Level-0 cell of a point from its longitude and FakeLL latitude + 90
-// (`laf`); false when the point lies outside the domain.
 struct Loc {
     int ix, iy;
     double fu, fv;
@@ -419,6 +401,30 @@ __device__ __forceinline__ bool domain_locate(const QueryView& Q, double lo, dou
     return true;
 }
 
+// The label of a point whose coarse cell has no edges (or that lies outside
+// the domain), 0 for a mixed cell and for unusual coordinates.  Straight to
+// the coarse cell, without the top cell: a point that rounding puts beyond a
+// coarse border is within the margin of both cells, and beyond the domain's
+// end a partial last cell has the outside's label if it has one.  Pass 1 of a
+// query over the whole sphere is bound by its instructions (62-69 % of the
+// issue slots at 60 to 85 per 32 points, through the top cell, its checks and
+// the tests of the domain's sides), so this is straight-line code of about 15:
+// conversions that saturate at 0, one minimum per axis, the ring of the
+// summary for everything outside.
+__device__ __forceinline__ uint32_t coarse_label(const QueryView& Q, const uint32_t* __restrict__ sum, double lo,
+                                                 double la)
+{
+    double u = fma(lo, Q.cu, Q.cu0);
+    if (Q.cwrap) u += u < 1.0 ? Q.cu360 : 0.0;
+    const double v = fma(la, Q.cv, Q.cv0);
+    const unsigned int x = min(__double2uint_rz(u), (unsigned int)Q.SW - 1u);
+    const unsigned int y = min(__double2uint_rz(v), (unsigned int)Q.SH - 1u);
+    const unsigned int c = y * (unsigned int)Q.SW + x;
+    const uint32_t w = sum[c >> 4] >> ((c & 15u) << 1);
+    const bool ok = (fabs(lo) <= 180.0) & (fabs(la) <= 90.0);
+    return ok ? w & 3u : 0u;
+}
+
 // A cell fraction in [0, 1) as a 32-bit binary fraction, saturating (below 0
 // gives 0, 1 and above all ones).  Its base-4 digits are the children that
 // the recursion f -> 4 f - floor(4 f) (clamped to 0..3) visits: that FP64
@@ -428,15 +434,19 @@ __device__ __forceinline__ bool domain_locate(const QueryView& Q, double lo, dou
 constexpr int MAX_DESCENT = 16;
 __device__ __forceinline__ uint32_t frac_bits(double f) { return __double2uint_rz(f * 4294967296.0); }
 
-__device__ __forceinline__ uint32_t descend(const QueryView& Q, uint32_t w, double fu, double fv)
+__device__ __forceinline__ uint32_t descend_bits(const QueryView& Q, uint32_t w, uint32_t U, uint32_t V)
 {
-    uint32_t U = frac_bits(fu), V = frac_bits(fv);
     while ((w & KIND_MASK) == KIND_INNER) {
         w = __ldg(Q.nodes + (w & INDEX_MASK) + (V >> 30) * FAN + (U >> 30));
         U <<= 2;
         V <<= 2;
     }
     return w;
+}
+
+__device__ __forceinline__ uint32_t descend(const QueryView& Q, uint32_t w, double fu, double fv)
+{
+    return descend_bits(Q, w, frac_bits(fu), frac_bits(fv));
 }
 
 // block-reduced count of inside labels (statistics only)
@@ -453,157 +463,170 @@ __device__ __forceinline__ void count_inside(int v, unsigned long long* dst)
 
 constexpr int LOC_UNROLL = 4;
 constexpr uint8_t LABEL_PENDING = 0;
-// Leaf word of a queued point that pass 1 did not locate (a pure node
-// without a label, which is never queued).
+// Leaf word of a queued point that was not located (its coordinates are
+// unusual, or it is out of a pure node).
 constexpr uint32_t LEAF_UNKNOWN = KIND_PURE;
 
-// Pass 1: every point whose cell has no edges gets its label; the others are
-// queued (index within this chunk) for pass 2.  Lean on registers and
-// instructions so that many warps keep loads in flight; lon/lat and labels
-// stream with an evict-first policy so the node table stays in L2.  The index
-// arithmetic need not match the canonical conversion bit for bit: every cap
-// carries a margin far above its rounding (see LOC_MARGIN).
-// Pass 1 over points [first, first + count) of one polygon, in tiles of
-// TPB * LOC_UNROLL points (tiles tile0, tile0 + tstride, ...): every point
-// whose cell has no edges gets its label; the others are queued (their index
-// `first + local`) for pass 2.  Lean on registers and instructions so that
-// many warps keep loads in flight; lon/lat and labels stream with an
-// evict-first policy so the node table stays in L2.  The index arithmetic
-// need not match the canonical conversion bit for bit: every cap carries a
-// margin far above its rounding (see LOC_MARGIN).
-template <bool STATS, bool LOCKSTEP = false, int UNROLL = LOC_UNROLL>
-__device__ __forceinline__ void locate_range(const QueryView& Q, const uint32_t* s_sum,
-                                             const double2* __restrict__ ll, uint8_t* __restrict__ out,
-                                             uint32_t* __restrict__ queue, uint32_t* __restrict__ leafq,
-                                             unsigned int* __restrict__ qcount, long long first, int count,
-                                             int tile0, int tstride, int& inside)
+__device__ __forceinline__ bool usual(double lo, double laf) { return laf >= 0.0 && laf <= 180.0 && fabs(lo) <= 540.0; }
+
+// The point's context, and its node word: `known` when it was located (any
+// leaf the locate arithmetic finds serves: every cell's rectangle holds its
+// points with a margin above that arithmetic's rounding), else a descent from
+// the top, for unusual input from the canonical XYZ itself.
+__device__ __forceinline__ uint32_t point_leaf(const QueryView& Q, double2 p, PointCtx& P,
+                                              uint32_t known = LEAF_UNKNOWN)
 {
+    P.lat = gahhg_canon_query_lat(p.y);
+    P.lon = p.x;
+    if (known != LEAF_UNKNOWN) return known;
+    double lo = P.lon, la = P.lat;
+    if (!(fabs(lo) <= 540.0 && fabs(la) <= 90.0)) {
+        double q[3];
+        gahhg_canon_vertex_xyz(P.lon, P.lat, q);
+        la = asin(fmin(1.0, fmax(-1.0, q[1]))) / RAD;
+        lo = atan2(q[0], q[2]) / RAD;
+    }
+    Loc L;
+    const bool in = domain_locate(Q, lo, la + 90.0, L);
+    return in ? descend(Q, __ldg(Q.nodes + (size_t)L.iy * Q.W + L.ix), L.fu, L.fv) : Q.outside;
+}
+
+// ------------------------------------------------------- pass 1 (locate) --
+
+// The pass-1 queue is filled in parts, block b into part b % parts, each with
+// its own counter on a line of its own: an atomic that returns a value takes
+// about 1.3 ns on one address, one after the other, so a single counter held
+// queries whose points in leaves are spread over all tiles to 0.75 G tiles/s
+// (1e8 uniform points on the 1,100-edge polygon, a few in every tile: 1075 us
+// of locate, of which the counter was the most).  A part has room for all
+// points of its blocks.
+constexpr int QUEUE_PARTS = 64;
+constexpr int COUNTER_STRIDE = 32;  // words between counters
+
+// Pass 1 over one polygon.  A warp's points in mixed blocks wait in shared
+// memory and descend 32 at a time: most tiles of a query over the whole sphere
+// have a few of them, and descending where they stood cost a tile up to four
+// chains of node loads one after the other, on a few lanes each.
+constexpr int LOC_QUEUE = 32 + 32 * LOC_UNROLL;
+// 32 registers, 64 warps per SM: the pass is bound by the latency of its
+// streams (17 B a point; 255 us for 1e8 points at the copy rate), and warps
+// hide it better than loads in flight per warp do: six blocks 354 us where
+// eight take 296 (1e8 uniform points on the 1.1M-edge polygon).
+constexpr int LOC_BLOCKS = 8;
+
+// A warp's tile is LOC_UNROLL / 2 rows of 64 points, a lane's two of a row
+// side by side, through 16-byte loads.  (1e8 uniform points on the 1.1M-edge
+// polygon: 295 us of locate this way, 320-330 with 32-byte loads or evict-first
+// hints on them; on the 1,100-edge polygon 286, and 323 with evict-first.)
+template <bool STATS>
+__device__ __forceinline__ void locate_points(const QueryView& Q, const uint32_t* __restrict__ sum,
+                                              const double2* __restrict__ ll, int n, uint8_t* __restrict__ out,
+                                              uint32_t* __restrict__ queue, uint32_t* __restrict__ leafq,
+                                              unsigned int* __restrict__ qcount, uint32_t qbase, uint32_t* mixed,
+                                              int& inside)
+{
+    constexpr int ROWS = LOC_UNROLL / 2;
+    static_assert(LOC_UNROLL == 4, "rows of two points per lane, four labels in a word");
     const int lane = threadIdx.x & 31;
-    const int cs = Q.cshift, cw = Q.CW;
-    constexpr int TILE = TPB * UNROLL;
-    for (int base = tile0 * TILE; base < count; base += tstride * TILE) {
-        const bool full = base + TILE <= count;
-        double2 p[UNROLL];
+    int nm = 0;  // points in `mixed`, the same in every lane
+    constexpr int TILE = TPB * LOC_UNROLL;
+    for (int base = blockIdx.x * TILE;; base += gridDim.x * TILE) {
+        const bool last = base >= n;
+        if (!last) {
+            const int i = base + (threadIdx.x & ~31) * LOC_UNROLL + 2 * lane;  // row r: points i + 64 r, i + 64 r + 1
+            uint32_t lab = 0;   // labels, a byte each; 0: mixed (or LABEL_PENDING, the same)
+            uint32_t skip = 0;  // beyond the last point
+            if (base + TILE <= n) {
+                double2 a[ROWS], b[ROWS];
 #pragma unroll
-        for (int k = 0; k < UNROLL; k++) {
-            const int i = base + k * TPB + threadIdx.x;
-            p[k] = (full || i < count) ? __ldcs(ll + first + i) : make_double2(0.0, 0.0);
-        }
-        uint8_t lab[UNROLL];
-        bool push[UNROLL];
-        bool any = false;
-        // LOCKSTEP: the node words of all points are loaded first and the
-        // descents advance one level per round, so a thread keeps one
-        // independent load per point in flight (points that mostly need the
-        // node table, as around small polygons, are bound by its latency)
-        uint32_t w[UNROLL];
-        uint32_t fu[UNROLL], fv[UNROLL];  // cell fractions as binary fractions (frac_bits)
+                for (int r = 0; r < ROWS; r++) {
+                    a[r] = __ldg(ll + i + 64 * r);
+                    b[r] = __ldg(ll + i + 64 * r + 1);
+                }
 #pragma unroll
-        for (int k = 0; k < UNROLL; k++) {
-            const int i = base + k * TPB + threadIdx.x;
-            const double lo = p[k].x;
-            const double laf = p[k].y + 90.0;  // the reference's FakeLL latitude + 90
-            lab[k] = LABEL_PENDING;
-            push[k] = false;
-            w[k] = KIND_PURE;
-            if (full || i < count) {
-                if (laf >= 0.0 && laf <= 180.0 && fabs(lo) <= 540.0) {
-                    Loc L;
-                    if (!domain_locate(Q, lo, laf, L)) {
-                        lab[k] = (uint8_t)Q.outside;
+                for (int r = 0; r < ROWS; r++) {
+                    const uint32_t l = coarse_label(Q, sum, a[r].x, a[r].y) | coarse_label(Q, sum, b[r].x, b[r].y) << 8;
+                    lab |= l << (16 * r);
+                    out[i + 64 * r] = (uint8_t)l;
+                    out[i + 64 * r + 1] = (uint8_t)(l >> 8);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < LOC_UNROLL; k++) {
+                    const int j = i + 64 * (k >> 1) + (k & 1);
+                    if (j < n) {
+                        const double2 q = __ldg(ll + j);
+                        const uint32_t l = coarse_label(Q, sum, q.x, q.y);
+                        lab |= l << (8 * k);
+                        out[j] = (uint8_t)l;
                     } else {
-                        const int c = (L.iy >> cs) * cw + (L.ix >> cs);
-                        const uint32_t code = (s_sum[c >> 4] >> ((c & 15) << 1)) & 3u;
-                        if (code < 2u) {
-                            lab[k] = (uint8_t)(code + 1u);  // coarse cell without edges: most points end here
-                        } else if (LOCKSTEP) {
-                            w[k] = __ldg(Q.nodes + (size_t)L.iy * Q.W + L.ix);
-                            fu[k] = frac_bits(L.fu);
-                            fv[k] = frac_bits(L.fv);
-                        } else {
-                            const uint32_t d = descend(Q, __ldg(Q.nodes + (size_t)L.iy * Q.W + L.ix), L.fu, L.fv);
-                            if ((d & KIND_MASK) == KIND_PURE)
-                                lab[k] = (uint8_t)(d & 3u);
-                            else
-                                push[k] = true;
-                            w[k] = d;
-                        }
-                    }
-                } else {
-                    // unusual coordinates go to pass 2; non-finite input stays undefined
-                    push[k] = isfinite(lo) && isfinite(laf);
-                }
-            }
-            if (!LOCKSTEP) any |= push[k];
-        }
-        if (LOCKSTEP) {
-            bool inner = true;
-            while (inner) {
-                inner = false;
-#pragma unroll
-                for (int k = 0; k < UNROLL; k++)
-                    if ((w[k] & KIND_MASK) == KIND_INNER) {
-                        w[k] = __ldg(Q.nodes + (w[k] & INDEX_MASK) + (fv[k] >> 30) * FAN + (fu[k] >> 30));
-                        fu[k] <<= 2;
-                        fv[k] <<= 2;
-                        inner = true;
-                    }
-            }
-#pragma unroll
-            for (int k = 0; k < UNROLL; k++) {
-                if (lab[k] == LABEL_PENDING && !push[k]) {
-                    const int i = base + k * TPB + threadIdx.x;
-                    if (full || i < count) {
-                        if ((w[k] & KIND_MASK) == KIND_PURE) {
-                            if (w[k] != KIND_PURE) lab[k] = (uint8_t)(w[k] & 3u);  // KIND_PURE alone: no node read
-                        } else {
-                            push[k] = true;
-                        }
+                        skip |= 1u << (8 * k);
                     }
                 }
-                any |= push[k];
             }
-        }
-        if (__any_sync(0xffffffffu, any)) {
-            // one atomic on the queue counter per warp and tile: every thread of
-            // the grid pushes through this one counter, and where most points
-            // are queued (points near the edges) the counter itself limits pass 1
-            // (one per block and tile, which takes block-wide barriers, made
-            // uniform points 14 % slower and near-edge points 2 % faster)
-            unsigned int total = 0;
+            if (STATS) inside += __popc(lab & 0x02020202u);
+            const uint32_t mixed4 = ~(lab | (lab >> 1) | skip) & 0x01010101u;  // a bit per mixed point
+            if (__any_sync(0xffffffffu, mixed4 != 0)) {
 #pragma unroll
-            for (int k = 0; k < UNROLL; k++) total += __popc(__ballot_sync(0xffffffffu, push[k]));
-            unsigned int pos = 0;
-            if (lane == 0) pos = atomicAdd(qcount, total);
-            pos = __shfl_sync(0xffffffffu, pos, 0);
-#pragma unroll
-            for (int k = 0; k < UNROLL; k++) {
-                const unsigned int mk = __ballot_sync(0xffffffffu, push[k]);
-                if (push[k]) {
-                    const unsigned int at = pos + __popc(mk & ((1u << lane) - 1u));
-                    queue[at] = (uint32_t)(first + base + k * TPB + threadIdx.x);
-                    // w is the leaf word, or KIND_PURE (LEAF_UNKNOWN) for an unlocated point
-                    if (leafq) leafq[at] = w[k];
+                for (int k = 0; k < LOC_UNROLL; k++) {
+                    const bool push = (mixed4 >> (8 * k)) & 1u;
+                    const unsigned int mk = __ballot_sync(0xffffffffu, push);
+                    if (push) mixed[nm + __popc(mk & ((1u << lane) - 1u))] = (uint32_t)(i + 64 * (k >> 1) + (k & 1));
+                    nm += __popc(mk);
                 }
-                pos += __popc(mk);
             }
+            __syncwarp();  // (orders the labels before those that B writes, too)
         }
-#pragma unroll
-        for (int k = 0; k < UNROLL; k++) {
-            const int i = base + k * TPB + threadIdx.x;
-            if (full || i < count) __stcs(out + first + i, lab[k]);
-            if (STATS) inside += lab[k] == CELL_IN;
+        while (nm >= 32 || (last && nm > 0)) {
+            const int m = min(nm, 32);
+            nm -= m;
+            uint32_t i = 0, w = KIND_PURE | 1u;
+            if (lane < m) {
+                i = mixed[nm + lane];
+                const double2 p = __ldg(ll + i);
+                const double laf = p.y + 90.0;
+                Loc L;
+                if (usual(p.x, laf))
+                    w = domain_locate(Q, p.x, laf, L)
+                            ? descend(Q, __ldg(Q.nodes + (size_t)L.iy * Q.W + L.ix), L.fu, L.fv)
+                            : Q.outside;
+                else if (isfinite(p.x) && isfinite(p.y))
+                    w = LEAF_UNKNOWN;  // unusual coordinates: tier 1 locates them
+                else
+                    w = KIND_PURE | 4u;  // non-finite input stays undefined (LABEL_PENDING)
+                if ((w & KIND_MASK) == KIND_PURE && (w & 3u)) {
+                    out[i] = (uint8_t)(w & 3u);
+                    if (STATS) inside += (w & 3u) == CELL_IN;
+                }
+            }
+            const bool leaf = (w & KIND_MASK) != KIND_PURE || w == LEAF_UNKNOWN;
+            const unsigned int mk = __ballot_sync(0xffffffffu, leaf);
+            if (mk) {
+                unsigned int pos = 0;
+                if (lane == 0) pos = atomicAdd(qcount, (unsigned int)__popc(mk));
+                pos = __shfl_sync(0xffffffffu, pos, 0) + qbase + __popc(mk & ((1u << lane) - 1u));
+                if (leaf) {
+                    queue[pos] = i;
+                    leafq[pos] = w;
+                }
+            }
+            __syncwarp();
         }
+        if (last) break;
     }
 }
 
 template <bool STATS>
-__global__ void __launch_bounds__(TPB) k_locate(const double2* __restrict__ ll, int n, uint8_t* __restrict__ out,
-                                               QueryView Q, uint32_t* __restrict__ queue,
-                                               uint32_t* __restrict__ leafq, unsigned int* __restrict__ qcount,
-                                               unsigned long long* ctr, int poll_limit)
+__global__ void __launch_bounds__(TPB, LOC_BLOCKS) k_locate(const double2* __restrict__ ll, int n,
+                                                           uint8_t* __restrict__ out,
+                                                           const __grid_constant__ QueryView Q,
+                                                           uint32_t* __restrict__ queue, uint32_t* __restrict__ leafq,
+                                                           unsigned int* __restrict__ qcount, int parts,
+                                                           unsigned int part_cap, unsigned long long* ctr,
+                                                           int poll_limit)
 {
     extern __shared__ __align__(16) uint32_t s_sum[];
+    __shared__ uint32_t s_mixed[TPB / 32][LOC_QUEUE];
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ int s_late;
     if (threadIdx.x == 0) {
@@ -614,75 +637,254 @@ __global__ void __launch_bounds__(TPB) k_locate(const double2* __restrict__ ll, 
     __syncthreads();
     if (!mbar_wait(&s_bar, 0, poll_limit)) s_late = 1;
     __syncthreads();
-    const bool late = s_late != 0;
-    // after a wait that ran out the block reads the summary from global
-    // memory and never touches s_sum, which the pending copy still targets
-    if (late && threadIdx.x == 0) atomicAdd(&g_tma_timeouts, 1u);
+    const unsigned int part = blockIdx.x % (unsigned int)parts;
+    uint32_t* mixed = s_mixed[threadIdx.x >> 5];
     int inside = 0;
-    locate_range<STATS>(Q, late ? Q.summary : s_sum, ll, out, queue, leafq, qcount, 0, n, blockIdx.x, gridDim.x,
-                        inside);
-    if (late) mbar_wait(&s_bar, 0);  // the copy in flight ends before the block does (bounded)
+    if (s_late == 0) {
+        locate_points<STATS>(Q, s_sum, ll, n, out, queue, leafq, qcount + part * COUNTER_STRIDE, part * part_cap, mixed,
+                             inside);
+    } else {
+        // after a wait that ran out the block reads the summary from global
+        // memory and never touches s_sum, which the pending copy still targets
+        if (threadIdx.x == 0) atomicAdd(&g_tma_timeouts, 1u);
+        locate_points<STATS>(Q, Q.summary, ll, n, out, queue, leafq, qcount + part * COUNTER_STRIDE, part * part_cap,
+                             mixed, inside);
+        mbar_wait(&s_bar, 0);  // the copy in flight ends before the block does (bounded)
+    }
     allow_dependents();
     if (STATS && ctr) count_inside(inside, ctr + 3);
 }
 
-// The leaf of a queued point (the point context filled in), or its label
-// with KIND_PURE when its cell has no edges.
-// The point's context, and its node word: `known` when pass 1 located the
-// point (any leaf it finds serves: every leaf cap holds its points with a
-// margin above the locate arithmetic's rounding), else a descent from the top.
-__device__ __forceinline__ uint32_t point_leaf(const QueryView& Q, double2 p, PointCtx& P,
-                                              uint32_t known = LEAF_UNKNOWN)
+// ----------------------------------------------------- a query, one launch --
+//
+// Queries that cannot fill the chip for long (INLINE_MAX) take a point from
+// its coordinates to its label in one launch, without scratch and without
+// counters to clear: a warp works on its own tiles of points, with queues of
+// its own in shared memory between the steps, so a step runs when 32 points
+// need it, on a full warp, and no step waits for other warps:
+//   A  the tile's points: level-0 cell, then the coarse summary; a block of
+//      cells without edges gives the label, the others are queued with their
+//      cell and their place in it;
+//   B  32 points in mixed blocks: node table, down to a pure node (the
+//      label) or a leaf (queued);
+//   C  32 points in leaves: tier 1; a label, or queued for tier 2 with the
+//      mask of undecided edges (FP64-filter queries: queued as they are);
+//   D  32 points: tier 2, then the complete test for what is left.
+// Every step's loads are independent across the lanes.  Large queries run the
+// passes as launches of their own (k_locate, k_leaf_t1, k_leaf_t2), where each
+// has the registers it needs at the warps it can use; a small one paid for
+// four launches, an allocation and a memset there (18 us a call).  Four blocks
+// per SM (64 registers, 100 bytes spilled in tier 2) against two without:
+// 1,048,576 points near the 1.1M-edge polygon's edges 102 us and 114, uniform
+// ones 14 and 15.
+template <int U>
+struct WarpSpace {
+    static constexpr int TILE = 32 * U;
+    uint32_t p1[32 + TILE], c1[32 + TILE], u1[32 + TILE], v1[32 + TILE];  // B: points, cells, places in them
+    uint32_t p2[64], w2[64];                                              // C: points, leaf words
+    uint32_t p3[64], w3[64], m3[64];                                      // D: points, leaf words, masks
+};
+
+struct QueryCounts {
+    int inside = 0, boundary = 0, fp64 = 0, exact = 0;
+};
+
+template <bool FP32, bool STATS, int U>
+__device__ __forceinline__ void query_tiles(const QueryView& Q, const uint32_t* s_sum, int first, int stride, int n,
+                                            const double2* __restrict__ ll, uint8_t* __restrict__ out,
+                                            WarpSpace<U>& s, QueryCounts& c)
 {
-    P.lat = gahhg_canon_query_lat(p.y);
-    P.lon = p.x;
-    P.have64 = false;
-    double lo = P.lon, la = P.lat;
-    if (!(fabs(lo) <= 540.0 && fabs(la) <= 90.0)) {
-        // unusual input: locate from the canonical XYZ itself
-        P.need64();
-        la = asin(fmin(1.0, fmax(-1.0, P.q[1]))) / RAD;
-        lo = atan2(P.q[0], P.q[2]) / RAD;
+    constexpr int TILE = WarpSpace<U>::TILE;
+    const int lane = threadIdx.x & 31;
+    const unsigned int below = (1u << lane) - 1u;
+    int n1 = 0, n2 = 0, n3 = 0;  // queued points, the same in every lane
+    for (int base = first;; base += stride) {
+        const bool last = base >= n;
+        if (!last) {  // A
+            double2 pt[U];
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                const int i = base + k * 32 + lane;
+                pt[k] = i < n ? __ldg(ll + i) : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                const int i = base + k * 32 + lane;
+                const bool have = i < n;
+                uint8_t lab = (uint8_t)coarse_label(Q, s_sum, pt[k].x, pt[k].y);
+                bool push = false;
+                uint32_t cell = 0xFFFFFFFFu, fu = 0, fv = 0;  // unusual coordinates: not located
+                if (lab == LABEL_PENDING) {
+                    Loc L;
+                    if (usual(pt[k].x, pt[k].y + 90.0)) {
+                        push = domain_locate(Q, pt[k].x, pt[k].y + 90.0, L);
+                        if (push) {
+                            cell = (uint32_t)(L.iy * Q.W + L.ix);
+                            fu = frac_bits(L.fu);
+                            fv = frac_bits(L.fv);
+                        } else {
+                            lab = (uint8_t)Q.outside;
+                        }
+                    } else {
+                        push = isfinite(pt[k].x) && isfinite(pt[k].y);  // non-finite input stays undefined
+                    }
+                }
+                push = push && have;
+                if (have && !push) {
+                    out[i] = lab;
+                    if (STATS) c.inside += lab == CELL_IN;
+                }
+                const unsigned int mk = __ballot_sync(0xffffffffu, push);
+                if (push) {
+                    const int at = n1 + __popc(mk & below);
+                    s.p1[at] = (uint32_t)i;
+                    s.c1[at] = cell;
+                    s.u1[at] = fu;
+                    s.v1[at] = fv;
+                }
+                n1 += __popc(mk);
+            }
+            __syncwarp();
+        }
+        for (;;) {
+            const bool doB = n1 >= 32 || (last && n1 > 0);
+            if (doB) {
+                const int m = min(n1, 32);
+                n1 -= m;
+                uint32_t i = 0, w = KIND_PURE | 1u;
+                if (lane < m) {
+                    i = s.p1[n1 + lane];
+                    const uint32_t cell = s.c1[n1 + lane];
+                    w = LEAF_UNKNOWN;
+                    if (cell != 0xFFFFFFFFu) {
+                        w = descend_bits(Q, __ldg(Q.nodes + cell), s.u1[n1 + lane], s.v1[n1 + lane]);
+                        if ((w & KIND_MASK) == KIND_PURE) {
+                            const uint8_t lab = (uint8_t)(w & 3u);
+                            out[i] = lab;
+                            if (STATS) c.inside += lab == CELL_IN;
+                        }
+                    }
+                }
+                const bool leaf = (w & KIND_MASK) == KIND_LEAF || w == LEAF_UNKNOWN;
+                const unsigned int mk = __ballot_sync(0xffffffffu, leaf);
+                if (leaf) {
+                    const int at = n2 + __popc(mk & below);
+                    s.p2[at] = i;
+                    s.w2[at] = w;
+                }
+                n2 += __popc(mk);
+                __syncwarp();
+            }
+            const bool doC = n2 >= 32 || (last && n1 == 0 && n2 > 0);
+            if (doC) {
+                const int m = min(n2, 32);
+                n2 -= m;
+                bool defer = false;
+                uint32_t i = 0, w = 0, mask = MASK_ALL;
+                if (lane < m) {
+                    i = s.p2[n2 + lane];
+                    w = s.w2[n2 + lane];
+                    if (FP32) {
+                        LeafLoad L;
+                        const bool known = (w & KIND_MASK) == KIND_LEAF;
+                        if (known) L = load_leaf<false>(Q.leaves + (w & INDEX_MASK));
+                        PointCtx P;
+                        w = point_leaf(Q, __ldg(ll + i), P, w);
+                        uint8_t lab = (uint8_t)(w & 3u);
+                        if ((w & KIND_MASK) != KIND_PURE) {
+                            if (STATS) c.boundary++;
+                            if (!known) L = load_leaf<false>(Q.leaves + (w & INDEX_MASK));
+                            lab = leaf_label_fp32<false>(Q.recs + L.off, L, P, mask);
+                            defer = lab == LABEL_DEFER;
+                            if (STATS) c.fp64 += defer;
+                        }
+                        if (!defer) {
+                            out[i] = lab;
+                            if (STATS) c.inside += lab == CELL_IN;
+                        }
+                    } else {
+                        defer = true;
+                    }
+                }
+                const unsigned int mk = __ballot_sync(0xffffffffu, defer);
+                if (defer) {
+                    const int at = n3 + __popc(mk & below);
+                    s.p3[at] = i;
+                    s.w3[at] = w;
+                    if (FP32) s.m3[at] = mask;
+                }
+                n3 += __popc(mk);
+                __syncwarp();
+            }
+            const bool doD = n3 >= 32 || (last && n1 == 0 && n2 == 0 && n3 > 0);
+            if (doD) {
+                const int m = min(n3, 32);
+                n3 -= m;
+                if (lane < m) {
+                    const uint32_t i = s.p3[n3 + lane];
+                    PointCtx P;
+                    const uint32_t w = point_leaf(Q, __ldg(ll + i), P, s.w3[n3 + lane]);
+                    uint8_t lab = (uint8_t)(w & 3u);
+                    if ((w & KIND_MASK) != KIND_PURE) {
+                        if (STATS && !FP32) c.boundary++;
+                        lab = leaf_label_fp64(Q, w & INDEX_MASK, P, FP32 ? s.m3[n3 + lane] : MASK_ALL);
+                        if (lab == LABEL_DEFER) {
+                            if (STATS) c.exact++;
+                            lab = leaf_label_exact(&Q, w & INDEX_MASK, P.lon, P.lat);
+                        }
+                    }
+                    out[i] = lab;
+                    if (STATS) c.inside += lab == CELL_IN;
+                }
+                __syncwarp();
+            }
+            if (!(doB || doC || doD)) break;
+        }
+        if (last) break;
     }
-    Loc L;
-    double lr = lo;
-    if (lr > 180.0) lr -= 360.0;
-    if (lr > 180.0) lr -= 360.0;
-    if (lr < -180.0) lr += 360.0;
-    if (lr < -180.0) lr += 360.0;
-    P.lon_r = lr;
-    P.lat_r = la;
-    if (known != LEAF_UNKNOWN) return known;
-    const bool in = domain_locate(Q, lo, la + 90.0, L);
-    return in ? descend(Q, __ldg(Q.nodes + (size_t)L.iy * Q.W + L.ix), L.fu, L.fv) : Q.outside;
 }
 
-// One point through the untiered path (escalations inline, counted per test).
-template <bool FP32>
-__device__ __forceinline__ uint8_t leaf_point(const QueryView& Q, double2 p, unsigned long long* ctr)
+__device__ __forceinline__ void count_stats(unsigned long long* ctr, const QueryCounts& c)
 {
-    PointCtx P;
-    const uint32_t w = point_leaf(Q, p, P);
-    if ((w & KIND_MASK) == KIND_PURE) return (uint8_t)(w & 3u);
-    if (ctr) atomicAdd(ctr + 2, 1ull);
-    return leaf_label(Q, w & INDEX_MASK, P, FP32, ctr);
+    count_inside(c.inside, ctr + 3);
+    count_inside(c.boundary, ctr + 2);
+    count_inside(c.fp64, ctr + 0);
+    count_inside(c.exact, ctr + 1);
 }
 
-// Pass 2: exact crossing tests for the queued points.
-template <bool FP32>
-__global__ void __launch_bounds__(TPB) k_leaf(const double2* __restrict__ ll, uint8_t* __restrict__ out,
-                                             QueryView Q, const uint32_t* __restrict__ queue,
-                                             const unsigned int* __restrict__ qcount, unsigned long long* ctr)
+// STAGE: the coarse summary is copied to shared memory first (a query of a
+// few thousand points reads the words it needs instead).
+template <bool FP32, bool STATS, int U, bool STAGE>
+__global__ void __launch_bounds__(TPB, U == 1 ? 2 : 4) k_query(const double2* __restrict__ ll, int n, uint8_t* __restrict__ out,
+                                                 const __grid_constant__ QueryView Q, unsigned long long* ctr,
+                                                 int poll_limit)
 {
-    const unsigned int m = *qcount;
-    int inside = 0;
-    for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
-        const uint32_t i = queue[t];
-        const uint8_t lab = leaf_point<FP32>(Q, ll[i], ctr);
-        out[i] = lab;
-        inside += lab == CELL_IN;
+    extern __shared__ __align__(16) uint32_t s_sum[];
+    constexpr int WARPS = TPB / 32, TILE = WarpSpace<U>::TILE;
+    __shared__ WarpSpace<U> s_q[WARPS];
+    __shared__ __align__(8) uint64_t s_bar;
+    __shared__ int s_late;
+    bool late = false;
+    if (STAGE) {
+        if (threadIdx.x == 0) {
+            s_late = 0;
+            mbar_init(&s_bar);
+            bulk_stage(s_sum, Q.summary, summary_bytes(Q.swords), &s_bar);
+        }
+        __syncthreads();
+        if (!mbar_wait(&s_bar, 0, poll_limit)) s_late = 1;
+        __syncthreads();
+        late = s_late != 0;
+        // after a wait that ran out the block reads the summary from global
+        // memory and never touches s_sum, which the pending copy still targets
+        if (late && threadIdx.x == 0) atomicAdd(&g_tma_timeouts, 1u);
     }
-    if (ctr) count_inside(inside, ctr + 3);
+    QueryCounts c;
+    const int warp = threadIdx.x >> 5;
+    query_tiles<FP32, STATS, U>(Q, STAGE && !late ? s_sum : Q.summary, (blockIdx.x * WARPS + warp) * TILE,
+                                gridDim.x * WARPS * TILE, n, ll, out, s_q[warp], c);
+    if (STAGE && late) mbar_wait(&s_bar, 0);  // the copy in flight ends before the block does (bounded)
+    if (STATS && ctr) count_stats(ctr, c);
 }
 
 // ------------------------------------------------------------- batches --
@@ -695,69 +897,185 @@ struct BatchChunk {
     long long start;
 };
 
-constexpr int BATCH_SUMMARY_WORDS = 4096;  // 16 KB of shared memory
-// Launch shapes of the batch locate: points per thread in flight (in
-// lockstep) and blocks per SM (all resident; each holds 32 KB of shared
-// memory, and the register budget per thread follows from the blocks).  The
-// default, five points at five blocks (48 registers), took a 1,024-polygon
-// C3 batch from 75.6 (8 points, two blocks) to 106.5 Gpts/s; 4 x 5 101.2,
-// 6 x 4 101.8, 6 x 5 102.3, 4 x 6 91.2, 8 x 3 93.5 (labels identical): more
-// warps hide more of the node descents' latency than more points per
-// thread (2 x 6 spills at 40 registers and ran at 56.6).  Batches of other
-// point mixes may prefer another row (4 x 4 leaves fewer lanes idle in
-// chunks of few points); the batch autotuner measures them.
+// Launch shapes of the batch locate: points a thread loads at a time and
+// blocks per SM (all resident; the register budget per thread follows from the
+// blocks).  Batches of other point mixes may prefer another row; the batch
+// autotuner measures them.
 struct BatchShape {
     int unroll, blocks;
 };
 constexpr BatchShape BATCH_SHAPES[] = {{5, 5}, {4, 4}, {6, 4}, {8, 3}};
 constexpr int BATCH_NSHAPES = (int)(sizeof(BATCH_SHAPES) / sizeof(BATCH_SHAPES[0]));
 
+// Pass 1 over the points of one chunk, by a block whose warps take tiles of
+// 32 * U points: as locate_points, the points in mixed blocks wait in the
+// warp's queue; B_DESCENTS per lane descend in lockstep (1, 2 and 3 per lane:
+// 89, 79 and 80 us for the 6 x 4 shape on 28M points in 160 polygons, the
+// others within 3 us).  Descending every point where it stood, five to a
+// thread, the same points took 228 us in the same chunks as 150 now.
+constexpr int B_DESCENTS = 2;
+template <bool STATS, int U>
+__device__ __forceinline__ void locate_chunk(const QueryView& Q, const uint32_t* sum, const double2* __restrict__ ll,
+                                             int n, uint8_t* __restrict__ out, uint32_t first,
+                                             uint32_t* __restrict__ queue, uint32_t* __restrict__ leafq,
+                                             unsigned int* qcount, uint32_t* mixed, int& inside)
+{
+    const int lane = threadIdx.x & 31;
+    int nm = 0;
+    for (int base = (threadIdx.x >> 5) * 32 * U;; base += TPB * U) {
+        const bool last = base >= n;
+        if (!last) {
+            double2 p[U];
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                const int i = base + 32 * k + lane;
+                p[k] = i < n ? __ldg(ll + i) : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                const int i = base + 32 * k + lane;
+                const uint32_t l = coarse_label(Q, sum, p[k].x, p[k].y);
+                if (i < n) out[i] = (uint8_t)l;
+                if (STATS) inside += (l == CELL_IN) & (i < n);
+                const bool push = l == 0 && i < n;
+                const unsigned int mk = __ballot_sync(0xffffffffu, push);
+                if (push) mixed[nm + __popc(mk & ((1u << lane) - 1u))] = (uint32_t)i;
+                nm += __popc(mk);
+            }
+            __syncwarp();
+        }
+        while (nm >= 32 * B_DESCENTS || (last && nm > 0)) {
+            const int m = min(nm, 32 * B_DESCENTS);
+            nm -= m;
+            uint32_t i[B_DESCENTS], w[B_DESCENTS], fu[B_DESCENTS], fv[B_DESCENTS];
+#pragma unroll
+            for (int d = 0; d < B_DESCENTS; d++) {
+                w[d] = KIND_PURE | 4u;  // no point, or non-finite input, which stays undefined (LABEL_PENDING)
+                i[d] = fu[d] = fv[d] = 0;
+                if (lane + 32 * d < m) {
+                    i[d] = mixed[nm + lane + 32 * d];
+                    const double2 p = __ldg(ll + i[d]);
+                    const double laf = p.y + 90.0;
+                    Loc L;
+                    if (usual(p.x, laf)) {
+                        w[d] = Q.outside;
+                        if (domain_locate(Q, p.x, laf, L)) {
+                            w[d] = __ldg(Q.nodes + (size_t)L.iy * Q.W + L.ix);
+                            fu[d] = frac_bits(L.fu);
+                            fv[d] = frac_bits(L.fv);
+                        }
+                    } else if (isfinite(p.x) && isfinite(p.y)) {
+                        w[d] = LEAF_UNKNOWN;  // unusual coordinates: tier 1 locates them
+                    }
+                }
+            }
+            bool inner = true;
+            while (inner) {
+                inner = false;
+#pragma unroll
+                for (int d = 0; d < B_DESCENTS; d++)
+                    if ((w[d] & KIND_MASK) == KIND_INNER) {
+                        w[d] = __ldg(Q.nodes + (w[d] & INDEX_MASK) + (fv[d] >> 30) * FAN + (fu[d] >> 30));
+                        fu[d] <<= 2;
+                        fv[d] <<= 2;
+                        inner = true;
+                    }
+            }
+            unsigned int mk[B_DESCENTS], total = 0;
+#pragma unroll
+            for (int d = 0; d < B_DESCENTS; d++) {
+                const bool pure = (w[d] & KIND_MASK) == KIND_PURE;
+                if (pure && (w[d] & 3u)) {
+                    out[i[d]] = (uint8_t)(w[d] & 3u);
+                    if (STATS) inside += (w[d] & 3u) == CELL_IN;
+                }
+                mk[d] = __ballot_sync(0xffffffffu, !pure || w[d] == LEAF_UNKNOWN);
+                total += __popc(mk[d]);
+            }
+            if (total) {
+                unsigned int pos = 0;
+                if (lane == 0) pos = atomicAdd(qcount, total);
+                pos = __shfl_sync(0xffffffffu, pos, 0) + first;
+#pragma unroll
+                for (int d = 0; d < B_DESCENTS; d++) {
+                    if (mk[d] >> lane & 1u) {
+                        const unsigned int at = pos + __popc(mk[d] & ((1u << lane) - 1u));
+                        queue[at] = first + i[d];
+                        leafq[at] = w[d];
+                    }
+                    pos += __popc(mk[d]);
+                }
+            }
+            __syncwarp();
+        }
+        if (last) break;
+    }
+}
+
 // Pass 1 over a batch: a persistent grid takes chunks in order from an atomic
-// counter (polygons of very different sizes balance themselves), stages the
-// chunk's polygon summary in shared memory and runs the single-polygon tile
-// loop on it.
+// counter (polygons of very different sizes balance themselves; the next
+// chunk's number is on its way while a chunk is worked on), copies the chunk's
+// view and polygon summary to shared memory and runs the tile loop on it.  A
+// chunk's points in leaves are queued from the chunk's own first place,
+// counted in shared memory: no global atomic (see QUEUE_PARTS).
 template <bool STATS, int UNROLL, int BLOCKS>
 __global__ void __launch_bounds__(TPB, BLOCKS) k_batch_locate(const QueryView* __restrict__ views,
                                                      const BatchChunk* __restrict__ chunks, int nchunks,
                                                      unsigned int* next_chunk, const double2* __restrict__ ll,
                                                      uint8_t* __restrict__ out, uint32_t* __restrict__ queue,
-                                                     uint32_t* __restrict__ leafq, unsigned int* __restrict__ qcount,
+                                                     uint32_t* __restrict__ leafq, unsigned int* __restrict__ ccount,
                                                      unsigned long long* ctr, int poll_limit)
 {
-    // s_sum receives the bulk copies; after a wait runs out the block loads
-    // summaries itself into s_own, which no copy writes
-    __shared__ __align__(16) uint32_t s_sum[BATCH_SUMMARY_WORDS];
-    __shared__ __align__(16) uint32_t s_own[BATCH_SUMMARY_WORDS];
+    __shared__ __align__(16) uint32_t s_sum[SUMMARY_WORDS_MAX];  // receives the bulk copies
+    __shared__ __align__(16) uint32_t s_view[sizeof(QueryView) / 4];
+    __shared__ uint32_t s_mixed[TPB / 32][32 * (B_DESCENTS + UNROLL)];
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ int s_chunk, s_late;
+    __shared__ unsigned int s_queued;
+    static_assert(sizeof(QueryView) % 4 == 0 && sizeof(QueryView) / 4 <= TPB, "a word of the view per thread");
     if (threadIdx.x == 0) {
         s_late = 0;
         mbar_init(&s_bar);
+        s_chunk = (int)atomicAdd(next_chunk, 1u);
+        s_queued = 0;
     }
     uint32_t phase = 0;
     bool late = false;  // the same in every thread: read from s_late after a barrier
     int inside = 0;
+    __syncthreads();
     for (;;) {
-        if (threadIdx.x == 0) s_chunk = (int)atomicAdd(next_chunk, 1u);
-        __syncthreads();
         const int ci = s_chunk;
         if (ci >= nchunks) break;
         const BatchChunk c = chunks[ci];
-        const QueryView Q = views[c.view];
-        const uint32_t* sum = s_sum;
+        if (threadIdx.x < sizeof(QueryView) / 4) s_view[threadIdx.x] = __ldg((const uint32_t*)(views + c.view) + threadIdx.x);
+        __syncthreads();
+        const QueryView& Q = *(const QueryView*)s_view;
+        unsigned int next = 0;
+        if (threadIdx.x == 0) {
+            if (!late) bulk_stage(s_sum, Q.summary, summary_bytes(Q.swords), &s_bar);
+            next = atomicAdd(next_chunk, 1u);
+        }
         if (!late) {
-            if (threadIdx.x == 0) bulk_stage(s_sum, Q.summary, summary_bytes(Q.swords), &s_bar);
             if (!mbar_wait(&s_bar, phase, poll_limit)) s_late = 1;  // any thread's timeout switches the block
             phase ^= 1u;
             __syncthreads();
             late = s_late != 0;
         }
-        if (late) {
-            for (int k = threadIdx.x; k < Q.swords; k += TPB) s_own[k] = __ldg(Q.summary + k);
-            sum = s_own;
-            __syncthreads();
+        uint32_t* mixed = s_mixed[threadIdx.x >> 5];
+        // after a wait that ran out the block reads the summaries from global
+        // memory and never touches s_sum, which the pending copy still targets
+        if (!late)
+            locate_chunk<STATS, UNROLL>(Q, s_sum, ll + c.start, c.count, out + c.start, (uint32_t)c.start, queue, leafq,
+                                        &s_queued, mixed, inside);
+        else
+            locate_chunk<STATS, UNROLL>(Q, Q.summary, ll + c.start, c.count, out + c.start, (uint32_t)c.start, queue,
+                                        leafq, &s_queued, mixed, inside);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            ccount[ci] = s_queued;
+            s_queued = 0;
+            s_chunk = (int)next;
         }
-        locate_range<STATS, true, UNROLL>(Q, sum, ll, out, queue, leafq, qcount, c.start, c.count, 0, 1, inside);
         __syncthreads();
     }
     if (late) {
@@ -768,55 +1086,183 @@ __global__ void __launch_bounds__(TPB, BLOCKS) k_batch_locate(const QueryView* _
     if (STATS && ctr) count_inside(inside, ctr + 3);
 }
 
-// Escalation queues of one pass-2 run.  cnt[0] / cnt[1] count the points
-// deferred to tier 2 / tier 3 (they keep counting past the capacities);
-// cnt[2] is raised when a point found its queue full: it stays unlabelled
-// (pass 1 wrote LABEL_PENDING) and the final sweep gives it the complete
-// test, so no tier carries the code of the tiers after it.
-// Every queue of points has a parallel array of leaf words (l1 for the
-// pass-1 queue): the node word pass 1 found for the point, or LEAF_UNKNOWN
-// when it did not locate it, so the tiers need not descend again.
+// Prefix sums of the chunks' queue counts, by one block: pre[c] entries come
+// before chunk c's, pre[nchunks] in all.
+constexpr int CS_TPB = 1024, CS_ITEMS = 8;
+__global__ void __launch_bounds__(CS_TPB) k_chunk_scan(const unsigned int* __restrict__ ccount, int nchunks,
+                                                      unsigned int* __restrict__ pre)
+{
+    __shared__ unsigned int s_w[CS_TPB / 32];
+    wait_for_predecessor();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned int before = 0;
+    for (int base = 0; base < nchunks; base += CS_TPB * CS_ITEMS) {
+        const int b0 = base + threadIdx.x * CS_ITEMS;
+        unsigned int c[CS_ITEMS], run = 0;
+#pragma unroll
+        for (int k = 0; k < CS_ITEMS; k++) {
+            c[k] = b0 + k < nchunks ? ccount[b0 + k] : 0u;
+            run += c[k];
+        }
+        unsigned int x = run;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_w[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            const unsigned int v = s_w[lane];
+            unsigned int z = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned int y = __shfl_up_sync(0xffffffffu, z, o);
+                if (lane >= o) z += y;
+            }
+            s_w[lane] = z;
+        }
+        __syncthreads();
+        unsigned int at = before + (warp ? s_w[warp - 1] : 0u) + x - run;
+#pragma unroll
+        for (int k = 0; k < CS_ITEMS; k++) {
+            if (b0 + k < nchunks) pre[b0 + k] = at;
+            at += c[k];
+        }
+        before += s_w[CS_TPB / 32 - 1];
+        __syncthreads();  // s_w is rewritten
+    }
+    if (threadIdx.x == 0) pre[nchunks] = before;
+    allow_dependents();
+}
+
+// --------------------------------------------- the tiers as launches of their own --
+
+// A queue in parts: place p * cap + k holds entry k of part p, counted on
+// cnt[p * COUNTER_STRIDE] (which keeps counting past cap).
+struct PartQueue {
+    unsigned int* cnt = nullptr;
+    int parts = 1;
+    unsigned int cap = 0;
+};
+
 struct Tiers {
-    uint32_t* q2;
-    uint32_t* q3;
-    uint32_t* l1;
-    uint32_t* l2;
-    uint32_t* l3;
-    uint32_t* m2;   // per tier-2 entry: tier 1's mask of undecided records (leaf_label_fp32)
-    unsigned int* cnt;
-    unsigned int cap2, cap3;
-    // the pass-1 queue in window order (k_part_scatter), used by the first
-    // tier when *sorted == 1
+    // pass 1's queue: points in leaves and their leaf words, in parts (one
+    // polygon), or from each chunk's first place (batches: chunks, pre)
+    const uint32_t* q1;
+    const uint32_t* l1;
+    PartQueue p1;
+    const BatchChunk* chunks = nullptr;
+    const unsigned int* pre = nullptr;
+    int nchunks = 0;
+    // that queue in window or leaf order, used when *sorted == 1
     const uint32_t* spts = nullptr;
     const uint32_t* sleaf = nullptr;
     const unsigned int* sorted = nullptr;
     int sstride = 1;  // words from one ordered entry to the next (2: leaf order's interleaved pairs)
+    // tier 2's queue behind tier 1: points, leaf words, masks of undecided records
+    uint32_t* q2 = nullptr;
+    uint32_t* l2 = nullptr;
+    uint32_t* m2 = nullptr;
+    PartQueue p2;
+    unsigned int* over = nullptr;  // raised when a part of it is full
 };
 
-// The pass-1 queue as the first tier reads it: in window order when
-// k_part_scatter ran, else in pass-1 order.
-__device__ __forceinline__ void first_tier_source(const Tiers& T, const uint32_t*& pts, const uint32_t*& leaf,
-                                                  unsigned int& stride)
-{
-    stride = 1;
-    if (T.sorted && *(const volatile unsigned int*)T.sorted == 1u) {
-        pts = T.spts;
-        leaf = T.sleaf;
-        stride = (unsigned int)T.sstride;
+// The entries of a part queue in one sequence, part after part, for a warp:
+// lanes hold the parts' prefix sums.
+struct PartEntries {
+    unsigned int pa, pb, total, cap;  // entries before part `lane` and part `lane + 32`
+
+    __device__ __forceinline__ void begin(const PartQueue& P)
+    {
+        static_assert(QUEUE_PARTS <= 64, "two parts per lane");
+        const int lane = threadIdx.x & 31;
+        cap = P.cap;
+        const unsigned int a = lane < P.parts ? min(P.cnt[lane * COUNTER_STRIDE], cap) : 0u;
+        const unsigned int b = lane + 32 < P.parts ? min(P.cnt[(lane + 32) * COUNTER_STRIDE], cap) : 0u;
+        unsigned int x = a, y = b;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int u = __shfl_up_sync(0xffffffffu, x, o), v = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= o) {
+                x += u;
+                y += v;
+            }
+        }
+        const unsigned int ta = __shfl_sync(0xffffffffu, x, 31);
+        pa = x - a;
+        pb = ta + y - b;
+        total = ta + __shfl_sync(0xffffffffu, y, 31);
     }
-}
+    __device__ __forceinline__ unsigned int before(int p) const  // p the same in every lane
+    {
+        const unsigned int x = __shfl_sync(0xffffffffu, p < 32 ? pa : pb, p & 31);
+        return p < 64 ? x : total;
+    }
+    // the place of entry t = t0 + lane (t0 < total); every lane calls
+    __device__ __forceinline__ unsigned int place(unsigned int t0) const
+    {
+        const unsigned int t = t0 + (threadIdx.x & 31);
+        int p = __popc(__ballot_sync(0xffffffffu, pa <= t0)) + __popc(__ballot_sync(0xffffffffu, pb <= t0)) - 1;
+        unsigned int lo = before(p), hi = before(p + 1), at = 0;
+        for (;;) {
+            if (t >= lo) at = (unsigned int)p * cap + (t - lo);
+            if (hi >= total || !__any_sync(0xffffffffu, t >= hi)) return at;
+            p++;
+            lo = hi;
+            hi = before(p + 1);
+        }
+    }
+};
 
 // Where a queued point's index view comes from: one polygon...
 struct OneView {
     QueryView Q;
+    struct Source {
+        PartEntries E;
+        bool ordered;
+    };
     __device__ __forceinline__ const QueryView& of(uint32_t) const { return Q; }
+    __device__ __forceinline__ const QueryView& view(int) const { return Q; }
+    __device__ __forceinline__ unsigned int begin(const Tiers& T, Source& S) const
+    {
+        S.ordered = T.sorted && *(const volatile unsigned int*)T.sorted == 1u;
+        S.E.begin(T.p1);
+        return S.E.total;
+    }
+    // entry t0 + lane of pass 1's queue: point and leaf word; every lane calls
+    __device__ __forceinline__ void fetch(const Tiers& T, const Source& S, unsigned int t0, uint32_t& i, uint32_t& w,
+                                          int&) const
+    {
+        const unsigned int at = S.E.place(t0);
+        if (t0 + (threadIdx.x & 31) >= S.E.total) return;
+        if (S.ordered) {  // (an ordered queue has one part)
+            i = T.spts[at * T.sstride];
+            w = T.sleaf[at * T.sstride];
+        } else {
+            i = T.q1[at];
+            w = T.l1[at];
+        }
+    }
 };
 
-// ...or the chunk holding it (binary search of the chunk starts).
+// The last p with pre[p] <= t, p in [0, n).
+__device__ __forceinline__ int last_before(const unsigned int* __restrict__ pre, int n, unsigned int t)
+{
+    int lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(pre + mid) <= t) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// ...or its chunk's.
 struct ChunkViews {
     const QueryView* views;
     const BatchChunk* chunks;
     int nchunks;
+    struct Source {
+        unsigned int total;
+    };
     __device__ __forceinline__ const QueryView& of(uint32_t i) const
     {
         int lo = 0, hi = nchunks;  // chunks[lo].start <= i < chunks[hi].start
@@ -827,112 +1273,108 @@ struct ChunkViews {
         }
         return views[__ldg(&chunks[lo].view)];
     }
+    __device__ __forceinline__ const QueryView& view(int v) const { return views[v]; }
+    __device__ __forceinline__ unsigned int begin(const Tiers& T, Source& S) const
+    {
+        S.total = T.pre[nchunks];
+        return S.total;
+    }
+    __device__ __forceinline__ void fetch(const Tiers& T, const Source& S, unsigned int t0, uint32_t& i, uint32_t& w,
+                                          int& v) const
+    {
+        const unsigned int t = t0 + (threadIdx.x & 31);
+        if (t >= S.total) return;
+        const int c = last_before(T.pre, nchunks, t);
+        const unsigned int at = (unsigned int)__ldg(&chunks[c].start) + (t - __ldg(T.pre + c));
+        v = __ldg(&chunks[c].view);
+        i = T.q1[at];
+        w = T.l1[at];
+    }
 };
 
-// Appends i to q through counter *c, one atomic per group of converged
-// threads; false when the queue is full.
-__device__ __forceinline__ bool push_deferred(uint32_t i, uint32_t w, uint32_t* q, uint32_t* l, unsigned int* c,
-                                              unsigned int cap, uint32_t* extra = nullptr, uint32_t x = 0u)
+// A warp's deferred points to tier 2's queue, one atomic on its part's
+// counter; a point that finds the part full is marked, and the tier 2 launch
+// finishes it from pass 1's queue (pass 1 wrote LABEL_PENDING for every queued
+// point, so a mark is never something else's).
+constexpr uint8_t LABEL_OVER = 0xFE;
+__device__ __forceinline__ void push_deferred(bool defer, uint32_t i, uint32_t w, uint32_t mask, const Tiers& T,
+                                              uint8_t* out)
 {
-    const unsigned int act = __activemask();
+    const unsigned int bal = __ballot_sync(0xffffffffu, defer);
+    if (!bal) return;
     const int lane = threadIdx.x & 31;
-    const int leader = __ffs(act) - 1;
-    unsigned int base = 0;
-    if (lane == leader) base = atomicAdd(c, (unsigned int)__popc(act));
-    base = __shfl_sync(act, base, leader);
-    const unsigned int pos = base + __popc(act & ((1u << lane) - 1u));
-    if (pos >= cap) return false;
-    q[pos] = i;
-    l[pos] = w;
-    if (extra) extra[pos] = x;
-    return true;
+    const unsigned int part = blockIdx.x % (unsigned int)T.p2.parts;
+    unsigned int pos = 0;
+    if (lane == 0) pos = atomicAdd(T.p2.cnt + part * COUNTER_STRIDE, (unsigned int)__popc(bal));
+    pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(bal & ((1u << lane) - 1u));
+    if (!defer) return;
+    if (pos < T.p2.cap) {
+        const unsigned int at = part * T.p2.cap + pos;
+        T.q2[at] = i;
+        T.l2[at] = w;
+        T.m2[at] = mask;
+    } else {
+        out[i] = LABEL_OVER;
+        *T.over = 1u;
+    }
 }
 
-__device__ __forceinline__ void count_stats(unsigned long long* ctr, int inside, int boundary, int fp64, int exact)
-{
-    count_inside(inside, ctr + 3);
-    count_inside(boundary, ctr + 2);
-    count_inside(fp64, ctr + 0);
-    count_inside(exact, ctr + 1);
-}
-
-// Tier 1 over the pass-1 queue.
+// Tier 1 over the pass-1 queue, perhaps ordered.  A warp takes 32 entries at a
+// time, the next 32 entries' points and leaf words loaded ahead, and meets no
+// other warp (the block's rounds used to end in three barriers around one
+// atomic; with the counter in parts a warp's own atomic costs nothing).  Four
+// blocks per SM: 64 registers, no spills, 279 us against 315 at five (48) for
+// the 9.1M points in leaves of 2e7 near-edge points.
+constexpr int T1_BLOCKS = 4;
 template <class VS>
-__global__ void __launch_bounds__(TPB, T1_BLOCKS) k_leaf_t1(VS vs, const double2* __restrict__ ll,
-                                                         uint8_t* __restrict__ out, const uint32_t* __restrict__ queue,
-                                                         const unsigned int* __restrict__ qcount, Tiers T,
-                                                         unsigned long long* ctr)
+__global__ void __launch_bounds__(TPB, T1_BLOCKS) k_leaf_t1(const __grid_constant__ VS vs,
+                                                         const double2* __restrict__ ll, uint8_t* __restrict__ out,
+                                                         const __grid_constant__ Tiers T, unsigned long long* ctr)
 {
-    __shared__ unsigned int s_wcnt[TPB / 32];
-    __shared__ unsigned int s_base;
     wait_for_predecessor();
-    const unsigned int m = *qcount;
-    const uint32_t* src = queue;
-    const uint32_t* src_leaf = T.l1;
-    unsigned int st;
-    first_tier_source(T, src, src_leaf, st);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int inside = 0, boundary = 0, fp64 = 0;
-    // block-uniform loop: the deferred points of a block's round take one
-    // atomic on the tier-2 counter (about half the points defer on near-edge
-    // inputs, and one counter serves the whole grid)
-    for (unsigned int b0 = blockIdx.x * blockDim.x; b0 < m; b0 += gridDim.x * blockDim.x) {
-        const unsigned int t = b0 + threadIdx.x;
+    typename VS::Source S;
+    const unsigned int m = vs.begin(T, S);
+    QueryCounts c;
+    const unsigned int step = gridDim.x * blockDim.x, lane = threadIdx.x & 31;
+    unsigned int t0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+    uint32_t ni = 0, nw = 0;
+    int nv = 0;
+    if (t0 < m) vs.fetch(T, S, t0, ni, nw, nv);
+    for (; t0 < m; t0 += step) {
+        const uint32_t i = ni, known = nw;
+        const QueryView& Q = vs.view(nv);
+        const bool mine = t0 + lane < m;
         bool defer = false;
-        uint32_t i = 0, w = 0, mask = 0;
-        if (t < m) {
-            i = src[t * st];
-            const uint32_t known = src_leaf[t * st];
-            const QueryView& Q = vs.of(i);
-            // the leaf record (a point pass 1 located in a leaf) is loaded
-            // with the point's coordinates, not after them
-            const bool in_leaf = (known & KIND_MASK) == KIND_LEAF;
-            LeafRec L0;
-            if (in_leaf) L0 = Q.leaves[known & INDEX_MASK];
-            PointCtx P;
-            w = point_leaf(Q, ll[i], P, known);
-            uint8_t lab;
-            if ((w & KIND_MASK) == KIND_PURE) {
-                lab = (uint8_t)(w & 3u);
-            } else {
-                boundary++;
-                lab = leaf_label_fp32(Q, in_leaf ? L0 : Q.leaves[w & INDEX_MASK], P, mask);
+        uint32_t w = 0, mask = 0;
+        PointCtx P{0.0, 0.0};
+        LeafLoad L;
+        double2 p = make_double2(0.0, 0.0);
+        const bool in_leaf = (known & KIND_MASK) == KIND_LEAF;
+        if (mine) {
+            p = ll[i];
+            if (in_leaf) L = load_leaf<false>(Q.leaves + (known & INDEX_MASK));
+        }
+        if (t0 + step < m) vs.fetch(T, S, t0 + step, ni, nw, nv);
+        if (mine) {
+            w = point_leaf(Q, p, P, known);
+            uint8_t lab = (uint8_t)(w & 3u);
+            if ((w & KIND_MASK) != KIND_PURE) {
+                c.boundary++;
+                if (!in_leaf) L = load_leaf<false>(Q.leaves + (w & INDEX_MASK));
+                lab = leaf_label_fp32<false>(Q.recs + L.off, L, P, mask);
             }
-            if (lab == LABEL_DEFER) {
-                fp64++;
-                defer = true;
+            defer = lab == LABEL_DEFER;
+            if (defer) {
+                c.fp64++;
             } else {
                 out[i] = lab;
-                inside += lab == CELL_IN;
+                c.inside += lab == CELL_IN;
             }
         }
-        const unsigned int bal = __ballot_sync(0xffffffffu, defer);
-        if (lane == 0) s_wcnt[warp] = __popc(bal);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned int tot = 0;
-            for (int k = 0; k < TPB / 32; k++) {
-                const unsigned int c = s_wcnt[k];
-                s_wcnt[k] = tot;
-                tot += c;
-            }
-            s_base = tot ? atomicAdd(T.cnt, tot) : 0u;
-        }
-        __syncthreads();
-        if (defer) {
-            const unsigned int pos = s_base + s_wcnt[warp] + __popc(bal & ((1u << lane) - 1u));
-            if (pos < T.cap2) {
-                T.q2[pos] = i;
-                T.l2[pos] = w;
-                T.m2[pos] = mask;
-            } else {
-                T.cnt[2] = 1;  // the tier-3 sweep labels it
-            }
-        }
-        __syncthreads();  // s_wcnt / s_base are rewritten next round
+        push_deferred(defer, i, w, mask, T, out);
     }
     allow_dependents();
-    if (ctr) count_stats(ctr, inside, boundary, fp64, 0);
+    if (ctr) count_stats(ctr, c);
 }
 
 // ---------------------------------- tier 1 with the edge lists staged --
@@ -959,21 +1401,18 @@ __global__ void __launch_bounds__(TPB, T1_BLOCKS) k_leaf_t1(VS vs, const double2
 // per-warp gathers leaf order already makes one request per warp and leaf;
 // the staging adds a block barrier and a wait per tile and copies every
 // leaf of the tile's range.  It is therefore an option (pass-2 order 3).
-constexpr int T1S_LEAVES = 256;  // 8 KB of leaf records per tile
-constexpr int T1S_RECS = 1536;   // 24 KB of edge records per tile
+constexpr int T1S_LEAVES = 256;  // 16 KB of leaf records per tile
+constexpr int T1S_RECS = 1024;   // 16 KB of edge records per tile
 constexpr int T1S_BLOCKS = 5;
 
-__global__ void __launch_bounds__(TPB, T1S_BLOCKS) k_leaf_t1s(QueryView Q, const double2* __restrict__ ll,
+__global__ void __launch_bounds__(TPB, T1S_BLOCKS) k_leaf_t1s(const __grid_constant__ QueryView Q, const double2* __restrict__ ll,
                                                             uint8_t* __restrict__ out,
-                                                            const uint32_t* __restrict__ queue,
-                                                            const unsigned int* __restrict__ qcount, Tiers T,
+                                                            const __grid_constant__ Tiers T,
                                                             unsigned long long* ctr, int polls)
 {
     __shared__ __align__(16) LeafRec s_leaf[T1S_LEAVES];
     __shared__ __align__(16) float4 s_rec[T1S_RECS];
     __shared__ __align__(8) uint64_t s_bar;
-    __shared__ unsigned int s_wcnt[TPB / 32];
-    __shared__ unsigned int s_base;
     __shared__ uint32_t s_l0, s_r0, s_nr;  // first staged leaf, first staged record, records staged
     __shared__ int s_nl;                   // leaves staged for the tile (0: none)
     __shared__ int s_broken;               // a wait ran out: no more staging
@@ -983,14 +1422,14 @@ __global__ void __launch_bounds__(TPB, T1S_BLOCKS) k_leaf_t1s(QueryView Q, const
     }
     __syncthreads();
     wait_for_predecessor();
-    const unsigned int m = *qcount;
-    const uint32_t* src = queue;
-    const uint32_t* src_leaf = T.l1;
-    unsigned int st;
-    first_tier_source(T, src, src_leaf, st);
+    // (an ordered queue has one part: entries are at t * st)
+    const unsigned int m = *T.p1.cnt;
+    const bool ordered = *(const volatile unsigned int*)T.sorted == 1u;
+    const uint32_t* src = ordered ? T.spts : T.q1;
+    const uint32_t* src_leaf = ordered ? T.sleaf : T.l1;
+    const unsigned int st = ordered ? (unsigned int)T.sstride : 1u;
     const bool sorted = src_leaf != T.l1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int inside = 0, boundary = 0, fp64 = 0;
+    QueryCounts c;
     uint32_t phase = 0;  // parity of the barrier's current phase
     // Thread 0 works a tile ahead so that a tile's copy goes out as the tile
     // starts: while the block labels tile k it loads the first and last leaf
@@ -1062,7 +1501,7 @@ __global__ void __launch_bounds__(TPB, T1S_BLOCKS) k_leaf_t1s(QueryView Q, const
         const unsigned int t = b0 + threadIdx.x;
         bool defer = false;
         uint32_t i = 0, w = 0, mask = 0;
-        PointCtx P;
+        PointCtx P{0.0, 0.0};
         if (t < m) {
             i = src[t * st];
             w = point_leaf(Q, ll[i], P, src_leaf[t * st]);
@@ -1076,144 +1515,128 @@ __global__ void __launch_bounds__(TPB, T1S_BLOCKS) k_leaf_t1s(QueryView Q, const
             if (!staged) atomicOr(&s_broken, 1);  // any thread whose wait ran out
         }
         if (t < m) {
-            uint8_t lab;
-            if ((w & KIND_MASK) == KIND_PURE) {
-                lab = (uint8_t)(w & 3u);
-            } else {
-                boundary++;
+            uint8_t lab = (uint8_t)(w & 3u);
+            if ((w & KIND_MASK) != KIND_PURE) {
+                c.boundary++;
                 const uint32_t li = (w & INDEX_MASK) - s_l0;  // wraps above nl below the first leaf
                 bool done = false;
                 if (staged && li < (uint32_t)nl) {
-                    const LeafRec L = s_leaf[li];
+                    const LeafLoad L = load_leaf<true>(s_leaf + li);
                     const uint32_t ro = L.off - s_r0;
-                    if (ro <= s_nr && (uint32_t)L.cnt <= s_nr - ro) {
-                        lab = leaf_label_fp32_at<true>(s_rec + ro, L, P, mask);
+                    if (ro <= s_nr && (uint32_t)L.cnt() <= s_nr - ro) {
+                        lab = leaf_label_fp32<true>(s_rec + ro, L, P, mask);
                         done = true;
                     }
                 }
-                if (!done) lab = leaf_label_fp32(Q, Q.leaves[w & INDEX_MASK], P, mask);
+                if (!done) {
+                    const LeafLoad L = load_leaf<false>(Q.leaves + (w & INDEX_MASK));
+                    lab = leaf_label_fp32<false>(Q.recs + L.off, L, P, mask);
+                }
             }
-            if (lab == LABEL_DEFER) {
-                fp64++;
-                defer = true;
+            defer = lab == LABEL_DEFER;
+            if (defer) {
+                c.fp64++;
             } else {
                 out[i] = lab;
-                inside += lab == CELL_IN;
+                c.inside += lab == CELL_IN;
             }
         }
         if (threadIdx.x == 0 && sorted && b0 + bstep < m) tile_bounds();  // the next tile's, ahead of its start
-        const unsigned int bal = __ballot_sync(0xffffffffu, defer);
-        if (lane == 0) s_wcnt[warp] = __popc(bal);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned int tot = 0;
-            for (int k = 0; k < TPB / 32; k++) {
-                const unsigned int c = s_wcnt[k];
-                s_wcnt[k] = tot;
-                tot += c;
-            }
-            s_base = tot ? atomicAdd(T.cnt, tot) : 0u;
-        }
-        __syncthreads();
-        if (defer) {
-            const unsigned int pos = s_base + s_wcnt[warp] + __popc(bal & ((1u << lane) - 1u));
-            if (pos < T.cap2) {
-                T.q2[pos] = i;
-                T.l2[pos] = w;
-                T.m2[pos] = mask;
-            } else {
-                T.cnt[2] = 1;  // the tier-3 sweep labels it
-            }
-        }
-        __syncthreads();  // s_wcnt / s_base and the staged slices are rewritten next round
+        push_deferred(defer, i, w, mask, T, out);
+        __syncthreads();  // the staged slices are rewritten next round
     }
     allow_dependents();
     if (threadIdx.x == 0 && s_broken) {
         atomicAdd(&g_tma_timeouts, 1u);
         mbar_wait(&s_bar, phase ^ 1u);  // the copy whose wait ran out
     }
-    if (ctr) count_stats(ctr, inside, boundary, fp64, 0);
+    if (ctr) count_stats(ctr, c);
 }
 
-// Tier 2's shape: blocks of 128 threads, five per SM (96 registers, about
-// 60 bytes spilled) hold 20 warps per SM where 256-thread blocks at 110
-// registers held 16: FP64-filter queries of C2 (tier 2 over the whole
-// pass-1 queue) 15.8 -> 16.6 Gpts/s; six blocks (80 registers, 200 bytes
-// spilled) 12.8; the FP32 filter's tier 2 is unchanged by any of them.
+// Tier 2's shape: blocks of 128 threads, six per SM: 24 warps hide more of the
+// chain entry -> point and aux sector -> edge ends than the registers of
+// larger groups in flight.
 constexpr int T2_TPB = 128;
-constexpr int T2_BLOCKS = 5;
+constexpr int T2_BLOCKS = 6;
 
-// Tier 2 over the tier-1 queue, or (FROM_PASS1, FP64-filter queries) over
-// the pass-1 queue itself.
-template <class VS, bool FROM_PASS1>
-__global__ void __launch_bounds__(T2_TPB, T2_BLOCKS) k_leaf_t2(VS vs, const double2* __restrict__ ll, uint8_t* __restrict__ out,
-                                                const uint32_t* __restrict__ src, const uint32_t* __restrict__ src_leaf,
-                                                const unsigned int* __restrict__ src_count, unsigned int src_cap,
-                                                Tiers T, unsigned long long* ctr)
+// Tier 2, then the complete test for what it leaves, over the queue of
+// deferred points; ALL: FP64-filter queries, over pass 1's queue.  The next
+// entry is loaded ahead, as in tier 1.
+template <class VS, bool ALL>
+__global__ void __launch_bounds__(T2_TPB, T2_BLOCKS) k_leaf_t2(const __grid_constant__ VS vs,
+                                                              const double2* __restrict__ ll,
+                                                              uint8_t* __restrict__ out,
+                                                              const __grid_constant__ Tiers T,
+                                                              unsigned long long* ctr)
 {
     wait_for_predecessor();
-    const unsigned int m = min(*src_count, src_cap);
-    const uint32_t* sp = src;
-    const uint32_t* sl = src_leaf;
-    unsigned int st = 1;
-    if (FROM_PASS1) first_tier_source(T, sp, sl, st);
-    int inside = 0, boundary = 0, exact = 0;
-    for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
-        const uint32_t i = sp[t * st];
-        const QueryView& Q = vs.of(i);
-        PointCtx P;
-        const uint32_t w = point_leaf(Q, ll[i], P, sl[t * st]);
-        uint8_t lab;
-        if ((w & KIND_MASK) == KIND_PURE) {
-            lab = (uint8_t)(w & 3u);
+    typename VS::Source S;
+    PartEntries E;
+    unsigned int m;
+    if (ALL) {
+        m = vs.begin(T, S);
+    } else {
+        E.begin(T.p2);
+        m = E.total;
+    }
+    QueryCounts c;
+    const unsigned int step = gridDim.x * blockDim.x, lane = threadIdx.x & 31;
+    unsigned int t0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+    uint32_t ni = 0, nw = 0, nm = MASK_ALL;
+    int nv = 0;
+    auto fetch = [&](unsigned int at0) {
+        if (ALL) {
+            vs.fetch(T, S, at0, ni, nw, nv);
         } else {
-            if (FROM_PASS1) boundary++;
-            lab = leaf_label_fp64(Q, w & INDEX_MASK, P, FROM_PASS1 ? MASK_ALL : T.m2[t]);
+            const unsigned int at = E.place(at0);
+            if (at0 + lane < m) {
+                ni = T.q2[at];
+                nw = T.l2[at];
+                nm = T.m2[at];
+            }
+        }
+    };
+    if (t0 < m) fetch(t0);
+    for (; t0 < m; t0 += step) {
+        const uint32_t i = ni, known = nw, mask = nm;
+        const int v = nv;
+        const bool mine = t0 + lane < m;
+        double2 p = make_double2(0.0, 0.0);
+        if (mine) p = ll[i];
+        if (t0 + step < m) fetch(t0 + step);
+        if (!mine) continue;
+        const QueryView& Q = ALL ? vs.view(v) : vs.of(i);
+        PointCtx P;
+        const uint32_t w = point_leaf(Q, p, P, known);
+        uint8_t lab = (uint8_t)(w & 3u);
+        if ((w & KIND_MASK) != KIND_PURE) {
+            if (ALL) c.boundary++;
+            lab = leaf_label_fp64(Q, w & INDEX_MASK, P, mask);
             if (lab == LABEL_DEFER) {
-                exact++;
-                if (!push_deferred(i, w, T.q3, T.l3, T.cnt + 1, T.cap3)) T.cnt[2] = 1;
-                continue;
+                c.exact++;
+                lab = leaf_label_exact(&Q, w & INDEX_MASK, P.lon, P.lat);
             }
         }
         out[i] = lab;
-        inside += lab == CELL_IN;
+        c.inside += lab == CELL_IN;
+    }
+    if (!ALL && *(const volatile unsigned int*)T.over) {
+        // points that found their part of tier 2's queue full
+        const unsigned int n = vs.begin(T, S);
+        for (t0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); t0 < n; t0 += step) {
+            vs.fetch(T, S, t0, ni, nw, nv);
+            if (t0 + lane >= n || out[ni] != LABEL_OVER) continue;
+            const QueryView& Q = vs.view(nv);
+            PointCtx P;
+            const uint32_t w = point_leaf(Q, ll[ni], P, nw);
+            c.exact++;
+            const uint8_t lab = leaf_label_exact(&Q, w & INDEX_MASK, P.lon, P.lat);
+            out[ni] = lab;
+            c.inside += lab == CELL_IN;
+        }
     }
     allow_dependents();
-    if (ctr) count_stats(ctr, inside, boundary, 0, exact);
-}
-
-// Tier 3 over the tier-2 queue, then, after a queue overflow, the complete
-// test for every pass-1 point still unlabelled.
-template <class VS>
-__global__ void __launch_bounds__(TPB) k_leaf_t3(VS vs, const double2* __restrict__ ll, uint8_t* __restrict__ out,
-                                                const uint32_t* __restrict__ queue,
-                                                const unsigned int* __restrict__ qcount, Tiers T,
-                                                unsigned long long* ctr)
-{
-    wait_for_predecessor();
-    const unsigned int m3 = min(T.cnt[1], T.cap3);
-    const bool sweep = T.cnt[2] != 0;
-    const unsigned int m = sweep ? *qcount : 0;
-    int inside = 0;
-    for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < m3 + m; t += gridDim.x * blockDim.x) {
-        uint32_t i, known;
-        if (t < m3) {
-            i = T.q3[t];
-            known = T.l3[t];
-        } else {
-            i = queue[t - m3];
-            if (out[i] != LABEL_PENDING) continue;
-            known = T.l1[t - m3];
-        }
-        const QueryView& Q = vs.of(i);
-        PointCtx P;
-        const uint32_t w = point_leaf(Q, ll[i], P, known);
-        const uint8_t lab = ((w & KIND_MASK) == KIND_PURE) ? (uint8_t)(w & 3u)
-                                                            : leaf_label(Q, w & INDEX_MASK, P, false, nullptr);
-        out[i] = lab;
-        inside += lab == CELL_IN;
-    }
-    if (ctr) count_inside(inside, ctr + 3);
+    if (ctr) count_stats(ctr, c);
 }
 
 // ------------------------------------- pass-2 queue in leaf-window order --
@@ -1380,7 +1803,6 @@ struct LeafSortScratch {
     unsigned int* done;   // set to 1 with the sorted arrays; zero before the pass
     int nb;               // buckets: leaves + 1
     int tiles;            // ceil(nb / LS_TILE)
-    bool stage;           // tier 1 stages each tile's edge lists (k_leaf_t1s)
 };
 
 __device__ __forceinline__ int leaf_bucket(uint32_t w, int nb)
@@ -1513,48 +1935,27 @@ void launch_dependent(void (*kernel)(KArgs...), int grid, cudaStream_t s, Args..
     launch_dependent_tpb(kernel, grid, TPB, s, args...);
 }
 
-// Tier counters (T.cnt[0..2]) must be zero.  stage_t1 (one polygon, queue
-// in leaf order): tier 1 reads each tile's edge lists from shared memory
-// (k_leaf_t1s).
-template <class VS>
-void leaf_tiers_launch(const VS& vs, const double2* ll, uint8_t* out, const uint32_t* queue,
-                       const unsigned int* qcount, const Tiers& T, int precision, unsigned long long* ctr, int sms,
-                       cudaStream_t s, bool stage_t1 = false)
+// Tier 2's queue for `points` points: half of them (near-edge points defer 41 %
+// of those in leaves), in equal parts with room for the blocks of tier 1
+// being unequal; what finds its part full the tier 2 launch finishes.
+PartQueue tier2_parts(long long points, unsigned int* cnt)
 {
-    if (precision == GAHHG_QUERY_FP64_FILTER) {
-        launch_dependent_tpb(k_leaf_t2<VS, true>, sms * T2_BLOCKS, T2_TPB, s, vs, ll, out, queue,
-                             (const uint32_t*)T.l1, qcount, 0xffffffffu, T, ctr);
-    } else {
-        bool staged = false;
-        if constexpr (std::is_same<VS, OneView>::value) {
-            if (stage_t1) {
-                launch_dependent(k_leaf_t1s, sms * T1S_BLOCKS, s, vs.Q, ll, out, queue, qcount, T, ctr,
-                                 (int)knob(GAHHG_KNOB_STAGING_POLL_LIMIT));
-                staged = true;
-            }
-        }
-        if (!staged) launch_dependent(k_leaf_t1<VS>, sms * T1_BLOCKS, s, vs, ll, out, queue, qcount, T, ctr);
-        launch_dependent_tpb(k_leaf_t2<VS, false>, sms * T2_BLOCKS, T2_TPB, s, vs, ll, out, (const uint32_t*)T.q2,
-                             (const uint32_t*)T.l2, (const unsigned int*)T.cnt, T.cap2, T, ctr);
-    }
-    launch_dependent(k_leaf_t3<VS>, sms * 2, s, vs, ll, out, queue, qcount, T, ctr);
+    return PartQueue{cnt, QUEUE_PARTS, (unsigned int)(points / 2 / QUEUE_PARTS + 1024)};
 }
 
-// Escalation queue capacities for a pass-2 queue of `points` entries.
-inline void tier_caps(long long points, unsigned int* cap2, unsigned int* cap3)
+template <class VS>
+void tier2_launch(const VS& vs, const double2* ll, uint8_t* out, const Tiers& T, int precision,
+                  unsigned long long* ctr, int sms, cudaStream_t s)
 {
-    *cap2 = (unsigned int)(points / 2 + 1024);
-    *cap3 = (unsigned int)(points / 8 + 1024);
+    if (precision == GAHHG_QUERY_FP64_FILTER)
+        launch_dependent_tpb(k_leaf_t2<VS, true>, sms * T2_BLOCKS, T2_TPB, s, vs, ll, out, T, ctr);
+    else
+        launch_dependent_tpb(k_leaf_t2<VS, false>, sms * T2_BLOCKS, T2_TPB, s, vs, ll, out, T, ctr);
 }
 
 }  // namespace
 
 // ------------------------------------------------------------------ host --
-
-gahhg_status lattice_query_with(const QueryView& Q, const double* d_lonlat, long long n, uint8_t* d_labels,
-                                int precision, cudaStream_t s, uint64_t* d_counters, uint32_t* queue,
-                                unsigned int* qcount, long long chunk, int device, const Tiers* tiers,
-                                const PartScratch* part = nullptr, const LeafSortScratch* lsort = nullptr);
 
 static const QueryView& make_view(const Grid* g) { return g->lattice->views[0]; }
 
@@ -1568,168 +1969,207 @@ void set_leaf_windows(QueryView& Q, long long nleaves, long long nrecs)
     Q.part_scale = Q.nparts > 1 ? (float)((double)Q.nparts / (double)nleaves) : 0.0f;
 }
 
-// Points per pass; the pass-2 queue holds one 4-byte index per point.
+// Points per pass.
 constexpr long long QUERY_CHUNK = 1LL << 27;
+// Queries of at most this many points run as one launch with every tier
+// inline (k_query).  us a call, one launch | passes of their own:
+//   points      uniform      near the edges   (1.1M-edge polygon, FP32 filter)
+//     32,000     7 | 19         13 | 27
+//    131,072     9 | 19         23 | 31
+//    524,288    11 | 19         58 | 59
+//  1,048,576    14 | 20        102 | 89
+//  2,097,152    19 | 23        178 | 157
+// The line is where the two gains are about equal.
+constexpr long long INLINE_MAX = 1LL << 20;
+// ... and of at most this many with a point per lane and the summary read in
+// place: less than a block per SM, so the query's time is one point's latency
+// (staging the summary first: 2 us more).
+constexpr long long TINY_MAX = 1LL << 15;
+
+namespace {
+
+int sm_count(int device)
+{
+    static std::atomic<int> cache[64];
+    int sms = (device >= 0 && device < 64) ? cache[device].load(std::memory_order_relaxed) : 0;
+    if (!sms) {
+        sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        if (device >= 0 && device < 64) cache[device].store(sms, std::memory_order_relaxed);
+    }
+    return sms;
+}
+
+template <bool FP32, int U, bool STAGE>
+void launch_query(const QueryView& Q, const double2* ll, int n, uint8_t* out, unsigned long long* ctr, int sms,
+                  cudaStream_t s)
+{
+    constexpr int POINTS = TPB * U;
+    const int grid = (int)std::min<long long>(((long long)n + POINTS - 1) / POINTS, sms * (U == 1 ? 2LL : 4LL));
+    const int polls = (int)knob(GAHHG_KNOB_STAGING_POLL_LIMIT);
+    auto kern = ctr ? k_query<FP32, true, U, STAGE> : k_query<FP32, false, U, STAGE>;
+    kern<<<grid, TPB, STAGE ? summary_bytes(Q.swords) : 0, s>>>(ll, n, out, Q, ctr, polls);
+}
+
+// Every tier in one launch, no scratch.
+void query_inline(const QueryView& Q, const double2* ll, int n, uint8_t* out, int precision, unsigned long long* ctr,
+                  int sms, cudaStream_t s)
+{
+    if (precision == GAHHG_QUERY_FP64_FILTER) {
+        if (n <= TINY_MAX) launch_query<false, 1, false>(Q, ll, n, out, ctr, sms, s);
+        else launch_query<false, 2, true>(Q, ll, n, out, ctr, sms, s);
+    } else {
+        if (n <= TINY_MAX) launch_query<true, 1, false>(Q, ll, n, out, ctr, sms, s);
+        else launch_query<true, 2, true>(Q, ll, n, out, ctr, sms, s);
+    }
+}
+
+}  // namespace
 
 gahhg_status lattice_query(Grid* g, const double* d_lonlat, size_t n, uint8_t* d_labels, int precision,
                            cudaStream_t s, uint64_t* d_counters)
 {
     if (n == 0) return GAHHG_OK;
-    const QueryView Q = make_view(g);
+    const QueryView& Q = make_view(g);
+    const int sms = sm_count(g->device);
+    unsigned long long* ctr = (unsigned long long*)d_counters;
+    const bool fp64 = precision == GAHHG_QUERY_FP64_FILTER;
     const long long chunk = std::min<long long>((long long)n, QUERY_CHUNK);
-    // Words: [pass-2 queue: chunk][control: 192 (queue fill at +32, tier
-    // counters at +33..35, window-order flag at +36, entries per window at
-    // +64, windows' cursors at +128)][pass-2 leaf words: chunk][tier-2 queue]
-    // [its leaf words][tier-3 queue][its leaf words][tier-2 masks][queue in
-    // window order: points, leaf words (chunk each)].
-    // One memset per pass clears the control words from the queue fill on.
-    // [leaf order only: entries per leaf: nb][leaf starts: nb + 1][tile
-    // sums][ranks: chunk].
-    unsigned int cap2 = 0, cap3 = 0;
-    tier_caps(chunk, &cap2, &cap3);
     const long long order = knob(GAHHG_KNOB_GROUPED_PASS2);
     const bool windows = order == 1 && Q.nparts > 1 && chunk >= PART_MIN_QUEUE;
     const bool leaves = (order == 2 || order == 3) && chunk >= PART_MIN_QUEUE && g->lattice->nleaves > 0 &&
                         g->lattice->nleaves < (1LL << 30);
+    const bool ordered = windows || leaves;
+    if (!ordered && (long long)n <= INLINE_MAX) {
+        query_inline(Q, (const double2*)d_lonlat, (int)n, d_labels, precision, ctr, sms, s);
+        GAHHG_CUDA_TRY(cudaGetLastError());
+        return GAHHG_OK;
+    }
+    const long long ptiles = (chunk + TPB * LOC_UNROLL - 1) / (TPB * LOC_UNROLL);
+    const int lgrid = (int)std::min<long long>(ptiles, sms * 8LL);
+    const int parts = ordered ? 1 : std::min(QUEUE_PARTS, lgrid);
+    // room for the points of a part's blocks (the last chunk's grid is never larger)
+    const long long part_cap = ordered ? chunk
+                                       : (long long)((lgrid + parts - 1) / parts) * ((ptiles + lgrid - 1) / lgrid) *
+                                             (TPB * LOC_UNROLL);
+    if (part_cap * parts > 0xFFFFFFFFll) {
+        set_error("query queue of %lld places", part_cap * parts);
+        return GAHHG_ERR_CAPACITY;
+    }
+    const size_t qcap = (size_t)part_cap * parts;
+    // Words: [control: overflow flag at 0, order flag at 1, entries per window at +64, windows'
+    // cursors at +128, queue counts from CTL_QUEUE, tier 2's from CTL_TIER2]
+    // [queue of points in leaves: points, leaf words][FP32 filter: tier 2's
+    // queue: points, leaf words, masks][with an order: the ordered queue][leaf order: entries
+    // per leaf: nb][leaf starts: nb + 1][tile sums][ranks].
+    constexpr size_t CTL_QUEUE = 192, CTL_TIER2 = CTL_QUEUE + QUEUE_PARTS * COUNTER_STRIDE,
+                     CTL_WORDS = CTL_TIER2 + QUEUE_PARTS * COUNTER_STRIDE;
+    const PartQueue q2parts = tier2_parts(chunk, nullptr);
+    const size_t cap2 = fp64 ? 0 : (size_t)q2parts.parts * q2parts.cap;
     const int nb = leaves ? (int)g->lattice->nleaves + 1 : 0;
     const int tiles = (nb + LS_TILE - 1) / LS_TILE;
-    const size_t l1_at = (size_t)chunk + 192;
-    // even, so that the leaf order's (point, leaf word) pairs are 8-byte aligned
-    const size_t sorted_at = (l1_at + (size_t)chunk + 3 * (size_t)cap2 + 2 * (size_t)cap3 + 1) & ~(size_t)1;
-    const size_t ls_at = sorted_at + 2 * (size_t)chunk;
-    const size_t words = windows ? ls_at : leaves ? ls_at + 2 * (size_t)nb + 1 + tiles + (size_t)chunk : sorted_at;
-    uint32_t* queue = nullptr;
-    GAHHG_TRY(pool_alloc((void**)&queue, sizeof(uint32_t) * words, g->device, s));
-    unsigned int* qcount = (unsigned int*)(queue + chunk + 32);
-    Tiers T;
-    T.cnt = qcount + 1;
-    T.l1 = queue + l1_at;
-    T.q2 = T.l1 + chunk;
-    T.l2 = T.q2 + cap2;
-    T.q3 = T.l2 + cap2;
-    T.l3 = T.q3 + cap3;
-    T.m2 = T.l3 + cap3;
-    T.cap2 = cap2;
-    T.cap3 = cap3;
-    PartScratch W;
-    W.done = qcount + 4;
-    W.total = queue + chunk + 64;
-    W.cursor = queue + chunk + 128;
-    W.spts = queue + sorted_at;
-    W.sleaf = queue + sorted_at + chunk;
-    W.np = Q.nparts;
-    W.scale = Q.part_scale;
-    LeafSortScratch LS;
-    LS.done = qcount + 4;
-    LS.sent = (uint2*)(queue + sorted_at);
-    LS.cnt = queue + ls_at;
-    LS.start = LS.cnt + nb;
-    LS.tsum = LS.start + nb + 1;
-    LS.rank = LS.tsum + tiles;
-    LS.nb = nb;
-    LS.tiles = tiles;
-    LS.stage = order == 3;
-    const gahhg_status st = lattice_query_with(Q, d_lonlat, (long long)n, d_labels, precision, s, d_counters,
-                                               queue, qcount, chunk, g->device, &T, windows ? &W : nullptr,
-                                               leaves ? &LS : nullptr);
-    cudaFreeAsync(queue, s);
-    return st;
-}
-
-// tiers == nullptr: one pass-2 launch with escalations inline (no queues
-// beyond the pass-2 queue); else qcount[1..3] are the tier counters.
-gahhg_status lattice_query_with(const QueryView& Q, const double* d_lonlat, long long n, uint8_t* d_labels,
-                                int precision, cudaStream_t s, uint64_t* d_counters, uint32_t* queue,
-                                unsigned int* qcount, long long chunk, int device, const Tiers* tiers,
-                                const PartScratch* part, const LeafSortScratch* lsort)
-{
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    unsigned long long* ctr = (unsigned long long*)d_counters;
-    for (long long off = 0; off < n; off += chunk) {
-        const int m = (int)std::min<long long>(chunk, n - off);
+    size_t words = CTL_WORDS;
+    auto take = [&words](size_t k) {
+        const size_t at = words;
+        words += (k + 1) & ~(size_t)1;  // even: pairs are 8-byte aligned
+        return at;
+    };
+    const size_t q2 = take(cap2), l2 = take(cap2), m2 = take(cap2);
+    const size_t q1 = take(qcap), l1 = take(qcap);
+    const size_t so = take(ordered ? 2 * (size_t)chunk : 0);
+    const size_t lc = take(nb), ls = take(leaves ? nb + 1 : 0), lt = take(tiles), lr = take(leaves ? chunk : 0);
+    uint32_t* mem = nullptr;
+    GAHHG_TRY(pool_alloc((void**)&mem, sizeof(uint32_t) * words, g->device, s));
+    gahhg_status st = GAHHG_OK;
+    for (long long off = 0; off < (long long)n && st == GAHHG_OK; off += chunk) {
+        const int m = (int)std::min<long long>(chunk, (long long)n - off);
         const double2* ll = (const double2*)d_lonlat + off;
-        // the queue fill, the tier counters and, when ordering by window, the
-        // flag, the counts and the cursors (the control words run up to them)
-        const size_t zero_words = part ? (size_t)(part->cursor + PART_MAX - qcount) : lsort ? 5 : (tiers ? 4 : 1);
-        GAHHG_CUDA_TRY(cudaMemsetAsync(qcount, 0, sizeof(unsigned int) * zero_words, s));
-        if (lsort) GAHHG_CUDA_TRY(cudaMemsetAsync(lsort->cnt, 0, sizeof(unsigned int) * lsort->nb, s));
-        const long long tiles = ((long long)m + TPB * LOC_UNROLL - 1) / (TPB * LOC_UNROLL);
-        const int grid = (int)std::min<long long>(tiles, (long long)sms * 8);
-        uint32_t* leafq = tiers ? tiers->l1 : nullptr;
+        uint8_t* out = d_labels + off;
+        unsigned int* ctl = mem;
+        unsigned int* qc = ctl + CTL_QUEUE;
+        if (cudaMemsetAsync(ctl, 0, sizeof(unsigned int) * CTL_WORDS, s) != cudaSuccess ||
+            (leaves && cudaMemsetAsync(mem + lc, 0, sizeof(unsigned int) * nb, s) != cudaSuccess)) {
+            set_error("query scratch: %s", cudaGetErrorString(cudaGetLastError()));
+            st = GAHHG_ERR_CUDA;
+            break;
+        }
+        Tiers T;
+        T.q2 = mem + q2;
+        T.l2 = mem + l2;
+        T.m2 = mem + m2;
+        T.p2 = q2parts;
+        T.p2.cnt = ctl + CTL_TIER2;
+        T.over = ctl;
+        // the points in leaves, queued with their leaf words
+        uint32_t *queue = mem + q1, *leafq = mem + l1;
+        T.q1 = queue;
+        T.l1 = leafq;
+        T.p1 = PartQueue{qc, parts, (unsigned int)part_cap};
+        const long long mtiles = ((long long)m + TPB * LOC_UNROLL - 1) / (TPB * LOC_UNROLL);
         const int polls = (int)knob(GAHHG_KNOB_STAGING_POLL_LIMIT);
         auto kl = ctr ? k_locate<true> : k_locate<false>;
-        kl<<<grid, TPB, summary_bytes(Q.swords), s>>>(ll, m, d_labels + off, Q, queue, leafq, qcount, ctr, polls);
-        if (tiers && part) {
-            // the pass-1 queue in window order, then the tiers over it
-            launch_dependent_tpb(k_part_count, sms * 4, P_TPB, s, (const uint32_t*)tiers->l1,
-                                 (const unsigned int*)qcount, *part);
-            launch_dependent_tpb(k_part_scatter, sms * 4, P_TPB, s, (const uint32_t*)queue,
-                                 (const uint32_t*)tiers->l1, (const unsigned int*)qcount, *part);
-            Tiers T = *tiers;
-            T.spts = part->spts;
-            T.sleaf = part->sleaf;
-            T.sorted = part->done;
-            leaf_tiers_launch(OneView{Q}, ll, d_labels + off, queue, qcount, T, precision, ctr, sms, s);
-        } else if (tiers && lsort) {
-            // the pass-1 queue in leaf order, then the tiers over it
-            const uint32_t* l1 = tiers->l1;
-            const unsigned int* qc = qcount;
-            launch_dependent_tpb(k_ls_count, sms * 8, LS_TPB, s, l1, qc, *lsort);
-            launch_dependent_tpb(k_ls_tile_sums, std::min(lsort->tiles, sms * 8), LS_TPB, s, qc, *lsort);
-            launch_dependent_tpb(k_ls_scan, std::min(lsort->tiles, sms * 8), LS_TPB, s, qc, *lsort);
-            launch_dependent_tpb(k_ls_scatter, sms * 8, LS_TPB, s, (const uint32_t*)queue, l1, qc, *lsort);
-            Tiers T = *tiers;
-            T.spts = (const uint32_t*)lsort->sent;
-            T.sleaf = T.spts + 1;
-            T.sstride = 2;
-            T.sorted = lsort->done;
-            leaf_tiers_launch(OneView{Q}, ll, d_labels + off, queue, qcount, T, precision, ctr, sms, s,
-                              lsort->stage);
-        } else if (tiers) {
-            leaf_tiers_launch(OneView{Q}, ll, d_labels + off, queue, qcount, *tiers, precision, ctr, sms, s);
+        kl<<<(int)std::min<long long>(mtiles, lgrid), TPB, summary_bytes(Q.swords), s>>>(
+            ll, m, out, Q, queue, leafq, qc, parts, (unsigned int)part_cap, ctr, polls);
+        if (ordered) {
+            // ... put in window or leaf order
+            T.sorted = ctl + 1;
+            if (windows) {
+                PartScratch W;
+                W.done = ctl + 1;
+                W.total = ctl + 64;
+                W.cursor = ctl + 128;
+                W.spts = mem + so;
+                W.sleaf = W.spts + chunk;
+                W.np = Q.nparts;
+                W.scale = Q.part_scale;
+                launch_dependent_tpb(k_part_count, sms * 4, P_TPB, s, (const uint32_t*)T.l1, (const unsigned int*)qc, W);
+                launch_dependent_tpb(k_part_scatter, sms * 4, P_TPB, s, (const uint32_t*)queue, (const uint32_t*)T.l1,
+                                     (const unsigned int*)qc, W);
+                T.spts = W.spts;
+                T.sleaf = W.sleaf;
+            } else {
+                LeafSortScratch LS;
+                LS.done = ctl + 1;
+                LS.sent = (uint2*)(mem + so);
+                LS.cnt = mem + lc;
+                LS.start = mem + ls;
+                LS.tsum = mem + lt;
+                LS.rank = mem + lr;
+                LS.nb = nb;
+                LS.tiles = tiles;
+                const uint32_t* l1p = T.l1;
+                launch_dependent_tpb(k_ls_count, sms * 8, LS_TPB, s, l1p, (const unsigned int*)qc, LS);
+                launch_dependent_tpb(k_ls_tile_sums, std::min(tiles, sms * 8), LS_TPB, s, (const unsigned int*)qc, LS);
+                launch_dependent_tpb(k_ls_scan, std::min(tiles, sms * 8), LS_TPB, s, (const unsigned int*)qc, LS);
+                launch_dependent_tpb(k_ls_scatter, sms * 8, LS_TPB, s, (const uint32_t*)queue, l1p, (const unsigned int*)qc, LS);
+                T.spts = (const uint32_t*)LS.sent;
+                T.sleaf = T.spts + 1;
+                T.sstride = 2;
+            }
         }
-        else if (precision == GAHHG_QUERY_FP64_FILTER)
-            k_leaf<false><<<sms * 4, TPB, 0, s>>>(ll, d_labels + off, Q, queue, qcount, ctr);
-        else
-            k_leaf<true><<<sms * 4, TPB, 0, s>>>(ll, d_labels + off, Q, queue, qcount, ctr);
-        GAHHG_CUDA_TRY(cudaGetLastError());
+        if (!fp64 && leaves && order == 3)
+            launch_dependent(k_leaf_t1s, sms * T1S_BLOCKS, s, Q, ll, out, T, ctr, polls);
+        else if (!fp64)
+            launch_dependent(k_leaf_t1<OneView>, sms * T1_BLOCKS, s, OneView{Q}, ll, out, T, ctr);
+        tier2_launch(OneView{Q}, ll, out, T, precision, ctr, sms, s);
+        if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) {
+            set_error("query launch: %s", cudaGetErrorString(e));
+            st = GAHHG_ERR_CUDA;
+        }
     }
-    return GAHHG_OK;
+    cudaFreeAsync(mem, s);
+    return st;
 }
 
 // ------------------------------------------------- allocation-free query --
 //
-// The same two passes as lattice_query, with the pass-2 queue in a fixed
-// array in device memory instead of memory taken from the pool, for callers
-// that must not allocate (see gahhg_query_device_noalloc in include/gahhg.h).
-// Every device that loads this library reserves the array until the process
-// exits.  All calls share it: calls that overlap on the GPU race.
+// The query with every tier inline takes no scratch at all, so callers that
+// must not allocate (see gahhg_query_device_noalloc in include/gahhg.h) get
+// it at any size up to the entry point's limit.
 
 constexpr long long NOALLOC_MAX_POINTS = 1LL << 21;  // 2,097,152 points per call
-static __device__ __align__(256) uint32_t g_noalloc_queue[NOALLOC_MAX_POINTS + 64];
 
 long long lattice_noalloc_max_points() { return NOALLOC_MAX_POINTS; }
-
-// Device address of the array on the current device (the caller has made
-// g->device current).  In host code `g_noalloc_queue` names a host-side
-// stand-in, never the device array, so the address is asked of the runtime.
-// It is looked up on every call rather than cached: after cudaDeviceReset
-// (or any other teardown of the primary context) the module is loaded again
-// and the array may sit at another address.  The lookup allocates nothing;
-// the first one on a device loads the module there, which is why the first
-// call on a device should come before any stream capture.
-static gahhg_status noalloc_queue_address(int device, uint32_t** out)
-{
-    void* p = nullptr;
-    const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_queue);
-    if (e != cudaSuccess || !p) {
-        set_error("cudaGetSymbolAddress(g_noalloc_queue) on device %d: %s", device, cudaGetErrorString(e));
-        return GAHHG_ERR_CUDA;
-    }
-    *out = (uint32_t*)p;
-    return GAHHG_OK;
-}
 
 gahhg_status lattice_query_noalloc(Grid* g, const double* d_lonlat, size_t n, uint8_t* d_labels, int precision,
                                    cudaStream_t s)
@@ -1743,14 +2183,10 @@ gahhg_status lattice_query_noalloc(Grid* g, const double* d_lonlat, size_t n, ui
         set_error("exact queries read lon/lat in 16-byte units: the device buffer must be 16-byte aligned");
         return GAHHG_ERR_ARG;
     }
-    uint32_t* queue = nullptr;
-    GAHHG_TRY(noalloc_queue_address(g->device, &queue));
     if (n == 0) return GAHHG_OK;
-    const QueryView Q = make_view(g);
-    // the queue count lives after the queue; lattice_query_with zeroes it before each pass
-    unsigned int* qcount = (unsigned int*)(queue + NOALLOC_MAX_POINTS + 32);
-    return lattice_query_with(Q, d_lonlat, (long long)n, d_labels, precision, s, nullptr, queue, qcount,
-                              NOALLOC_MAX_POINTS, g->device, nullptr);
+    query_inline(make_view(g), (const double2*)d_lonlat, (int)n, d_labels, precision, nullptr, sm_count(g->device), s);
+    GAHHG_CUDA_TRY(cudaGetLastError());
+    return GAHHG_OK;
 }
 
 // ------------------------------------------------------- batch launcher --
@@ -1768,15 +2204,18 @@ gahhg_status lattice_staging_fallbacks(int device, unsigned long long* out)
 }
 
 // Chunks of at most `chunk_points` points, segment after segment.
-// A segment's chunks hold at least 16 points per word of its summary, so
-// staging the summary costs at most a quarter byte per point.
+// A segment's chunks hold at least 2 points per word of its summary, so
+// staging the summary costs at most two bytes per point, from L2.  (16 points
+// per word made chunks of 65,536 points, fewer than the blocks of the grid:
+// the SMs stood idle 43 % of the pass, 150 us where 2 per word take 85; 1 and
+// 4 per word 87 and 91.)
 void batch_write_chunks(const long long* offsets, int nseg, int chunk_points, const int* swords, const int* seg_view,
                         void* out, int* nchunks)
 {
     BatchChunk* v = (BatchChunk*)out;
     int n = 0;
     for (int p = 0; p < nseg; p++) {
-        const long long step = std::max<long long>(chunk_points, 16LL * (swords ? swords[p] : 0));
+        const long long step = std::max<long long>(chunk_points, 2LL * (swords ? swords[p] : 0));
         for (long long a = offsets[p]; a < offsets[p + 1]; a += step) {
             BatchChunk c;
             c.view = seg_view ? seg_view[p] : p;
@@ -1837,50 +2276,54 @@ bool batch_shape_info(int shape, int* points_per_thread, int* blocks_per_sm)
     return true;
 }
 
-size_t batch_queue_words(long long queue_cap)
+// [tier 2's counters][points in leaves: points, leaf words][tier 2's queue:
+// points, leaf words, masks][queue counts of the chunks, their prefix sums]
+size_t batch_queue_words(long long queue_cap, long long nchunks)
 {
-    unsigned int cap2 = 0, cap3 = 0;
-    tier_caps(queue_cap, &cap2, &cap3);
-    return 2 * ((size_t)queue_cap + cap2 + cap3) + cap2;
+    const PartQueue p2 = tier2_parts(queue_cap, nullptr);
+    return (size_t)QUEUE_PARTS * COUNTER_STRIDE + 2 * (size_t)queue_cap + 3 * (size_t)p2.parts * p2.cap +
+           2 * (size_t)nchunks + 1;
 }
 
-// counters: [0] queue count, [1] next chunk, [2..4] tier counters.  The
-// queue holds batch_queue_words(queue_cap) words: the pass-2 queue and its
-// leaf words, then the escalation queues, each followed by its leaf words.  Everything is enqueued on `s` (no allocation, no host
-// synchronisation), so it can be captured in a graph.
+// counters: [1] next chunk, [2] overflow flag.  The queue holds
+// batch_queue_words(queue_cap, nchunks) words.  Everything is enqueued on `s` (no
+// allocation, no host synchronisation), so it can be captured in a graph.
 gahhg_status batch_query_launch(const void* d_views, const void* d_chunks, int nchunks, const double* d_lonlat,
                                 uint8_t* d_labels, int precision, uint32_t* queue, long long queue_cap,
                                 unsigned int* counters, uint64_t* d_stats, cudaStream_t s, int device,
                                 bool zero_counters, int shape)
 {
     if (nchunks == 0) return GAHHG_OK;
-    static std::atomic<int> sms_cache[64];
-    int sms = (device >= 0 && device < 64) ? sms_cache[device].load(std::memory_order_relaxed) : 0;
-    if (!sms) {
-        sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        if (device >= 0 && device < 64) sms_cache[device].store(sms, std::memory_order_relaxed);
-    }
+    const int sms = sm_count(device);
     const QueryView* views = (const QueryView*)d_views;
     const BatchChunk* chunks = (const BatchChunk*)d_chunks;
     unsigned long long* ctr = (unsigned long long*)d_stats;
     if (zero_counters) GAHHG_CUDA_TRY(cudaMemsetAsync(counters, 0, 5 * sizeof(unsigned int), s));
+    const bool fp64 = precision == GAHHG_QUERY_FP64_FILTER;
     Tiers T;
-    tier_caps(queue_cap, &T.cap2, &T.cap3);
-    T.l1 = queue + queue_cap;
-    T.q2 = T.l1 + queue_cap;
-    T.l2 = T.q2 + T.cap2;
-    T.q3 = T.l2 + T.cap2;
-    T.l3 = T.q3 + T.cap3;
-    T.m2 = T.l3 + T.cap3;
-    T.cnt = counters + 2;
+    T.p2 = tier2_parts(queue_cap, queue);
+    const size_t cap2 = (size_t)T.p2.parts * T.p2.cap;
+    if (!fp64) GAHHG_CUDA_TRY(cudaMemsetAsync(T.p2.cnt, 0, sizeof(unsigned int) * QUEUE_PARTS * COUNTER_STRIDE, s));
+    uint32_t* q1 = queue + QUEUE_PARTS * COUNTER_STRIDE;
+    T.q1 = q1;
+    T.over = counters + 2;
+    T.l1 = q1 + queue_cap;
+    T.q2 = q1 + 2 * queue_cap;
+    T.l2 = T.q2 + cap2;
+    T.m2 = T.l2 + cap2;
+    unsigned int* ccount = T.m2 + cap2;
+    T.pre = ccount + nchunks;
     const int polls = (int)knob(GAHHG_KNOB_STAGING_POLL_LIMIT);
     if (shape < 0 || shape >= BATCH_NSHAPES) shape = 0;
     const int grid = std::min(nchunks, sms * BATCH_SHAPES[shape].blocks);  // persistent: every block resident
-    batch_locate_launch<0>(shape, grid, s, views, chunks, nchunks, counters + 1, (const double2*)d_lonlat, d_labels,
-                           queue, T.l1, counters, ctr, polls);
-    leaf_tiers_launch(ChunkViews{views, chunks, nchunks}, (const double2*)d_lonlat, d_labels, queue, counters, T,
-                      precision, ctr, sms, s);
+    const double2* ll = (const double2*)d_lonlat;
+    batch_locate_launch<0>(shape, grid, s, views, chunks, nchunks, counters + 1, ll, d_labels, q1, q1 + queue_cap, ccount,
+                           ctr, polls);
+    launch_dependent_tpb(k_chunk_scan, 1, CS_TPB, s, (const unsigned int*)ccount, nchunks, ccount + nchunks);
+    const ChunkViews vs{views, chunks, nchunks};
+    if (!fp64)
+        launch_dependent(k_leaf_t1<ChunkViews>, sms * T1_BLOCKS, s, vs, ll, d_labels, T, ctr);
+    tier2_launch(vs, ll, d_labels, T, precision, ctr, sms, s);
     GAHHG_CUDA_TRY(cudaGetLastError());
     return GAHHG_OK;
 }

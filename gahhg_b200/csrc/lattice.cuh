@@ -47,10 +47,19 @@ constexpr int MAX_LEVEL = 9;
 constexpr long long NODE_BUDGET = 1LL << 27;
 constexpr long long PAIR_BUDGET = 1LL << 30;
 
-// Leaf: its center as the lon/lat it was placed at (R = their canonical XYZ),
-// its edge records' first index (`off`, in the arrays of edge words and of
-// records), its center's label, the sine and cosine of the center's canonical
-// latitude rounded to float (the FP32 tier's frame, local_frame::frame_at).
+// Leaf, 64 bytes (two sectors of one line): its center as the lon/lat it was
+// placed at (R = their canonical XYZ), its edges' first index (`off`, in the
+// arrays of edge words and of records), its center's label, the sine and
+// cosine of the center's canonical latitude rounded to float (the FP32 tier's
+// frame, local_frame::frame_at), and its first two edge records: a leaf of a
+// polyline mostly has one or two edges, so the FP32 tier reads one place per
+// point instead of a leaf and then its records.
+//
+// An edge record is a float4 (a1, a2, b1, b2): the edge's ends in the leaf's
+// tangent frame (local_frame::edge_record), ordered so that orient(A, B, R) =
+// +1.  The edge id and the sign of orient(A, B, R) in the edge's own order are
+// in a parallel array of words (edge | (sign > 0) << 31).
+constexpr int LEAF_INLINE = 2;
 struct __align__(16) LeafRec {
     double lon, lat;
     uint32_t off;
@@ -58,13 +67,24 @@ struct __align__(16) LeafRec {
     uint8_t label;
     uint8_t pad;
     float sb, cb;
+    float4 rec[LEAF_INLINE];  // records 0 and 1; the others are recs[off + k]
 };
-static_assert(sizeof(LeafRec) == 32, "LeafRec");
+static_assert(sizeof(LeafRec) == 64, "LeafRec");
 
-// (leaf, edge) records of the FP32 tier: float4 (a1, a2, b1, b2), the edge's
-// ends in the leaf's tangent frame (local_frame::edge_record), ordered so that
-// orient(A, B, R) = +1.  The edge id and the sign of orient(A, B, R) in the
-// edge's own order are in a parallel array of words (edge | (sign > 0) << 31).
+// What the FP64 tier needs of a leaf, 128 bytes (one line): the center's
+// canonical XYZ as the query would compute it, the leaf's counts again, and
+// the FP64 ends of its first two edges (ax ay az bx by bz), so that a point of
+// a leaf with one or two edges reads one line instead of leaf, edge words and
+// ends one after the other.
+struct __align__(128) LeafAux {
+    double R[3];
+    uint32_t off;
+    uint16_t cnt;
+    uint8_t label;
+    uint8_t signs;  // bit k: orient(A, B, R) > 0 for edge k
+    double ends[LEAF_INLINE][6];
+};
+static_assert(sizeof(LeafAux) == 128, "LeafAux");
 
 // Level-0 grid over a lon/lat domain: W x H cells of dlon0 x dlat0 degrees
 // starting at (lon0, lat0).  full_lon: the domain spans all longitudes
@@ -174,18 +194,23 @@ struct QueryView {
     double U360;              // cells per 360 degrees of longitude
     int full_lon, to_north, to_south;
     uint32_t outside;         // label outside the domain (pure node word)
-    int cshift;               // coarse cell = (1 << cshift) x (1 << cshift) top cells
-    int CW;                   // coarse columns
-    int swords;               // 32-bit words of the coarse summary
-    const uint32_t* summary;  // 2 bits per coarse cell: 0 out, 1 in, 2 mixed
+    // the coarse summary: 2 bits per coarse cell (blocks of 2^cshift x
+    // 2^cshift top cells): the label of a cell without edges, 0 for the others.
+    // A ring of cells around the domain holds the outside's label (where the
+    // domain goes round or reaches a pole, its last cells' codes again), so a
+    // lookup clamps to the ring instead of testing the domain's sides:
+    // column = lon * cu + cu0 (+ cu360 below 1 when cwrap), row = lat * cv + cv0
+    double cu, cu0, cu360, cv, cv0;
+    int cwrap;
+    int SW, SH;               // cells of the summary, the ring included
+    int swords;               // 32-bit words of the summary
+    const uint32_t* summary;
     const uint32_t* nodes;
     const LeafRec* leaves;
-    const float4* recs;       // per record: the FP32 tier's tangent-frame ends
+    const float4* recs;       // per record (from the third of a leaf): the FP32 tier's tangent-frame ends
     const uint32_t* eids;     // per record: edge id | (orient(A, B, R) > 0) << 31
     const double2* ends;      // per edge: A.xy, A.z B.x, B.yz (48 B, one aligned load each)
-    const double* leafR;      // per leaf: the center's canonical XYZ (3 doubles), as leaf_label computes it
-    const D3* pv;
-    const int* pe;
+    const LeafAux* aux;       // per leaf
     int nparts;               // windows of consecutive leaves the pass-2 queue is ordered by (1: none)
     float part_scale;         // window of leaf i: floor(i * part_scale), clamped to nparts - 1
 };
@@ -208,17 +233,31 @@ inline void set_view_geo(QueryView& Q, const Geo& g)
 }
 
 // Coarse summary shape of a level-0 grid: cells of 2^cshift x 2^cshift top
-// cells, at most 65,536 of them (16 KB of 2-bit codes).
-inline void summary_shape(int W, int H, int* cshift, int* CW, int* CH)
+// cells and the ring around them, at most 65,536 in all (16 KB of 2-bit codes).
+inline void summary_shape(int W, int H, int* cshift, int* SW, int* SH)
 {
     int cs = 0;
-    auto blocks = [&](int c) { return (long long)((W + (1 << c) - 1) >> c) * ((H + (1 << c) - 1) >> c); };
-    while (blocks(cs) > 65536) cs++;
+    auto side = [&](int n, int c) { return (long long)((n + (1 << c) - 1) >> c) + 2; };
+    while (side(W, cs) * side(H, cs) > 65536) cs++;
     *cshift = cs;
-    *CW = (W + (1 << cs) - 1) >> cs;
-    *CH = (H + (1 << cs) - 1) >> cs;
+    *SW = (int)side(W, cs);
+    *SH = (int)side(H, cs);
 }
 
+// The coarse lookup of a view (set_view_geo done).
+inline void set_view_coarse(QueryView& Q, const Geo& g, int cshift, int SW, int SH)
+{
+    const double f = (double)(1 << cshift);
+    Q.SW = SW;
+    Q.SH = SH;
+    const double lon0 = !g.full_lon && g.lon0 < -180.0 ? g.lon0 + 360.0 : g.lon0;  // in [-180, 180)
+    Q.cu = Q.su_lon / f;
+    Q.cu0 = 1.0 - lon0 * Q.cu;
+    Q.cu360 = 360.0 * Q.cu;
+    Q.cwrap = !g.full_lon && lon0 + g.W * g.dlon0 > 180.0;
+    Q.cv = Q.su_lat / f;
+    Q.cv0 = 1.0 - g.lat0 * Q.cv;
+}
 
 // The exact indexes of the polygons of one build.
 struct LatticeSet {
@@ -230,7 +269,7 @@ struct LatticeSet {
     DevArray<float4> recs;
     DevArray<uint32_t> eids;
     DevArray<double2> ends;
-    DevArray<double> leafR;
+    DevArray<LeafAux> aux;
     DevArray<uint32_t> summary;
     std::vector<QueryView> views;  // per polygon
     std::vector<int> swords;       // per polygon: words of its summary

@@ -1638,7 +1638,7 @@ __global__ void __launch_bounds__(TPB) k_child_exact(const double2* __restrict__
 __global__ void __launch_bounds__(TPB) k_leaf_records(const double2* __restrict__ ends, LevelView v,
                                                       const PolyGeo* __restrict__ pg, const int* __restrict__ lnode,
                                                       int nleaf, int leaf_base, long long rec_base, LeafRec* leaves,
-                                                      float4* recs, uint32_t* eids, double* leafR, int* bad)
+                                                      float4* recs, uint32_t* eids, LeafAux* aux, int* bad)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nleaf) return;
@@ -1669,15 +1669,19 @@ __global__ void __launch_bounds__(TPB) k_leaf_records(const double2* __restrict_
         L.sb = (float)sb;
         L.cb = (float)cb;
     }
-    leaves[leaf_base + i] = L;
-    // the center's canonical XYZ, bit for bit as the query would compute it
-    double* dst = leafR + 3 * (size_t)(leaf_base + i);
-    dst[0] = c.R[0];
-    dst[1] = c.R[1];
-    dst[2] = c.R[2];
     if (n > 65535) atomicAdd(bad + 2, 1);
     local_frame::Basis fb;
     local_frame::basis_at(c.lonc, c.latc, fb);
+    LeafAux X;
+    for (int k = 0; k < 3; k++) X.R[k] = c.R[k];
+    for (int k = 0; k < LEAF_INLINE; k++) {
+        L.rec[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < 6; j++) X.ends[k][j] = 0.0;
+    }
+    X.off = L.off;
+    X.cnt = L.cnt;
+    X.label = L.label;
+    X.signs = 0;
     for (int k = 0; k < n; k++) {
         const int e = list[k];
         D3 a, b;
@@ -1687,38 +1691,63 @@ __global__ void __launch_bounds__(TPB) k_leaf_records(const double2* __restrict_
         if (s1 == 0) atomicAdd(bad, 1);
         float r[4];
         local_frame::edge_record(A, B, fb, s1 < 0, r);
-        recs[ro + k] = make_float4(r[0], r[1], r[2], r[3]);
-        eids[ro + k] = (uint32_t)e | (s1 > 0 ? 0x80000000u : 0u);
+        const float4 rec = make_float4(r[0], r[1], r[2], r[3]);
+        const uint32_t word = (uint32_t)e | (s1 > 0 ? 0x80000000u : 0u);
+        if (k < LEAF_INLINE) {
+            L.rec[k] = rec;
+            for (int j = 0; j < 3; j++) {
+                X.ends[k][j] = A[j];
+                X.ends[k][3 + j] = B[j];
+            }
+            if (s1 > 0) X.signs |= (uint8_t)(1u << k);
+        } else {
+            recs[ro + k] = rec;
+        }
+        eids[ro + k] = word;
     }
+    leaves[leaf_base + i] = L;
+    aux[leaf_base + i] = X;
 }
 
-// Coarse summary of the top level: a coarse cell whose top cells are all
-// edge-free with one label gets that label, otherwise "mixed".  Coarse cell c
-// of polygon p (sc[p]: its first cell in the set) goes into its summary words
-// from soff[p].
-__global__ void k_summary(const uint32_t* nodes, const PolyGeo* __restrict__ pg, const long long* __restrict__ sc,
-                          const int* __restrict__ cshift, const long long* __restrict__ soff, int np,
+// Coarse summaries (QueryView): cell c of polygon p (sc[p]: its first cell in
+// the set) goes into its summary words from soff[p].  Four lanes share a
+// cell's rows.
+__global__ void k_summary(const uint32_t* __restrict__ nodes, const PolyGeo* __restrict__ pg,
+                          const long long* __restrict__ sc, const int* __restrict__ cshift,
+                          const long long* __restrict__ soff, int np, const uint8_t* __restrict__ outside,
                           uint32_t* summary)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long t = u >> 2;
     if (t >= sc[np]) return;
     const int p = find_range(sc, np, t);
     const int c = (int)(t - sc[p]);
-    const int W = pg[p].g.W, H = pg[p].g.H, cs = cshift[p];
+    const Geo& g = pg[p].g;
+    const int W = g.W, H = g.H, cs = cshift[p];
     const int f = 1 << cs;
-    const int CW = (W + f - 1) >> cs;
-    const int cx = c % CW, cy = c / CW;
-    const uint32_t* top = nodes + pg[p].top;
-    uint32_t code = 0xFFu;
-    for (int y = cy * f; y < min((cy + 1) * f, H) && code != 2u; y++)
-        for (int x = cx * f; x < min((cx + 1) * f, W); x++) {
-            const uint32_t w = top[(size_t)y * W + x];
-            const uint32_t v = ((w & KIND_MASK) == KIND_PURE) ? (w & 3u) - 1u : 2u;  // 0 out, 1 in, 2 mixed
-            if (code == 0xFFu) code = v;
-            else if (code != v) code = 2u;
-            if (code == 2u) break;
-        }
-    atomicOr(&summary[soff[p] + (c >> 4)], code << ((c & 15) * 2));
+    const int CW = (W + f - 1) >> cs, CH = (H + f - 1) >> cs;
+    int cx = c % (CW + 2) - 1, cy = c / (CW + 2) - 1;
+    uint32_t code = 3u;  // bits seen: 1 an out cell, 2 an in cell, 4 a cell with edges
+    // the ring: the domain's last cells where it goes round or reaches a pole
+    if (g.full_lon) cx = min(max(cx, 0), CW - 1);
+    if (g.to_south) cy = max(cy, 0);
+    if (g.to_north) cy = min(cy, CH - 1);
+    if (cx < 0 || cx >= CW || cy < 0 || cy >= CH) {
+        code = outside[p];
+    } else {
+        const uint32_t* top = nodes + pg[p].top;
+        uint32_t seen = 0;
+        for (int y = cy * f + (int)(u & 3); y < min((cy + 1) * f, H); y += 4)
+            for (int x = cx * f; x < min((cx + 1) * f, W); x++) {
+                const uint32_t w = top[(size_t)y * W + x];
+                seen |= (w & KIND_MASK) == KIND_PURE ? (w & 3u) : 4u;
+            }
+        const unsigned int grp = 0xFu << (threadIdx.x & 28);
+        seen |= __shfl_xor_sync(grp, seen, 1);
+        seen |= __shfl_xor_sync(grp, seen, 2);
+        code = seen == 1u || seen == 2u ? seen : 0u;
+    }
+    if ((u & 3) == 0 && code) atomicOr(&summary[soff[p] + (c >> 4)], code << ((c & 15) * 2));
 }
 
 }  // namespace
@@ -1850,13 +1879,13 @@ void LatticeSet::release()
     recs.release();
     eids.release();
     ends.release();
-    leafR.release();
+    aux.release();
     summary.release();
 }
 
 long long LatticeSet::bytes() const
 {
-    return nnodes * (long long)sizeof(uint32_t) + nleaves * (long long)(sizeof(LeafRec) + 3 * sizeof(double)) +
+    return nnodes * (long long)sizeof(uint32_t) + nleaves * (long long)(sizeof(LeafRec) + sizeof(LeafAux)) +
            nrecs * (long long)(sizeof(float4) + sizeof(uint32_t)) + nedges * 3 * (long long)sizeof(double2);
 }
 
@@ -1864,7 +1893,7 @@ long long LatticeSet::device_bytes() const
 {
     return (long long)(pv.cap * sizeof(D3) + pe.cap * sizeof(int) + nodes.cap * sizeof(uint32_t) +
                        leaves.cap * sizeof(LeafRec) + recs.cap * sizeof(float4) + eids.cap * sizeof(uint32_t) +
-                       ends.cap * sizeof(double2) + leafR.cap * sizeof(double) + summary.cap * sizeof(uint32_t));
+                       ends.cap * sizeof(double2) + aux.cap * sizeof(LeafAux) + summary.cap * sizeof(uint32_t));
 }
 
 namespace {
@@ -2314,7 +2343,7 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
     GAHHG_TRY(L->leaves.alloc(leaf_total + 1, s));
     GAHHG_TRY(L->recs.alloc(rec_total, s));
     GAHHG_TRY(L->eids.alloc(rec_total, s));
-    GAHHG_TRY(L->leafR.alloc(3 * (size_t)leaf_total, s));
+    GAHHG_TRY(L->aux.alloc(leaf_total, s));
     for (int lvl = 0; lvl < nlev; lvl++) {
         const LevelBuf& b = lv[lvl];
         GAHHG_CUDA_TRY(cudaMemcpyAsync(L->nodes.ptr + b.gstart, b.words.ptr, sizeof(uint32_t) * b.nn,
@@ -2323,18 +2352,16 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
             k_leaf_records<<<blocks_for(b.sums.leaves), TPB, 0, s>>>(ends, view(lvl), d_pg.ptr, b.lnode.ptr,
                                                                      b.sums.leaves, leaf_base[lvl], rec_base[lvl],
                                                                      L->leaves.ptr, L->recs.ptr, L->eids.ptr,
-                                                                     L->leafR.ptr, bad);
+                                                                     L->aux.ptr, bad);
     }
     // coarse summaries, each polygon's from a 16-byte aligned word
     std::vector<long long> sc(np + 1, 0), soff(np + 1, 0);
-    std::vector<int> cshift(np);
+    std::vector<int> cshift(np), SW(np), SH(np);
     L->swords.resize(np);
     for (int p = 0; p < np; p++) {
-        int cs, CW, CH;
-        summary_shape(pg[p].g.W, pg[p].g.H, &cs, &CW, &CH);
-        cshift[p] = cs;
-        L->swords[p] = (CW * CH + 15) / 16;
-        sc[p + 1] = sc[p] + (long long)CW * CH;
+        summary_shape(pg[p].g.W, pg[p].g.H, &cshift[p], &SW[p], &SH[p]);
+        L->swords[p] = (SW[p] * SH[p] + 15) / 16;
+        sc[p + 1] = sc[p] + (long long)SW[p] * SH[p];
         soff[p + 1] = soff[p] + ((L->swords[p] + 3) & ~3);
     }
     {
@@ -2345,8 +2372,8 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
         GAHHG_TRY(upload(d_cshift, cshift, s));
         // (a bulk copy of a summary reads up to its 16-byte multiple, inside soff's padding)
         GAHHG_TRY(alloc_zero(L->summary, soff[np], s));
-        k_summary<<<blocks_for(sc[np]), TPB, 0, s>>>(L->nodes.ptr, d_pg.ptr, d_sc.ptr, d_cshift.ptr, d_soff.ptr, np,
-                                                     L->summary.ptr);
+        k_summary<<<blocks_for(4 * sc[np]), TPB, 0, s>>>(L->nodes.ptr, d_pg.ptr, d_sc.ptr, d_cshift.ptr, d_soff.ptr, np,
+                                                         outl.ptr, L->summary.ptr);
     }
     GAHHG_CUDA_TRY(cudaGetLastError());
     // ---- the last round trip: failures, origins, outside labels
@@ -2390,11 +2417,8 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
         Q.recs = L->recs.ptr;
         Q.eids = L->eids.ptr;
         Q.ends = L->ends.ptr;
-        Q.leafR = L->leafR.ptr;
-        Q.pv = pv;
-        Q.pe = pe;
-        Q.cshift = cshift[p];
-        Q.CW = (pg[p].g.W + (1 << cshift[p]) - 1) >> cshift[p];
+        Q.aux = L->aux.ptr;
+        set_view_coarse(Q, pg[p].g, cshift[p], SW[p], SH[p]);
         Q.swords = L->swords[p];
         Q.summary = L->summary.ptr + soff[p];
         Q.nparts = 1;  // leaf windows: single-polygon queries set them

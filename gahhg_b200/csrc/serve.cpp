@@ -636,7 +636,7 @@ struct gahhg_server {
             GAHHG_CUDA_TRY(cudaEventCreate(&s.ev));
             GAHHG_CUDA_TRY(cudaHostAlloc((void**)&s.h, lcap + in_bytes, cudaHostAllocDefault));
             GAHHG_CUDA_TRY(cudaMalloc((void**)&s.d, lcap + in_bytes));
-            GAHHG_CUDA_TRY(cudaMalloc((void**)&s.d_queue, sizeof(uint32_t) * batch_queue_words(o.slot_points)));
+            GAHHG_CUDA_TRY(cudaMalloc((void**)&s.d_queue, sizeof(uint32_t) * batch_queue_words(o.slot_points, (long long)cap_chunks)));
         }
         GAHHG_TRY(workers.create(o.device, o.build_workers, lo));
         if (o.hbm_budget <= 0) {
