@@ -217,6 +217,7 @@ struct Grid {
     bool hierarchy = false;
     std::mutex hierarchy_mu;
 
+    Grid();
     ~Grid();
 };
 
