@@ -88,14 +88,18 @@ GHD bool project(const Frame& f, const D3& A, double& x, double& y)
 // line), so a rectangle over corners and, where dl = 0 lies between them, the
 // middles of the parallels, covers the cell; a rectangle covers the hull of
 // what it covers.
-GHD void corner(double sa, double ca, double dl, double dp, double& x, double& y)
+GHD void corner_at(double sa, double ca, double sl, double h, double sp, double cp, double& x, double& y)
 {
-    const double sp = sin(dp), cp = cos(dp), h = sin(0.5 * dl);
     const double cphi = ca * cp - sa * sp;
     const double v = 2.0 * h * h;  // 1 - cos dl
     const double i = 1.0 / (cp - ca * cphi * v);
-    x = cphi * sin(dl) * i;
+    x = cphi * sl * i;
     y = (sp + sa * cphi * v) * i;
+}
+
+GHD void corner(double sa, double ca, double dl, double dp, double& x, double& y)
+{
+    corner_at(sa, ca, sin(dl), sin(0.5 * dl), sin(dp), cos(dp), x, y);
 }
 
 // A rectangle [x0, x1] x [y0, y1] in the plane.
@@ -126,16 +130,10 @@ GHD Box own_box(double sa, double ca, double hl, double hp)
     return b;
 }
 
-// The cell at angle differences [l0, l1] x [p0, p1] from the center, l0 and
-// l1 on one side of it (a child of the 4 x 4 split never straddles its
-// parent's center).
-GHD Box offset_box(double sa, double ca, double l0, double l1, double p0, double p1)
+// The rectangle over four corners of a cell on one side of the center in
+// longitude (a child of the 4 x 4 split never straddles its parent's center).
+GHD Box corners_box(double xa, double ya, double xb, double yb, double xc, double yc, double xd, double yd)
 {
-    double xa, ya, xb, yb, xc, yc, xd, yd;
-    corner(sa, ca, l0, p0, xa, ya);
-    corner(sa, ca, l1, p0, xb, yb);
-    corner(sa, ca, l0, p1, xc, yc);
-    corner(sa, ca, l1, p1, xd, yd);
     Box b;
     b.x0 = fmin(fmin(xa, xb), fmin(xc, xd)) - MARGIN;
     b.x1 = fmax(fmax(xa, xb), fmax(xc, xd)) + MARGIN;
@@ -144,34 +142,63 @@ GHD Box offset_box(double sa, double ca, double l0, double l1, double p0, double
     return b;
 }
 
-// May segment a-b (projected edge ends) meet the rectangle?  Never false for
-// one that does.
-GHD bool meets(double ax, double ay, double bx, double by, const Box& b)
+// A projected edge, with what its tests share.
+struct alignas(16) Segment {
+    double ax, ay, bx, by;  // the ends
+    double x0, x1, y0, y1;  // around them
+    double dx, dy;          // b - a
+    double c1;              // side of the center
+    double n;               // magnitudes |a| + |b| + |d|
+};
+
+GHD Segment segment(double ax, double ay, double bx, double by)
 {
-    if (fmax(ax, bx) < b.x0 || fmin(ax, bx) > b.x1 || fmax(ay, by) < b.y0 || fmin(ay, by) > b.y1) return false;
-    const double cx = 0.5 * (b.x0 + b.x1), cy = 0.5 * (b.y0 + b.y1);
-    const double dx = bx - ax, dy = by - ay, ux = ax - cx, uy = ay - cy;
-    const double adx = fabs(dx), ady = fabs(dy);
-    const double side = fabs(ux * dy - uy * dx);
-    const double reach = (b.x1 - cx) * ady + (b.y1 - cy) * adx;
-    return side <= reach + ERR * (adx + ady + fabs(ux) + fabs(uy));
+    Segment s;
+    s.ax = ax;
+    s.ay = ay;
+    s.bx = bx;
+    s.by = by;
+    s.x0 = fmin(ax, bx);
+    s.x1 = fmax(ax, bx);
+    s.y0 = fmin(ay, by);
+    s.y1 = fmax(ay, by);
+    s.dx = bx - ax;
+    s.dy = by - ay;
+    s.c1 = ax * s.dy - ay * s.dx;
+    s.n = fabs(ax) + fabs(ay) + fabs(bx) + fabs(by) + fabs(s.dx) + fabs(s.dy);
+    return s;
 }
 
-// Does segment a-b cross the segment from the origin (the center) to q?  1 or
-// 0 when the signs of the four orientations are certain, -1 otherwise.
+// May the segment meet the rectangle?  Never false for one that does.
+GHD bool meets(const Segment& s, const Box& b)
+{
+    if (s.x1 < b.x0 || s.x0 > b.x1 || s.y1 < b.y0 || s.y0 > b.y1) return false;
+    const double cx = 0.5 * (b.x0 + b.x1), cy = 0.5 * (b.y0 + b.y1);
+    const double ux = s.ax - cx, uy = s.ay - cy;
+    const double side = fabs(ux * s.dy - uy * s.dx);
+    const double reach = (b.x1 - cx) * fabs(s.dy) + (b.y1 - cy) * fabs(s.dx);
+    return side <= reach + ERR * (s.n + fabs(ux) + fabs(uy));
+}
+
+GHD bool meets(double ax, double ay, double bx, double by, const Box& b) { return meets(segment(ax, ay, bx, by), b); }
+
+// Does the segment cross the one from the origin (the center) to q?  1 or 0
+// when the signs of the four orientations are certain, -1 otherwise.  One
+// bound serves all four (the largest of theirs).
+GHD int crosses_from_center(const Segment& s, double qx, double qy)
+{
+    const double e = ERR * (s.n + (fabs(qx) + fabs(qy)));
+    const double c2 = s.c1 + (s.dx * qy - s.dy * qx);  // side of q
+    const double c3 = qx * s.ay - qy * s.ax, c4 = qx * s.by - qy * s.bx;
+    const bool p1 = s.c1 > e, n1 = s.c1 < -e, p2 = c2 > e, n2 = c2 < -e;
+    const bool p3 = c3 > e, n3 = c3 < -e, p4 = c4 > e, n4 = c4 < -e;
+    if ((p1 & p2) | (n1 & n2) | (p3 & p4) | (n3 & n4)) return 0;
+    return (p1 | n1) & (p2 | n2) & (p3 | n3) & (p4 | n4) ? 1 : -1;
+}
+
 GHD int crosses_from_center(double ax, double ay, double bx, double by, double qx, double qy)
 {
-    const double dx = bx - ax, dy = by - ay;
-    const double na = fabs(ax) + fabs(ay), nb = fabs(bx) + fabs(by), nd = fabs(dx) + fabs(dy), nq = fabs(qx) + fabs(qy);
-    const double c1 = ax * dy - ay * dx;           // side of the center
-    const double c2 = c1 + (dx * qy - dy * qx);    // side of q
-    const double c3 = qx * ay - qy * ax, c4 = qx * by - qy * bx;
-    const double e1 = ERR * (na + nd), e2 = ERR * (na + nd + nq), e3 = ERR * (nq + na), e4 = ERR * (nq + nb);
-    const int s1 = c1 > e1 ? 1 : (c1 < -e1 ? -1 : 0), s2 = c2 > e2 ? 1 : (c2 < -e2 ? -1 : 0);
-    const int s3 = c3 > e3 ? 1 : (c3 < -e3 ? -1 : 0), s4 = c4 > e4 ? 1 : (c4 < -e4 ? -1 : 0);
-    if (s1 * s2 > 0 || s3 * s4 > 0) return 0;
-    if (s1 * s2 < 0 && s3 * s4 < 0) return 1;
-    return -1;
+    return crosses_from_center(segment(ax, ay, bx, by), qx, qy);
 }
 
 }  // namespace cellbox

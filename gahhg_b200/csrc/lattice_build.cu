@@ -1385,99 +1385,93 @@ __global__ void k_encode(LevelView v, const PolyGeo* __restrict__ pg, int child_
 }
 
 // A child as the pair pass takes it, in its parent's projection plane: the
-// rectangle around the cell (x0 > x1: the level uses caps) and the center.
-struct ChildRec {
+// rectangle around the cell and the center.
+struct ChildLane {
+    cellbox::Frame f;  // the parent's
+    bool boxes;        // false: the level uses caps
     cellbox::Box box;
     double qx, qy;
+    uint2 ixy;
 };
 
-// Children of the refined nodes: coordinates, polygon, rectangle; the
-// parent's frame (by its first child).
-__global__ void k_child_boxes(LevelView v, const PolyGeo* __restrict__ pg, const int* __restrict__ rnode, int nref,
-                              uint2* cixy, int* cpoly, ChildRec* child, cellbox::Frame* frame)
+constexpr int KIDS = FAN * FAN;
+constexpr int CORNERS = (FAN + 1) * (FAN + 1);
+
+// Child l of node p, by the 16 lanes of half a warp together: the children's
+// rows and columns share their sines and cosines and their corners, so a lane
+// takes one center's row or column, one border's, and two of the 25 corners,
+// which `s_pt` passes on.
+__device__ __forceinline__ ChildLane child_lane(const LevelView& v, const PolyGeo& P, int p, int l, double2* s_pt)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = t >> 4, l = t & 15;
-    if (r >= nref) return;
-    const int p = rnode[r];
-    const int poly = poly_of(v.npoly, p);
-    const PolyGeo& P = pg[poly];
+    constexpr unsigned int ALL = 0xffffffffu;
     const Geo& g = P.g;
     long long ix, iy;
     node_xy(v, P, p, ix, iy);
     const int cx = l & (FAN - 1), cy = l / FAN;
-    const long long jx = ix * FAN + cx, jy = iy * FAN + cy;
-    cixy[t] = make_uint2((unsigned)jx, (unsigned)jy);
-    if (cpoly) cpoly[t] = poly;
+    ChildLane c;
+    c.ixy = make_uint2((unsigned)(ix * FAN + cx), (unsigned)(iy * FAN + cy));
     const double sc = level_scale(v.lvl), sc1 = level_scale(v.lvl + 1);
-    const cellbox::Frame f = cellbox::frame_at(g.lon0 + ((double)ix + 0.5) * (g.dlon0 / sc),
-                                               g.lat0 + ((double)iy + 0.5) * (g.dlat0 / sc));
-    if (l == 0) frame[r] = f;
-    ChildRec c;
-    c.box = cellbox::Box{1.0, -1.0, 1.0, -1.0};
+    // lanes 0, 1: the parent's latitude and longitude; 2..5 columns, 6..9 rows
+    double deg = g.lat0 + ((double)iy + 0.5) * (g.dlat0 / sc);
+    if (l == 1) deg = g.lon0 + ((double)ix + 0.5) * (g.dlon0 / sc);
+    if (l >= 2) deg = g.lon0 + ((double)(ix * FAN + (l - 2)) + 0.5) * (g.dlon0 / sc1);
+    if (l >= 2 + FAN) deg = g.lat0 + ((double)(iy * FAN + min(l - 2 - FAN, FAN - 1)) + 0.5) * (g.dlat0 / sc1);
+    double sn, cs;
+    gahhg_canon_sincos(gahhg_canon_rad(deg), &sn, &cs);
+    c.f.sa = __shfl_sync(ALL, sn, 0, KIDS);
+    c.f.ca = __shfl_sync(ALL, cs, 0, KIDS);
+    c.f.so = __shfl_sync(ALL, sn, 1, KIDS);
+    c.f.co = __shfl_sync(ALL, cs, 1, KIDS);
+    const double so = __shfl_sync(ALL, sn, 2 + cx, KIDS), co = __shfl_sync(ALL, cs, 2 + cx, KIDS);
+    const double sa = __shfl_sync(ALL, sn, 2 + FAN + cy, KIDS), ca = __shfl_sync(ALL, cs, 2 + FAN + cy, KIDS);
     c.qx = c.qy = 0.0;
     double hl, hp;
-    if (level_boxes(g, v.lvl, hl, hp)) {
-        c.box = cellbox::offset_box(f.sa, f.ca, (cx - 2) * 0.5 * hl, (cx - 1) * 0.5 * hl, (cy - 2) * 0.5 * hp,
-                                    (cy - 1) * 0.5 * hp);
-        double q[3];
-        gahhg_canon_vertex_xyz(g.lon0 + ((double)jx + 0.5) * (g.dlon0 / sc1),
-                               g.lat0 + ((double)jy + 0.5) * (g.dlat0 / sc1), q);
-        cellbox::project(f, d3(q[0], q[1], q[2]), c.qx, c.qy);
+    c.boxes = level_boxes(g, v.lvl, hl, hp);
+    if (c.boxes) cellbox::project(c.f, d3(ca * so, sa, ca * co), c.qx, c.qy);
+    // lanes 0..4: the rows' borders, 5..9: the columns', at half the angle
+    sincos(l <= FAN ? (l - 2) * 0.5 * hp : (min(l - 1 - FAN, FAN) - 2) * 0.25 * hl, &sn, &cs);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int j = min(l + KIDS * k, CORNERS - 1), row = j / (FAN + 1), col = j - row * (FAN + 1);
+        const double sp = __shfl_sync(ALL, sn, row, KIDS), cp = __shfl_sync(ALL, cs, row, KIDS);
+        const double h = __shfl_sync(ALL, sn, FAN + 1 + col, KIDS), ch = __shfl_sync(ALL, cs, FAN + 1 + col, KIDS);
+        double2 q;
+        cellbox::corner_at(c.f.sa, c.f.ca, 2.0 * h * ch, h, sp, cp, q.x, q.y);
+        s_pt[j] = q;
     }
-    child[t] = c;
+    __syncwarp();
+    const double2* t = s_pt + cy * (FAN + 1) + cx;
+    const double2 q0 = t[0], q1 = t[1], q2 = t[FAN + 1], q3 = t[FAN + 2];
+    c.box = cellbox::corners_box(q0.x, q0.y, q1.x, q1.y, q2.x, q2.y, q3.x, q3.y);
+    __syncwarp();  // s_pt may be rewritten
+    return c;
 }
 
-// One edge of a refined node against its 16 children: bits of `hit` it is
-// listed in the child, of `cross` it crosses the arc from the parent's center
-// to the child's, of `unsure` that is not certain.
-__device__ __forceinline__ void child_tests(const D3& A, const D3& B, const cellbox::Frame& f, const ChildRec* child,
-                                            const Geo& g, int lvl, uint2 ixy0, unsigned int& hit, unsigned int& cross,
-                                            unsigned int& unsure)
-{
-    hit = cross = unsure = 0;
-    double ax, ay, bx, by;
-    if (child[0].box.x0 <= child[0].box.x1 && cellbox::project(f, A, ax, ay) && cellbox::project(f, B, bx, by)) {
-#pragma unroll 4
-        for (int l = 0; l < FAN * FAN; l++) {
-            const ChildRec c = child[l];
-            if (cellbox::meets(ax, ay, bx, by, c.box)) hit |= 1u << l;
-            const int x = cellbox::crosses_from_center(ax, ay, bx, by, c.qx, c.qy);
-            if (x > 0) cross |= 1u << l;
-            if (x < 0) unsure |= 1u << l;
-        }
-        return;
-    }
-    // cells too wide for a rectangle, or an edge too long to project: caps
-    // around the children, exact labels
-    unsure = 0xFFFFu;
-    for (int l = 0; l < FAN * FAN; l++) {
-        const NodeCap c = node_cap(g, lvl + 1, (long long)ixy0.x + (l & (FAN - 1)), (long long)ixy0.y + l / FAN);
-        if (edge_hits_cap(A, B, c.R, c.r)) hit |= 1u << l;
-    }
-}
-
-// The pair pass: every edge of a refined node against its children.  A warp
-// takes a node, a lane an edge (32 at a time): the hits go to hit[] (for the
-// fill), and ballots over the lanes give the children's counts and crossing
-// parities without atomics.  Nodes with more than PAIR_LONG edges are handed
-// to k_child_pairs_long, where a block takes each, so that no warp works on
-// one node for long.  Both the list test and the label's crossing test are a
-// few operations in the parent's plane once the edge is projected; the
-// predicates on XYZ that they replace loaded and crossed every edge again for
-// each child's label (4072 us for the 1.1M-edge polygon's four levels, and
-// 1945 us of cap tests).
+// The pair pass: every edge of a refined node against its 16 children, in the
+// list and across the arc between the centers.  Half a warp takes a node, a
+// lane a child: the lanes project 16 edges at a time into shared memory, then
+// each tests its child against them one after the other.  A ballot gives an
+// edge's hits (for the fill), and a child's count and crossing parity stay in
+// its lane.  The tests' FP64 instructions bound the pass (two thirds of the
+// issue slots), so what an edge's tests share is made once (Segment).  A warp
+// per node and a lane per edge left two thirds of the lanes idle (refined
+// nodes of the 1.1M-edge polygon have about ten edges) and took 16 ballots a
+// step besides: 655 us for its four levels, and 187 for a pass before that
+// wrote the children's rectangles, which the lanes make here: 506 for both
+// (six blocks per SM; four 631, eight 513, ten 558).
+//
+// Nodes with more than PAIR_LONG edges are handed to k_child_pairs_long, where
+// a block takes each, so that no warp works on one node for long.
 constexpr int PAIR_LONG = 256;
-constexpr int PAIR_WARPS = 4;
+constexpr int PAIR_TPB = 128;
 
 struct PairArgs {
     const double2* ends;
     const PolyGeo* pg;
     const int* rnode;
     int nref;
-    const uint2* cixy;
-    const ChildRec* child;
-    const cellbox::Frame* frame;
+    uint2* cixy;
+    int* cpoly;  // null for one polygon
     uint16_t* hit;
     int* ccnt;
     uint8_t* cpar;  // bit 0: parity of the center arc, bit 1: not certain
@@ -1485,91 +1479,111 @@ struct PairArgs {
     int* nlong;
 };
 
-__device__ __forceinline__ void pair_steps(const PairArgs& a, const LevelView& v, const ChildRec* child, int r, int p,
-                                           int first, int step, int& count, unsigned int& par, unsigned int& uns)
+// Edges first, first + 1, ... (16 of them), first + step, ... of a list of n
+// at `start`, by the half warp whose lanes hold the children `c`.  Both halves
+// of a warp step together.
+__device__ __forceinline__ void pair_steps(const PairArgs& a, const LevelView& v, const ChildLane& c, const Geo& g,
+                                           cellbox::Segment* s_edge, int start, int n, int first, int step, int& count,
+                                           unsigned int& par, unsigned int& uns)
 {
-    const int lane = threadIdx.x & 31;
-    const int n = v.cnt[p], start = v.off[p];
-    const cellbox::Frame f = a.frame[r];
-    const Geo& g = a.pg[poly_of(v.npoly, p)].g;
-    const uint2 ixy0 = a.cixy[FAN * FAN * (size_t)r];
-    for (int k0 = first; k0 < n; k0 += step) {
-        const int k = k0 + lane;
-        unsigned int m = 0, x = 0, u = 0;
-        if (k < n) {
+    constexpr unsigned int ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, l = lane & (KIDS - 1);
+    for (int k0 = first; __any_sync(ALL, k0 < n); k0 += step) {
+        const int m = max(0, min(KIDS, n - k0));
+        bool ok = false;
+        if (l < m) {
             D3 A, B;
-            load_edge(a.ends, v.list[start + k], A, B);
-            child_tests(A, B, f, child, g, v.lvl, ixy0, m, x, u);
-            a.hit[start + k] = (uint16_t)m;
+            load_edge(a.ends, v.list[start + k0 + l], A, B);
+            double ax, ay, bx, by;
+            ok = c.boxes && cellbox::project(c.f, A, ax, ay) && cellbox::project(c.f, B, bx, by);
+            if (ok) s_edge[l] = cellbox::segment(ax, ay, bx, by);
         }
-#pragma unroll
-        for (int l = 0; l < FAN * FAN; l++) {
-            const int c = __popc(__ballot_sync(0xffffffffu, (m >> l) & 1u));
-            if (lane == l) count += c;
+        const unsigned int planar = __ballot_sync(ALL, ok) >> (lane & KIDS);
+        __syncwarp();
+        const int most = __reduce_max_sync(ALL, m);
+        unsigned int mine = 0;
+        for (int k = 0; k < most; k++) {
+            bool hit = false;
+            if (k < m) {
+                if ((planar >> k) & 1u) {
+                    const cellbox::Segment e = s_edge[k];
+                    hit = cellbox::meets(e, c.box);
+                    const int x = cellbox::crosses_from_center(e, c.qx, c.qy);
+                    par ^= x > 0;
+                    uns |= x < 0;
+                } else {
+                    // cells too wide for a rectangle, or an edge too long to
+                    // project: caps around the children, exact labels
+                    D3 A, B;
+                    load_edge(a.ends, v.list[start + k0 + k], A, B);
+                    const NodeCap cap = node_cap(g, v.lvl + 1, (long long)c.ixy.x, (long long)c.ixy.y);
+                    hit = edge_hits_cap(A, B, cap.R, cap.r);
+                    uns = 1;
+                }
+            }
+            const unsigned int hits = (__ballot_sync(ALL, hit) >> (lane & KIDS)) & 0xffffu;
+            count += hit;
+            if (l == k) mine = hits;
         }
-        par ^= __reduce_xor_sync(0xffffffffu, x);
-        uns |= __reduce_or_sync(0xffffffffu, u);
+        if (l < m) a.hit[start + k0 + l] = (uint16_t)mine;
+        __syncwarp();  // s_edge is rewritten
     }
 }
 
-__global__ void __launch_bounds__(PAIR_WARPS * 32) k_child_pairs(PairArgs a, LevelView v)
+__global__ void __launch_bounds__(PAIR_TPB, 6) k_child_pairs(PairArgs a, LevelView v)
 {
-    __shared__ ChildRec s_child[PAIR_WARPS][FAN * FAN];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int r = blockIdx.x * PAIR_WARPS + warp;
-    if (r >= a.nref) return;
+    __shared__ cellbox::Segment s_edge[PAIR_TPB];
+    __shared__ double2 s_pt[PAIR_TPB / KIDS][CORNERS];
+    const int l = threadIdx.x & (KIDS - 1);
+    const long long t = (long long)blockIdx.x * PAIR_TPB + threadIdx.x;
+    const bool node = t < (long long)KIDS * a.nref;
+    const int r = node ? (int)(t / KIDS) : a.nref - 1;  // (halves beyond the last node repeat it, without edges)
     const int p = a.rnode[r];
-    if (v.cnt[p] > PAIR_LONG) {
-        if (lane == 0) a.longs[atomicAdd(a.nlong, 1)] = r;
-        return;
-    }
-    {
-        const double* src = (const double*)(a.child + FAN * FAN * (size_t)r);
-        double* dst = (double*)s_child[warp];
-        for (int k = lane; k < (int)(FAN * FAN * sizeof(ChildRec) / sizeof(double)); k += 32) dst[k] = src[k];
-    }
-    __syncwarp();
+    const int poly = poly_of(v.npoly, p);
+    const PolyGeo& P = a.pg[poly];
+    const ChildLane c = child_lane(v, P, p, l, s_pt[threadIdx.x / KIDS]);
+    const int len = v.cnt[p];
+    const bool here = node && len <= PAIR_LONG;
     int count = 0;
     unsigned int par = 0, uns = 0;
-    pair_steps(a, v, s_child[warp], r, p, 0, 32, count, par, uns);
-    if (lane < FAN * FAN) {
-        const size_t c = FAN * FAN * (size_t)r + lane;
-        a.ccnt[c] = count;
-        a.cpar[c] = (uint8_t)(((par >> lane) & 1u) | (((uns >> lane) & 1u) << 1));
+    pair_steps(a, v, c, P.g, s_edge + (threadIdx.x & ~(KIDS - 1)), v.off[p], here ? len : 0, 0, KIDS, count, par, uns);
+    if (!node) return;
+    a.cixy[t] = c.ixy;
+    if (a.cpoly) a.cpoly[t] = poly;
+    if (here) {
+        a.ccnt[t] = count;
+        a.cpar[t] = (uint8_t)(par | uns << 1);
+    } else if (l == 0) {
+        a.longs[atomicAdd(a.nlong, 1)] = r;
     }
 }
 
 __global__ void __launch_bounds__(TPB) k_child_pairs_long(PairArgs a, LevelView v)
 {
-    __shared__ ChildRec s_child[FAN * FAN];
-    __shared__ int s_cnt[FAN * FAN];
-    __shared__ unsigned int s_par, s_uns;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ cellbox::Segment s_edge[TPB];
+    __shared__ double2 s_pt[TPB / KIDS][CORNERS];
+    __shared__ int s_cnt[KIDS];
+    __shared__ unsigned int s_par[KIDS];
+    const int l = threadIdx.x & (KIDS - 1), half = threadIdx.x / KIDS;
     const int m = *a.nlong;
     for (int i = blockIdx.x; i < m; i += gridDim.x) {
-        const int r = a.longs[i];
+        const int r = a.longs[i], p = a.rnode[r];
         __syncthreads();
-        {
-            const double* src = (const double*)(a.child + FAN * FAN * (size_t)r);
-            double* dst = (double*)s_child;
-            for (int k = threadIdx.x; k < (int)(FAN * FAN * sizeof(ChildRec) / sizeof(double)); k += TPB) dst[k] = src[k];
-        }
-        if (threadIdx.x < FAN * FAN) s_cnt[threadIdx.x] = 0;
-        if (threadIdx.x == 0) s_par = s_uns = 0;
+        if (threadIdx.x < KIDS) s_cnt[threadIdx.x] = s_par[threadIdx.x] = 0;
         __syncthreads();
+        const PolyGeo& P = a.pg[poly_of(v.npoly, p)];
+        const ChildLane c = child_lane(v, P, p, l, s_pt[threadIdx.x / KIDS]);
         int count = 0;
         unsigned int par = 0, uns = 0;
-        pair_steps(a, v, s_child, r, a.rnode[r], warp * 32, TPB, count, par, uns);
-        if (lane < FAN * FAN && count) atomicAdd(&s_cnt[lane], count);
-        if (lane == 0) {
-            atomicXor(&s_par, par);
-            atomicOr(&s_uns, uns);
-        }
+        pair_steps(a, v, c, P.g, s_edge + half * KIDS, v.off[p], v.cnt[p], half * KIDS, TPB, count, par, uns);
+        if (count) atomicAdd(&s_cnt[l], count);
+        if (par) atomicXor(&s_par[l], 1u);
+        if (uns) atomicOr(&s_par[l], 2u);
         __syncthreads();
-        if (threadIdx.x < FAN * FAN) {
-            const size_t c = FAN * FAN * (size_t)r + threadIdx.x;
-            a.ccnt[c] = s_cnt[threadIdx.x];
-            a.cpar[c] = (uint8_t)(((s_par >> threadIdx.x) & 1u) | (((s_uns >> threadIdx.x) & 1u) << 1));
+        if (threadIdx.x < KIDS) {
+            const size_t o = KIDS * (size_t)r + threadIdx.x;
+            a.ccnt[o] = s_cnt[threadIdx.x];
+            a.cpar[o] = (uint8_t)s_par[threadIdx.x];
         }
     }
 }
@@ -2302,23 +2316,17 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
         c.nn = nref * FAN * FAN;
         c.gstart = (int)gnext;
         gnext += c.nn;
-        DevArray<ChildRec> child;
-        DevArray<cellbox::Frame> frame;
         DevArray<int> longs;
         GAHHG_TRY(c.ixy.alloc(c.nn, s));
         if (np > 1) GAHHG_TRY(c.poly.alloc(c.nn, s));
         GAHHG_TRY(c.cnt.alloc(c.nn, s));
         GAHHG_TRY(c.cpar.alloc(c.nn, s));
-        GAHHG_TRY(child.alloc(c.nn, s));
-        GAHHG_TRY(frame.alloc(nref, s));
         GAHHG_TRY(longs.alloc((size_t)b.sums.pairs / (PAIR_LONG + 1) + 1, s));
         GAHHG_TRY(b.hit.alloc(b.sums.pairs, s));
         GAHHG_CUDA_TRY(cudaMemsetAsync(w->sort, 0, sizeof w->sort, s));
-        k_child_boxes<<<blocks_for(c.nn), TPB, 0, s>>>(v, d_pg.ptr, b.rnode.ptr, nref, c.ixy.ptr, c.poly.ptr, child.ptr,
-                                                       frame.ptr);
-        const PairArgs a{ends, d_pg.ptr, b.rnode.ptr, nref, c.ixy.ptr, child.ptr, frame.ptr, b.hit.ptr, c.cnt.ptr,
+        const PairArgs a{ends, d_pg.ptr, b.rnode.ptr, nref, c.ixy.ptr, c.poly.ptr, b.hit.ptr, c.cnt.ptr,
                          c.cpar.ptr, longs.ptr, w->sort};
-        k_child_pairs<<<(nref + PAIR_WARPS - 1) / PAIR_WARPS, PAIR_WARPS * 32, 0, s>>>(a, v);
+        k_child_pairs<<<(c.nn + PAIR_TPB - 1) / PAIR_TPB, PAIR_TPB, 0, s>>>(a, v);
         k_child_pairs_long<<<sms * 2, TPB, 0, s>>>(a, v);
         GAHHG_CUDA_TRY(cudaGetLastError());
         GAHHG_TRY(scan(lvl + 1, lvl + 1 >= MAX_LEVEL));
