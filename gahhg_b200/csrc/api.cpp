@@ -104,6 +104,10 @@ gahhg_status Polygon::upload(cudaStream_t s, int device)
     GAHHG_CUDA_TRY(cudaMalloc(&d_pe, sizeof(int) * 2 * pv_num));
     GAHHG_CUDA_TRY(cudaMemcpy(d_pv, pv.data(), sizeof(D3) * pv_num, cudaMemcpyHostToDevice));
     GAHHG_CUDA_TRY(cudaMemcpy(d_pe, pe.data(), sizeof(int) * 2 * pv_num, cudaMemcpyHostToDevice));
+    // a copy from pageable memory returns when the host memory has been read,
+    // which can be before the device's has been written, and the streams that
+    // read these arrays do not wait for the legacy stream
+    GAHHG_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
     return GAHHG_OK;
 }
 
