@@ -111,7 +111,7 @@ gahhg_status WorkerPool::create(int device, int n, int priority)
     scans.assign(n, nullptr);
     for (int w = 0; w < n; w++) {
         if (cudaStreamCreateWithPriority(&streams[w], cudaStreamNonBlocking, priority) != cudaSuccess ||
-            scan_state_reserve(&scans[w], 1u << 26) != GAHHG_OK) {
+            scan_state_reserve(&scans[w], 1u << 22, streams[w]) != GAHHG_OK) {
             set_error("worker stream or scan state creation failed");
             return GAHHG_ERR_CUDA;
         }
@@ -167,10 +167,6 @@ gahhg_status gahhg_batch_build(const gahhg_polygon* const* polys, int count, con
     // group builds keep the GPU busy with a few workers; more only add scratch memory
     int nw = workers > 0 ? workers : (int)std::min(4u, std::max(1u, std::thread::hardware_concurrency()));
     nw = std::min(nw, count);
-    if (B->pool.create(B->device, nw) != GAHHG_OK) {
-        delete B;
-        return GAHHG_ERR_CUDA;
-    }
     const double t0 = now_seconds();
     // The workers' groups allocate and free their scratch concurrently: a
     // pool that trims its cache at every synchronisation would return it to
@@ -197,6 +193,11 @@ gahhg_status gahhg_batch_build(const gahhg_polygon* const* polys, int count, con
         gstart.push_back(count);
     }
     const int ngroups = (int)gstart.size() - 1;
+    // (a stream and a scan state for every worker that gets a group)
+    if (B->pool.create(B->device, std::min(nw, ngroups)) != GAHHG_OK) {
+        delete B;
+        return GAHHG_ERR_CUDA;
+    }
     B->groups.assign(ngroups, nullptr);
     {
         std::atomic<int> next(0), bad(-1);

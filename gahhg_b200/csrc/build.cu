@@ -17,7 +17,7 @@
 
 namespace gahhg {
 
-gahhg_status scan_state_reserve(void** state, size_t max_n);
+gahhg_status scan_state_reserve(void** state, size_t max_n, cudaStream_t s);
 void scan_state_destroy(void* state);
 
 namespace {
@@ -428,7 +428,7 @@ static gahhg_status div_grid(Grid* g, int L, bool* more)
     GAHHG_TRY(g->off_a.reserve(lv.cnum, s, false));
     GAHHG_TRY(g->off_b.reserve(lv.cnum, s, false));
     k_center_offsets<<<blocks_for(lv.cnum), TPB, 0, s>>>(g->C.ptr, lv.cstart, lv.cnum, g->cell_a.ptr, g->cell_b.ptr);
-    GAHHG_TRY(scan_state_reserve(&g->scan_state, lv.cnum));
+    GAHHG_TRY(scan_state_reserve(&g->scan_state, lv.cnum, s));
     GAHHG_TRY(scan_exclusive(g->cell_a.ptr, g->off_a.ptr, lv.cnum, g->d_counts + HC_SUM_A, g->scan_state, g->d_err, s));
     GAHHG_TRY(scan_exclusive(g->cell_b.ptr, g->off_b.ptr, lv.cnum, g->d_counts + HC_SUM_B, g->scan_state, g->d_err, s));
     GAHHG_CUDA_TRY(cudaGetLastError());
@@ -467,7 +467,7 @@ static gahhg_status div_grid(Grid* g, int L, bool* more)
     GAHHG_TRY(g->off_b.reserve(sumA, s, false));
     k_border_sc_offsets<<<blocks_for(sumA), TPB, 0, s>>>(g->B.ptr, g->C.ptr, nl.bstart, sumA, g->cell_a.ptr,
                                                          g->cell_b.ptr);
-    GAHHG_TRY(scan_state_reserve(&g->scan_state, sumA));
+    GAHHG_TRY(scan_state_reserve(&g->scan_state, sumA, s));
     GAHHG_TRY(scan_exclusive(g->cell_a.ptr, g->off_a.ptr, sumA, g->d_counts + HC_SUM_A2, g->scan_state, g->d_err, s));
     GAHHG_TRY(scan_exclusive(g->cell_b.ptr, g->off_b.ptr, sumA, g->d_counts + HC_SUM_B2, g->scan_state, g->d_err, s));
     k_create_border_sc<<<blocks_for(sumA), TPB, 0, s>>>(g->V.ptr, g->B.ptr, nl.bstart, sumA, g->C.ptr, nl.cstart,
@@ -498,7 +498,7 @@ static gahhg_status dispatch_last(Grid* g)
 
     k_edge_refs<WALK_COUNT><<<blocks_for(n), TPB, 0, s>>>(P->d_pv, P->d_pe, n, gv, level, g->levels[0].cnum, buf,
                                                          g->edge_cnt.ptr, nullptr, nullptr, g->d_err);
-    GAHHG_TRY(scan_state_reserve(&g->scan_state, n));
+    GAHHG_TRY(scan_state_reserve(&g->scan_state, n, s));
     GAHHG_TRY(scan_exclusive(g->edge_cnt.ptr, g->edge_off.ptr, n, g->d_counts + HC_REFS, g->scan_state, g->d_err, s));
     GAHHG_TRY(read_counts(g));
     const int R = g->h_counts[HC_REFS];
@@ -511,7 +511,7 @@ static gahhg_status dispatch_last(Grid* g)
                                                          g->edge_cnt.ptr, g->edge_off.ptr, g->ref_cell.ptr, g->d_err);
     GAHHG_CUDA_TRY(cudaMemsetAsync(g->ref_flag.ptr, 0, sizeof(int) * ((size_t)R + 1), s));
     k_edge_flags<<<blocks_for(n), TPB, 0, s>>>(g->edge_off.ptr, n, g->ref_flag.ptr, R);
-    GAHHG_TRY(scan_state_reserve(&g->scan_state, R));
+    GAHHG_TRY(scan_state_reserve(&g->scan_state, R, s));
     GAHHG_TRY(scan_exclusive(g->ref_flag.ptr, g->ref_edge.ptr, R, g->d_counts + HC_SUM_A, g->scan_state, g->d_err, s));
     k_add<<<blocks_for(R), TPB, 0, s>>>(g->ref_flag.ptr, g->ref_edge.ptr, R);
 
@@ -521,7 +521,7 @@ static gahhg_status dispatch_last(Grid* g)
     GAHHG_TRY(g->cell_b.reserve(cn, s, false));
     GAHHG_CUDA_TRY(cudaMemsetAsync(g->cell_a.ptr, 0, sizeof(int) * cn, s));
     k_count_per_cell<<<blocks_for(R), TPB, 0, s>>>(g->ref_cell.ptr, R, last.cstart, cn, g->cell_a.ptr, g->d_err);
-    GAHHG_TRY(scan_state_reserve(&g->scan_state, cn));
+    GAHHG_TRY(scan_state_reserve(&g->scan_state, cn, s));
     GAHHG_TRY(scan_exclusive(g->cell_a.ptr, g->off_a.ptr, cn, g->d_counts + HC_SUM_B, g->scan_state, g->d_err, s));
     GAHHG_CUDA_TRY(cudaMemcpyAsync(g->cell_b.ptr, g->off_a.ptr, sizeof(int) * cn, cudaMemcpyDeviceToDevice, s));
     k_scatter_refs<<<blocks_for(R), TPB, 0, s>>>(g->ref_cell.ptr, g->ref_edge.ptr, R, last.cstart, cn, g->cell_b.ptr,

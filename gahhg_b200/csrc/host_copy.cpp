@@ -2,6 +2,7 @@
 #include "host_copy.h"
 
 #include <algorithm>
+#include <chrono>
 #include <cstring>
 #include <new>
 
@@ -10,6 +11,15 @@
 #endif
 
 namespace gahhg {
+
+namespace {
+
+double now_seconds()
+{
+    return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
+}
+
+}  // namespace
 
 void copy_for_device(void* to, const void* from, size_t bytes)
 {
@@ -140,6 +150,7 @@ void CopyTeam::finish(bool abort)
 
 namespace {
 std::mutex g_stage_mu;
+std::condition_variable g_stage_cv;
 HostStage* g_stage = nullptr;  // never destroyed at exit: its threads may outlive static objects
 bool g_stage_busy = false;
 long long g_grids = 0;
@@ -174,12 +185,13 @@ bool HostStage::pageable(const void* host)
     return at.type == cudaMemoryTypeUnregistered;
 }
 
-HostStage* HostStage::acquire(int dev, const void* host, size_t bytes)
+HostStage* HostStage::acquire(int dev, const void* host, size_t bytes, bool wait)
 {
     if (bytes < MIN_BYTES || CopyTeam::default_workers() == 0) return nullptr;
     if (!pageable(host)) return nullptr;
-    std::lock_guard<std::mutex> lk(g_stage_mu);
-    if (g_stage_busy) return nullptr;
+    std::unique_lock<std::mutex> lk(g_stage_mu);
+    if (g_stage_busy && !wait) return nullptr;
+    g_stage_cv.wait(lk, [] { return !g_stage_busy; });
     if (!g_stage) {
         HostStage* s = new (std::nothrow) HostStage();
         if (!s) return nullptr;
@@ -212,8 +224,12 @@ void HostStage::release(HostStage* s)
 {
     if (!s) return;
     s->settle();  // the next user writes the ring, maybe from another device
-    std::lock_guard<std::mutex> lk(g_stage_mu);
-    g_stage_busy = false;
+    {
+        std::lock_guard<std::mutex> lk(g_stage_mu);
+        g_stage_busy = false;
+        s->used = now_seconds();
+    }
+    g_stage_cv.notify_one();
 }
 
 void HostStage::grid_made()
@@ -227,7 +243,8 @@ void HostStage::grid_gone()
     HostStage* gone = nullptr;
     {
         std::lock_guard<std::mutex> lk(g_stage_mu);
-        if (--g_grids == 0 && !g_stage_busy) std::swap(gone, g_stage);
+        if (--g_grids == 0 && !g_stage_busy && g_stage && now_seconds() - g_stage->used > KEEP_SECONDS)
+            std::swap(gone, g_stage);
     }
     delete gone;
 }
@@ -242,12 +259,37 @@ cudaError_t HostStage::settle()
 
 cudaError_t HostStage::to_device(void* d, const void* h, size_t bytes, cudaStream_t s)
 {
+    return fill(d, bytes, s, [h](size_t from, uint8_t* to, size_t n) { copy_for_device(to, (const uint8_t*)h + from, n); });
+}
+
+cudaError_t HostStage::to_device(void* d, const std::vector<Part>& parts, cudaStream_t s)
+{
+    std::vector<size_t> end(parts.size());
+    size_t bytes = 0;
+    for (size_t i = 0; i < parts.size(); i++) end[i] = bytes += parts[i].bytes;
+    return fill(d, bytes, s, [&](size_t from, uint8_t* to, size_t n) {
+        size_t k = std::upper_bound(end.begin(), end.end(), from) - end.begin();
+        while (n > 0) {
+            const size_t at = from - (end[k] - parts[k].bytes), m = std::min(n, parts[k].bytes - at);
+            copy_for_device(to, (const uint8_t*)parts[k].host + at, m);
+            from += m;
+            to += m;
+            n -= m;
+            k++;
+        }
+    });
+}
+
+// read(from, to, n): bytes [from, from + n) of the source
+cudaError_t HostStage::fill(void* d, size_t bytes, cudaStream_t s,
+                            const std::function<void(size_t, uint8_t*, size_t)>& read)
+{
     cudaError_t e = settle();
     if (e != cudaSuccess || bytes == 0) return e;
     const size_t n = (bytes + SLOT - 1) / SLOT;
     const auto end_of = [&](size_t i) { return std::min(bytes, i * SLOT); };
-    team.post(n, SLOTS, [=](size_t i) {
-        copy_for_device(ring + (i % SLOTS) * SLOT, (const uint8_t*)h + i * SLOT, std::min(SLOT, bytes - i * SLOT));
+    team.post(n, SLOTS, [=, &read](size_t i) {
+        read(i * SLOT, ring + (i % SLOTS) * SLOT, std::min(SLOT, bytes - i * SLOT));
     });
     size_t sent = 0, freed = 0;        // slices enqueued; slices whose copies have ended
     size_t run_end[SLOTS];             // by event: the end of the run it follows

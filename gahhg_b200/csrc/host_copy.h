@@ -66,8 +66,10 @@ private:
 // Pageable host memory <-> device through a ring of page-locked slots that a
 // team fills or empties while the copies of other slots run.  There is one per
 // process, made by the first call that needs it and given back when the last
-// grid goes; a call that finds it in use, or host memory that is page-locked
-// already, copies directly.
+// grid goes, unless it was in use within KEEP_SECONDS before (programs that
+// build, ask and drop one index after another would allocate it each time).  A
+// query that finds it in use, or host memory that is page-locked already, is
+// copied directly.
 class HostStage {
 public:
     // 6 MB page-locked (3.7 ms to allocate).  48 MB to the device in 1.15 ms
@@ -78,26 +80,36 @@ public:
     // than waking the threads costs.
     static constexpr size_t MIN_BYTES = 4 << 20;
 
-    // The process's stage for the calling thread, or null.
-    static HostStage* acquire(int device, const void* host, size_t bytes);
+    // The process's stage for the calling thread, or null; with `wait` a call
+    // that finds it in use waits for its turn.
+    static HostStage* acquire(int device, const void* host, size_t bytes, bool wait = false);
     static bool pageable(const void* host);
     static void release(HostStage* s);
+    static constexpr double KEEP_SECONDS = 2.0;
     static void grid_made();
     static void grid_gone();
 
-    // Enqueued on `s` when it returns; `h` has been read.
+    // Enqueued on `s` when it returns; the host memory has been read.  The
+    // second form: arrays that lie one behind the other on the device.
+    struct Part {
+        const void* host;
+        size_t bytes;
+    };
     cudaError_t to_device(void* d, const void* h, size_t bytes, cudaStream_t s);
+    cudaError_t to_device(void* d, const std::vector<Part>& parts, cudaStream_t s);
     // `h` has been written when it returns.
     cudaError_t to_host(void* h, const void* d, size_t bytes, cudaStream_t s);
     ~HostStage();
 
 private:
     bool create();
+    cudaError_t fill(void* d, size_t bytes, cudaStream_t s, const std::function<void(size_t, uint8_t*, size_t)>& read);
     cudaError_t settle();  // the ring's last copies have ended
     CopyTeam team;
     uint8_t* ring = nullptr;
     cudaEvent_t ev[SLOTS] = {};
     int device = -1;
+    double used = 0.0;
     int last = -1;  // event of the last copy enqueued
 };
 

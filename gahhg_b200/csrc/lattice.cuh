@@ -262,8 +262,6 @@ inline void set_view_coarse(QueryView& Q, const Geo& g, int cshift, int SW, int 
 // The exact indexes of the polygons of one build.
 struct LatticeSet {
     int count = 0;
-    DevArray<D3> pv;  // the set's vertices and edges, unless they are a polygon's own device copies
-    DevArray<int> pe;
     DevArray<uint32_t> nodes;
     DevArray<LeafRec> leaves;
     DevArray<float4> recs;

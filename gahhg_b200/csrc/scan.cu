@@ -29,6 +29,7 @@ constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 struct ScanState {
     unsigned long long* status;
     unsigned int* counter;
+    cudaStream_t stream;
     size_t max_tiles;
     unsigned int tile_base;
     unsigned int epoch;
@@ -141,64 +142,44 @@ size_t scan_state_bytes(size_t n)
     return sizeof(ScanState) + 256 + tiles * sizeof(unsigned long long);
 }
 
-// `state` points to a host-side ScanState allocated by scan_state_create.
-gahhg_status scan_state_create(void** state, size_t max_n)
-{
-    ScanState* st = new ScanState();
-    st->max_tiles = (max_n + SCAN_TILE - 1) / SCAN_TILE + 1;
-    if (cudaMalloc(&st->status, st->max_tiles * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&st->counter, sizeof(unsigned int)) != cudaSuccess) {
-        set_error("scan state allocation failed");
-        delete st;
-        return GAHHG_ERR_NOMEM;
-    }
-    cudaMemset(st->status, 0, st->max_tiles * sizeof(unsigned long long));
-    cudaMemset(st->counter, 0, sizeof(unsigned int));
-    st->tile_base = 0;
-    st->epoch = 1;
-    *state = st;
-    return GAHHG_OK;
-}
-
+// Status and counter come from the library's pool, ordered on the stream that
+// the scans run on (cudaMalloc and cudaFree took 100 us each, and a batch or a
+// hierarchy build makes a state).
 void scan_state_destroy(void* state)
 {
     ScanState* st = (ScanState*)state;
     if (!st) return;
-    cudaFree(st->status);
-    cudaFree(st->counter);
+    if (st->status) cudaFreeAsync(st->status, st->stream);
+    if (st->counter) cudaFreeAsync(st->counter, st->stream);
     delete st;
 }
 
-gahhg_status scan_state_reserve(void** state, size_t max_n)
+gahhg_status scan_state_reserve(void** state, size_t max_n, cudaStream_t s)
 {
+    const size_t need = (max_n + SCAN_TILE - 1) / SCAN_TILE + 1;
     ScanState* st = (ScanState*)*state;
-    size_t need = (max_n + SCAN_TILE - 1) / SCAN_TILE + 1;
     if (st && st->max_tiles >= need) return GAHHG_OK;
-    // growing: the new array starts cleared and the epoch sequence continues
-    unsigned int epoch = st ? st->epoch : 1, base = st ? st->tile_base : 0;
-    unsigned int* counter = st ? st->counter : nullptr;
-    if (st) {
-        cudaFree(st->status);
-        st->status = nullptr;
-    } else {
+    int dev = 0;
+    GAHHG_CUDA_TRY(cudaGetDevice(&dev));
+    if (!st) {
         st = new ScanState();
-        if (cudaMalloc(&counter, sizeof(unsigned int)) != cudaSuccess) {
-            delete st;
-            set_error("scan state allocation failed");
-            return GAHHG_ERR_NOMEM;
-        }
-        cudaMemset(counter, 0, sizeof(unsigned int));
+        st->status = nullptr;
+        st->counter = nullptr;
+        st->stream = s;
+        st->max_tiles = 0;
+        st->epoch = 1;
+        st->tile_base = 0;
+        *state = st;
+        GAHHG_TRY(pool_alloc((void**)&st->counter, sizeof(unsigned int), dev, s));
+        GAHHG_CUDA_TRY(cudaMemsetAsync(st->counter, 0, sizeof(unsigned int), s));
     }
-    st->max_tiles = need * 2;
-    if (cudaMalloc(&st->status, st->max_tiles * sizeof(unsigned long long)) != cudaSuccess) {
-        set_error("scan state allocation failed");
-        return GAHHG_ERR_NOMEM;
-    }
-    cudaMemset(st->status, 0, st->max_tiles * sizeof(unsigned long long));
-    st->counter = counter;
-    st->epoch = epoch;
-    st->tile_base = base;
-    *state = st;
+    // growing: the new array starts cleared and the epoch sequence continues
+    if (st->status) cudaFreeAsync(st->status, s);
+    st->status = nullptr;
+    st->max_tiles = 0;
+    GAHHG_TRY(pool_alloc((void**)&st->status, 2 * need * sizeof(unsigned long long), dev, s));
+    GAHHG_CUDA_TRY(cudaMemsetAsync(st->status, 0, 2 * need * sizeof(unsigned long long), s));
+    st->max_tiles = 2 * need;
     return GAHHG_OK;
 }
 
