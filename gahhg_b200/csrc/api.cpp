@@ -162,9 +162,8 @@ Grid::~Grid()
     type_old.release();
     type_cur.release();
     type_next.release();
-    if (d_err) cudaFree(d_err);
-    if (d_counts) cudaFree(d_counts);
-    if (h_counts) cudaFreeHost(h_counts);
+    if (d_err) cudaFreeAsync(d_err, stream);
+    if (d_counts) cudaFreeAsync(d_counts, stream);
     free_query_layout(qlayout);
     lattice_free(lattice);
     if (aux_stream) cudaStreamDestroy(aux_stream);

@@ -554,9 +554,8 @@ gahhg_status grid_build(Grid* g)
     GAHHG_TRY(g->edge_prev.reserve(n, s));
     GAHHG_TRY(g->edge_cnt.reserve(n, s));
     GAHHG_TRY(g->edge_off.reserve(n, s));
-    if (!g->d_err) GAHHG_CUDA_TRY(cudaMalloc(&g->d_err, sizeof(DeviceErrors)));
-    if (!g->d_counts) GAHHG_CUDA_TRY(cudaMalloc(&g->d_counts, 64 * sizeof(int)));
-    if (!g->h_counts) GAHHG_CUDA_TRY(cudaMallocHost(&g->h_counts, 64 * sizeof(int)));
+    if (!g->d_err) GAHHG_TRY(pool_alloc((void**)&g->d_err, sizeof(DeviceErrors), g->device, s));
+    if (!g->d_counts) GAHHG_TRY(pool_alloc((void**)&g->d_counts, 64 * sizeof(int), g->device, s));
     GAHHG_CUDA_TRY(cudaMemsetAsync(g->d_err, 0, sizeof(DeviceErrors), s));
     GAHHG_CUDA_TRY(cudaMemsetAsync(g->edge_cur.ptr, 0, sizeof(int) * n, s));
     GAHHG_CUDA_TRY(cudaMemsetAsync(g->edge_prev.ptr, 0, sizeof(int) * n, s));

