@@ -191,8 +191,9 @@ constexpr uint8_t LABEL_DEFER = 0xFF;
 // refused).
 constexpr uint32_t MASK_ALL = 0xFFFFFFFFu;
 
-// Records beyond the leaf's own two whose loads tier 1 issues together.
-constexpr int T1_GROUP = 4;
+// Records beyond the leaf's own two whose loads tier 1 issues together (most
+// leaves have at most four edges; groups of four: 263 us where two take 251).
+constexpr int T1_GROUP = 2;
 
 // A leaf as tier 1 reads it: four 16-byte loads of one line in flight.
 struct LeafLoad {
@@ -284,25 +285,51 @@ __device__ __forceinline__ uint8_t leaf_label_fp32(const float4* rec, const Leaf
 // Records beyond the leaf's own two whose ends the FP64 tier loads together.
 constexpr int T2_GROUP = 2;
 
+// A warp's 32 aux lines in shared memory: line r's 16-byte part q lies at
+// aux_slot(r, q) (the permutation keeps lanes that read the same part of their
+// lines off each other's banks).
+__device__ __forceinline__ int aux_slot(int r, int q) { return 8 * r + (q ^ (r & 7)); }
+
+// Brings the lines (null: none) there by the warp together, eight lanes a
+// line: an instruction touches four lines and not 32.
+__device__ __forceinline__ void copy_aux(uint4* s_aux, const LeafAux* mine)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const int r = 4 * j + (lane >> 3), q = lane & 7;
+        const unsigned long long a = __shfl_sync(0xffffffffu, (unsigned long long)mine, r);
+        if (a)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(s_aux + aux_slot(r, q))),
+                         "l"(a + 16 * q)
+                         : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
 // FP64 tier on the leaf's records selected by `mask` (MASK_ALL: every record,
 // from the leaf's label; else the records of bits 0..30, from the label of
-// bit 31): the leaf's aux line, and edge words and ends beyond its two edges.
-__device__ __forceinline__ uint8_t leaf_label_fp64(const QueryView& Q, uint32_t leaf, const PointCtx& P, uint32_t mask)
+// bit 31): the leaf's aux line (in the lane's place in shared memory, or
+// global memory when s_aux is null), and edge words and ends beyond its two
+// edges.  q: the point's canonical XYZ.
+template <bool SHARED>
+__device__ __forceinline__ uint8_t leaf_label_fp64(const QueryView& Q, uint32_t leaf, const uint4* s_aux,
+                                                   const double* q, uint32_t mask)
 {
     const LeafAux* X = Q.aux + leaf;
+    const int lane = threadIdx.x & 31;
     const uint4* xp = reinterpret_cast<const uint4*>(X);
-    const uint4 xa = __ldg(xp), xb = __ldg(xp + 1);
+    const uint4 xa = SHARED ? s_aux[aux_slot(lane, 0)] : __ldg(xp), xb = SHARED ? s_aux[aux_slot(lane, 1)] : __ldg(xp + 1);
     double2 e[T2_GROUP][3];
     static_assert(T2_GROUP == LEAF_INLINE, "the line's edges are the first group");
     // the line's ends go out with its header, the second edge's when it is asked for
 #pragma unroll
     for (int j = 0; j < LEAF_INLINE; j++) {
         const double2* p = reinterpret_cast<const double2*>(X->ends[j]);
-        if (mask >> j & 1u) {
-            e[j][0] = __ldg(p);
-            e[j][1] = __ldg(p + 1);
-            e[j][2] = __ldg(p + 2);
-        }
+        const double2* sp = reinterpret_cast<const double2*>(s_aux);
+        if (mask >> j & 1u)
+#pragma unroll
+            for (int k = 0; k < 3; k++) e[j][k] = SHARED ? sp[aux_slot(lane, 2 + 3 * j + k)] : __ldg(p + k);
     }
     const double LR[3] = {__hiloint2double((int)xa.y, (int)xa.x), __hiloint2double((int)xa.w, (int)xa.z),
                           __hiloint2double((int)xb.y, (int)xb.x)};
@@ -315,8 +342,6 @@ __device__ __forceinline__ uint8_t leaf_label_fp64(const QueryView& Q, uint32_t 
         left = max(0, cnt - 31);
         sel = cnt >= 31 ? 0x7fffffffu : (1u << cnt) - 1u;
     }
-    double q[3];
-    gahhg_canon_vertex_xyz(P.lon, P.lat, q);
     // bits of the group's edges and of their signs (orient(A, B, R) > 0)
     uint32_t group = sel & 3u, signs = xb.w >> 24, k0 = 0;
     sel &= ~3u;
@@ -827,7 +852,9 @@ __device__ __forceinline__ void query_tiles(const QueryView& Q, const uint32_t* 
                     uint8_t lab = (uint8_t)(w & 3u);
                     if ((w & KIND_MASK) != KIND_PURE) {
                         if (STATS && !FP32) c.boundary++;
-                        lab = leaf_label_fp64(Q, w & INDEX_MASK, P, FP32 ? s.m3[n3 + lane] : MASK_ALL);
+                        double q[3];
+                        gahhg_canon_vertex_xyz(P.lon, P.lat, q);
+                        lab = leaf_label_fp64<false>(Q, w & INDEX_MASK, nullptr, q, FP32 ? s.m3[n3 + lane] : MASK_ALL);
                         if (lab == LABEL_DEFER) {
                             if (STATS) c.exact++;
                             lab = leaf_label_exact(&Q, w & INDEX_MASK, P.lon, P.lat);
@@ -1323,8 +1350,11 @@ __device__ __forceinline__ void push_deferred(bool defer, uint32_t i, uint32_t w
 // time, the next 32 entries' points and leaf words loaded ahead, and meets no
 // other warp (the block's rounds used to end in three barriers around one
 // atomic; with the counter in parts a warp's own atomic costs nothing).  Four
-// blocks per SM: 64 registers, no spills, 279 us against 315 at five (48) for
-// the 9.1M points in leaves of 2e7 near-edge points.
+// blocks per SM: 64 registers, no spills, 251 us for the 9.1M points in leaves
+// of 2e7 near-edge points (five blocks, 48 registers: 315).  Half of the issue
+// slots and three quarters of the L1's tag lookups are taken (a lane loads its
+// own 64-byte leaf).  Copying the leaves to shared memory by the warp together
+// took 231 here but 36 us where a batch's tier 1 takes 30.
 constexpr int T1_BLOCKS = 4;
 template <class VS>
 __global__ void __launch_bounds__(TPB, T1_BLOCKS) k_leaf_t1(const __grid_constant__ VS vs,
@@ -1553,22 +1583,26 @@ __global__ void __launch_bounds__(TPB, T1S_BLOCKS) k_leaf_t1s(const __grid_const
     if (ctr) count_stats(ctr, c);
 }
 
-// Tier 2's shape: blocks of 128 threads, six per SM: 24 warps hide more of the
-// chain entry -> point and aux sector -> edge ends than the registers of
-// larger groups in flight.
+// Tier 2's shape: blocks of 128 threads; the warps hide the chain entry ->
+// point and aux line -> edge ends.  (us, blocks per SM 5 / 6 / 7 / 8, 2e7
+// points, half of them near the 1.1M-edge polygon's edges: all points of an
+// FP64-filter query 606 / 571 / 532 / 518, tier 1's deferred points 260 / 240
+// / 227 / 239.  A lane loading its own line: 614 and 233 at their best.)
 constexpr int T2_TPB = 128;
-constexpr int T2_BLOCKS = 6;
+constexpr int T2_ALL_BLOCKS = 8, T2_BLOCKS = 7;
 
 // Tier 2, then the complete test for what it leaves, over the queue of
 // deferred points; ALL: FP64-filter queries, over pass 1's queue.  The next
 // entry is loaded ahead, as in tier 1.
 template <class VS, bool ALL>
-__global__ void __launch_bounds__(T2_TPB, T2_BLOCKS) k_leaf_t2(const __grid_constant__ VS vs,
+__global__ void __launch_bounds__(T2_TPB, ALL ? T2_ALL_BLOCKS : T2_BLOCKS) k_leaf_t2(const __grid_constant__ VS vs,
                                                               const double2* __restrict__ ll,
                                                               uint8_t* __restrict__ out,
                                                               const __grid_constant__ Tiers T,
                                                               unsigned long long* ctr)
 {
+    __shared__ __align__(16) uint4 s_lines[T2_TPB / 32][8 * 32];
+    uint4* s_aux = s_lines[threadIdx.x >> 5];
     wait_for_predecessor();
     typename VS::Source S;
     PartEntries E;
@@ -1603,22 +1637,34 @@ __global__ void __launch_bounds__(T2_TPB, T2_BLOCKS) k_leaf_t2(const __grid_cons
         const bool mine = t0 + lane < m;
         double2 p = make_double2(0.0, 0.0);
         if (mine) p = ll[i];
+        const QueryView& Q = ALL ? vs.view(v) : vs.of(mine ? i : 0);
+        copy_aux(s_aux, mine && (known & KIND_MASK) == KIND_LEAF ? Q.aux + (known & INDEX_MASK) : nullptr);
         if (t0 + step < m) fetch(t0 + step);
-        if (!mine) continue;
-        const QueryView& Q = ALL ? vs.view(v) : vs.of(i);
-        PointCtx P;
-        const uint32_t w = point_leaf(Q, p, P, known);
-        uint8_t lab = (uint8_t)(w & 3u);
-        if ((w & KIND_MASK) != KIND_PURE) {
-            if (ALL) c.boundary++;
-            lab = leaf_label_fp64(Q, w & INDEX_MASK, P, mask);
-            if (lab == LABEL_DEFER) {
-                c.exact++;
-                lab = leaf_label_exact(&Q, w & INDEX_MASK, P.lon, P.lat);
-            }
+        PointCtx P{0.0, 0.0};
+        uint32_t w = KIND_PURE;
+        double q[3];
+        if (mine) {
+            w = point_leaf(Q, p, P, known);
+            gahhg_canon_vertex_xyz(P.lon, P.lat, q);
+            if (known == LEAF_UNKNOWN && (w & KIND_MASK) == KIND_LEAF)
+                for (int k = 0; k < 8; k++) s_aux[aux_slot(lane, k)] = __ldg((const uint4*)(Q.aux + (w & INDEX_MASK)) + k);
         }
-        out[i] = lab;
-        c.inside += lab == CELL_IN;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        if (mine) {
+            uint8_t lab = (uint8_t)(w & 3u);
+            if ((w & KIND_MASK) != KIND_PURE) {
+                if (ALL) c.boundary++;
+                lab = leaf_label_fp64<true>(Q, w & INDEX_MASK, s_aux, q, mask);
+                if (lab == LABEL_DEFER) {
+                    c.exact++;
+                    lab = leaf_label_exact(&Q, w & INDEX_MASK, P.lon, P.lat);
+                }
+            }
+            out[i] = lab;
+            c.inside += lab == CELL_IN;
+        }
+        __syncwarp();  // the lines are rewritten in the next round
     }
     if (!ALL && *(const volatile unsigned int*)T.over) {
         // points that found their part of tier 2's queue full
@@ -1948,7 +1994,7 @@ void tier2_launch(const VS& vs, const double2* ll, uint8_t* out, const Tiers& T,
                   unsigned long long* ctr, int sms, cudaStream_t s)
 {
     if (precision == GAHHG_QUERY_FP64_FILTER)
-        launch_dependent_tpb(k_leaf_t2<VS, true>, sms * T2_BLOCKS, T2_TPB, s, vs, ll, out, T, ctr);
+        launch_dependent_tpb(k_leaf_t2<VS, true>, sms * T2_ALL_BLOCKS, T2_TPB, s, vs, ll, out, T, ctr);
     else
         launch_dependent_tpb(k_leaf_t2<VS, false>, sms * T2_BLOCKS, T2_TPB, s, vs, ll, out, T, ctr);
 }
