@@ -693,8 +693,8 @@ def main():
         "cpu_baseline": cpu,
         "e2e": {"value": round(e2e_rate, 1), "unit": "Mpts/s", "h2d_bytes_per_step": 16 * e2e_n,
                 "d2h_bytes_per_step": e2e_n},
-        # per chunk of 2^27 points: k_locate and the three pass-2 tiers
-        "gpu_launches": 4 * args.steps * ((n + (1 << 27) - 1) // (1 << 27)),
+        # per chunk of 2^27 points: k_locate and the two tiers; up to 2^20 points one launch
+        "gpu_launches": args.steps * (1 if n <= 1 << 20 else 3 * ((n + (1 << 27) - 1) // (1 << 27))),
         "clocks": clk,
         "comparison": {
             "fp64_filter_exact_mpts": round(world * n / t64 / 1e6, 1),

@@ -159,20 +159,15 @@ gahhg_status gahhg_query(gahhg_grid* g, const double* lonlat, size_t n, uint8_t*
  * application that hands the whole device to its own allocator, a serving
  * loop that reserves all memory up front so a request can never fail on an
  * allocation, or code that must not hit the implicit synchronisation of
- * cudaMalloc/cudaFree.  gahhg_query_device takes its pass-2 scratch from a
- * stream-ordered pool; this variant uses a fixed 8 MB array in device memory
- * that the library reserves on every GPU that loads it, for as long as the
- * process lives.  Inputs and outputs are still the caller's device buffers.
+ * cudaMalloc/cudaFree.  gahhg_query_device takes large queries' scratch from a
+ * stream-ordered pool; this variant runs every query as one launch without
+ * scratch.  Inputs and outputs are still the caller's device buffers.
  *
  * Limits: at most gahhg_query_noalloc_max_points() points per call (2,097,152;
  * more returns GAHHG_ERR_CAPACITY); exact grids only (GAHHG_QUERY_AUTO,
- * _FP32_FILTER or _FP64_FILTER); no statistics are collected.  Every call
- * asks the runtime for the array's device address (nothing is cached, so the
- * address stays right after a cudaDeviceReset); the first call on a device
- * also loads the library's kernels there, so make that first call before any
- * stream capture.  All calls share the one array and it keeps the
- * last call's contents: calls whose work overlaps on the GPU (two streams,
- * two host threads) race, so order them on one stream or serialise them. */
+ * _FP32_FILTER or _FP64_FILTER); no statistics are collected.  The first call
+ * on a device also loads the library's kernels there, so make that first call
+ * before any stream capture.  Calls share nothing and may overlap. */
 gahhg_status gahhg_query_device_noalloc(gahhg_grid* g, const double* d_lonlat, size_t n, uint8_t* d_labels,
                                         int precision, void* stream);
 long long gahhg_query_noalloc_max_points(void);
@@ -209,7 +204,7 @@ int gahhg_batch_size(const gahhg_batch* b);
 /* Points per work chunk of the persistent query launch (default 4096). */
 gahhg_status gahhg_batch_set_chunk(gahhg_batch* b, int chunk_points);
 /* Launch shapes of the query's first pass (the descent to a leaf): shape
- * `shape` runs `points_per_thread` points per thread in lockstep at
+ * `shape` runs `points_per_thread` points per thread at a time at
  * `blocks_per_sm` resident blocks of 256 threads per SM.  Shapes are numbered
  * from 0 (the default) until gahhg_batch_shape_info answers GAHHG_ERR_ARG.
  * Labels do not depend on the shape; the fastest depends on the batch's mix
