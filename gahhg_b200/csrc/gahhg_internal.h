@@ -270,7 +270,6 @@ size_t lattice_device_bytes(const LatticeSet* L);   // capacity held on the devi
 long long lattice_scratch_bytes(const LatticeSet* L);  // held beside the index at the end of its build
 
 // scans (scan.cu)
-size_t scan_state_bytes(size_t n);
 gahhg_status scan_state_reserve(void** state, size_t max_n, cudaStream_t s);
 void scan_state_destroy(void* state);
 gahhg_status scan_exclusive(const int* d_in, int* d_out, int n, int* d_total, void* state, DeviceErrors* err,

@@ -37,7 +37,6 @@ namespace gahhg {
 namespace {
 
 constexpr int TPB = 256;
-inline int blocks_for(long long n) { return (int)std::max(1LL, (n + TPB - 1) / TPB); }
 
 // ------------------------------------------------------------- query ----
 
@@ -457,6 +456,7 @@ __device__ __forceinline__ uint32_t coarse_label(const QueryView& Q, const uint3
 // first 16 levels, and for the clamped out-of-range cases both give 0 or 3 at
 // every level.  The lattice has at most MAX_DESCENT levels below the top.
 constexpr int MAX_DESCENT = 16;
+static_assert(MAX_LEVEL <= MAX_DESCENT, "two bits of a fraction per level");
 __device__ __forceinline__ uint32_t frac_bits(double f) { return __double2uint_rz(f * 4294967296.0); }
 
 __device__ __forceinline__ uint32_t descend_bits(const QueryView& Q, uint32_t w, uint32_t U, uint32_t V)
@@ -719,7 +719,6 @@ __device__ __forceinline__ void query_tiles(const QueryView& Q, const uint32_t* 
                                             const double2* __restrict__ ll, uint8_t* __restrict__ out,
                                             WarpSpace<U>& s, QueryCounts& c)
 {
-    constexpr int TILE = WarpSpace<U>::TILE;
     const int lane = threadIdx.x & 31;
     const unsigned int below = (1u << lane) - 1u;
     int n1 = 0, n2 = 0, n3 = 0;  // queued points, the same in every lane

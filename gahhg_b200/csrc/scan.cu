@@ -136,12 +136,6 @@ k_scan_exclusive(const int* __restrict__ in, int* __restrict__ out, int n, int* 
 
 }  // namespace
 
-size_t scan_state_bytes(size_t n)
-{
-    size_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE + 1;
-    return sizeof(ScanState) + 256 + tiles * sizeof(unsigned long long);
-}
-
 // Status and counter come from the library's pool, ordered on the stream that
 // the scans run on (cudaMalloc and cudaFree took 100 us each, and a batch or a
 // hierarchy build makes a state).
