@@ -30,9 +30,7 @@ constexpr double RAD = GAHHG_PI_TRUNC / 180.0;  // degrees -> canonical radians 
 // the cell (along a parallel, then a meridian).  Children of a 4 x 4 split
 // have their centers within 3/4 of that bound from the parent's center and
 // bounds of about a quarter of it, so a factor of 1.25 keeps every child cap
-// inside its parent's cap with room for the distortion near the poles, and the
-// arc between two neighbouring top-level centers stays inside the union of
-// their caps.
+// inside its parent's cap with room for the distortion near the poles.
 constexpr double CAP_FACTOR = 1.25;
 
 // Edges per leaf before a cell splits, unless the caller chooses, and levels

@@ -10,8 +10,9 @@
 //   * a cell listing more than K edges is split 4 x 4, down to a depth limit;
 //   * every cell center has an exact label: the first center is reached from a
 //     point just left of an outer-ring edge through six fixed hub points, row
-//     0 and each column are chained by the crossing parity of the arcs between
-//     neighbouring centers, and a child takes its parent's label XOR the
+//     0 and each column are chained by the crossing parity of the paths
+//     center -> middle of the border -> neighbouring center, each half against
+//     its own cell's edges, and a child takes its parent's label XOR the
 //     parity of the arc parent center -> child center against the parent's
 //     edges.
 //
@@ -598,11 +599,12 @@ __global__ void k_l0_tables(const PolyGeo* __restrict__ pg, const long long* __r
 // its crossing parity with the half arcs center -> middle of the upper,
 // lower, left and right border (left and right on row 0 alone, where the
 // columns' chains start); bit 4 a crossing is not certain in the plane.  The
-// arc between two neighbouring centers goes through the border's middle, so
-// its parity is the XOR of two half arcs, each inside one cell and so against
-// that cell's list alone, found in the pass that tests the pair anyway: the
-// separate pass over merged lists with exact predicates took 2336 us on the
-// 1.1M-edge polygon.
+// path between two neighbouring centers goes through the border's middle, so
+// its parity is the XOR of two half arcs, each in the hull of one cell and so
+// against that cell's list alone, found in the pass that tests the pair
+// anyway: the separate pass over merged lists with exact predicates took 2336
+// us on the 1.1M-edge polygon.  (In a column that path is the arc between the
+// centers; in a row it has a corner, see l0_exact_parity.)
 constexpr uint32_t L0_HIT = 0x80000000u;
 constexpr uint32_t L0_UP = 1u, L0_DOWN = 2u, L0_LEFT = 4u, L0_RIGHT = 8u, L0_UNSURE = 16u;
 
@@ -1057,15 +1059,32 @@ __device__ int arc_parity_lists(const double2* ends, const double* P, const doub
     return par;
 }
 
-// Exact parity of the arc between two level-0 centers (each moved off a
-// vertex where it coincides with one) against both cells' lists.
+// Exact parity between two level-0 centers (each moved off a vertex where it
+// coincides with one) along a path that stays in their cells' hulls, where the
+// cells' lists hold every edge.  Upwards that is the arc itself: it leaves the
+// lower cell through the border between them.  Sideways it need not be: the
+// arc between two centers of row 0 rises above their parallel by hl^2 / 2 sin
+// cos, which in cells 64 times wider than high is above both cells.  The path
+// goes through the middle of the border between them instead, each half
+// against its own cell's list (as the plane's half arcs do); a middle that is
+// a vertex moves along the border.
 __device__ __noinline__ int l0_exact_parity(const double2* ends, const Geo& g, int i, int j, const int* La, int na,
                                             int i2, int j2, const int* Lb, int nb, int* bad)
 {
     NodeCap a = node_cap(g, 0, i, j), b = node_cap(g, 0, i2, j2);
     nudge_center(g, 0, a, ends, La, na);
     nudge_center(g, 0, b, ends, Lb, nb);
-    return arc_parity_lists(ends, a.R, b.R, La, na, Lb, nb, bad);
+    if (i == i2) return arc_parity_lists(ends, a.R, b.R, La, na, Lb, nb, bad);
+    const double lon = g.lon0 + (double)i2 * g.dlon0;
+    double lat = g.lat0 + ((double)j + 0.5) * g.dlat0, M[3];
+    gahhg_canon_vertex_xyz(lon, lat, M);
+    for (int tries = 0; tries < 8; tries++) {
+        if (!center_on_vertex(M, ends, La, na) && !center_on_vertex(M, ends, Lb, nb)) break;
+        lat += g.dlat0 * (1.0 / 2048.0);
+        gahhg_canon_vertex_xyz(lon, lat, M);
+    }
+    return arc_parity_lists(ends, a.R, M, La, na, nullptr, 0, bad) ^
+           arc_parity_lists(ends, M, b.R, Lb, nb, nullptr, 0, bad);
 }
 
 // Level-0 neighbour parities: per polygon its W (H - 1) vertical pairs, then
