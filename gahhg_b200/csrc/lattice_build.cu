@@ -729,7 +729,7 @@ struct L0View {
     const double2* cols;
 };
 
-// Work items of a long edge, in all polygons, and pairs of the short ones.
+// Work items of the long edges and list entries of all, in all polygons.
 struct L0Totals {
     unsigned long long items, pairs;
 };
@@ -792,10 +792,12 @@ template <int PASS>
 __global__ void __launch_bounds__(TPB) k_l0_items(L0View v, const EdgeBox* __restrict__ box,
                                                   const int* __restrict__ item_off, int total, int* cnt,
                                                   uint32_t* state, const int* off, int* cursor, int* list,
-                                                  unsigned long long* mask)
+                                                  unsigned long long* mask, L0Totals* totals)
 {
     static_assert(L0_CHUNK <= 64, "a 64-bit hit mask per item");
-    for (int it = blockIdx.x * TPB + threadIdx.x; it < total; it += gridDim.x * TPB) {
+    unsigned long long npr = 0;
+    for (long long i = (long long)blockIdx.x * TPB + threadIdx.x; i < total; i += gridDim.x * TPB) {
+        const int it = (int)i;
         unsigned long long m = 0;
         if (PASS == 1 && mask) {
             m = mask[it];
@@ -844,6 +846,7 @@ __global__ void __launch_bounds__(TPB) k_l0_items(L0View v, const EdgeBox* __res
         }
         if (PASS == 0) {
             if (mask) mask[it] = m;
+            npr += __popcll(m);
             for (unsigned long long r = m; r; r &= r - 1) atomicAdd(&cnt[row + xa + __ffsll((long long)r) - 1], 1);
         } else {
             for (unsigned long long r = m; r; r &= r - 1) {
@@ -851,6 +854,10 @@ __global__ void __launch_bounds__(TPB) k_l0_items(L0View v, const EdgeBox* __res
                 list[off[node] + atomicAdd(&cursor[node], 1)] = (int)t;
             }
         }
+    }
+    if (PASS == 0) {
+        for (int o = 16; o > 0; o >>= 1) npr += __shfl_down_sync(0xffffffffu, npr, o);
+        if ((threadIdx.x & 31) == 0 && npr) atomicAdd(&totals->pairs, npr);
     }
 }
 
@@ -1200,15 +1207,21 @@ __global__ void k_l0_polys(const long long* __restrict__ tops, int np, int nn, i
 // tile's status holds its sums, then its prefix; two 64-bit words per tile,
 // word 0 = list entries and leaves, word 1 = leaf records and refined nodes,
 // each with a 2-bit state; a warp per word looks back 32 tiles at a time).
+// The values' fields hold 16 entries for each of the level above, which has
+// 2^28 at most (PAIR_BUDGET), and any level's nodes; level 0's entries, which
+// may be more, are counted in 64 bits where they are found (L0Totals).
 // Waits are bounded; one that runs out sums the late tile's counts itself
 // (DeviceErrors::scan_lookback_timeout counts it).
 constexpr int LS_TPB = 256;
 constexpr int LS_ITEMS = 8;
 constexpr int LS_TILE = LS_TPB * LS_ITEMS;
-constexpr int LS_LO = 31;  // bits of a word's low value (entries, records); the state is in the top two bits
+constexpr int LS_LO = 33;  // bits of a word's low value (entries, records); the state is in the top two bits
+static_assert(4 * PAIR_BUDGET < 1LL << LS_LO, "16 entries for each of PAIR_BUDGET / 4");
+static_assert(INDEX_MASK / 4 < 1u << (62 - LS_LO) && NODE_BUDGET < 1LL << (62 - LS_LO), "a level's leaves");
 
 struct LevelSums {
-    int pairs, leaves, recs, refined;
+    long long pairs, recs;
+    int leaves, refined;
 };
 
 struct LevelScan {
@@ -1337,9 +1350,9 @@ __global__ void __launch_bounds__(LS_TPB) k_level_scan(LevelScan S)
     __syncthreads();
     constexpr unsigned long long LO = (1ull << LS_LO) - 1;
     if (t == 0 && (long long)(tile + 1) * LS_TILE >= S.nn) {
-        S.sums->pairs = (int)(s_total[0] & LO);
+        S.sums->pairs = (long long)(s_total[0] & LO);
         S.sums->leaves = (int)(s_total[0] >> LS_LO);
-        S.sums->recs = (int)(s_total[1] & LO);
+        S.sums->recs = (long long)(s_total[1] & LO);
         S.sums->refined = (int)(s_total[1] >> LS_LO);
     }
     unsigned long long r0 = s_prefix[0] + s_w[0][warp] + i0 - sum0, r1 = s_prefix[1] + s_w[1][warp] + i1 - sum1;
@@ -1978,8 +1991,10 @@ gahhg_status alloc_zero(DevArray<T>& d, size_t n, cudaStream_t s)
 
 // The whole build's small device words, cleared at its start.
 struct BuildWords {
-    L0Totals l0;
-    LevelSums sums;
+    struct {
+        L0Totals l0;
+        LevelSums level;
+    } sums;
     int bad[4];      // [0] coincidences, [1] unused, [2] long lists
     int sort[4];     // middling lists, next, long lists, next
     DeviceErrors err;
@@ -2019,7 +2034,7 @@ struct Builder {
     }
 
     // The level's prefixes and totals; `stop`: every non-empty node is a leaf.
-    gahhg_status scan(int lvl, bool stop)
+    gahhg_status scan_once(int lvl, bool stop)
     {
         LevelBuf& b = lv[lvl];
         b.kmax = stop ? INT_MAX : 0;
@@ -2030,11 +2045,33 @@ struct Builder {
         GAHHG_TRY(b.idx.alloc(b.nn, s));
         GAHHG_TRY(b.rec.alloc(b.nn, s));
         const LevelScan S{b.cnt.ptr, b.nn, polys_of_nodes(b), d_pg.ptr, b.kmax, b.off.ptr, b.idx.ptr, b.rec.ptr,
-                          status.ptr, (unsigned int*)(status.ptr + 2 * (size_t)tiles), &w->sums, &w->err,
+                          status.ptr, (unsigned int*)(status.ptr + 2 * (size_t)tiles), &w->sums.level, &w->err,
                           knob(GAHHG_KNOB_SCAN_SPIN_LIMIT)};
         k_level_scan<<<tiles, LS_TPB, 0, s>>>(S);
-        GAHHG_CUDA_TRY(cudaMemcpyAsync(&b.sums, &w->sums, sizeof(LevelSums), cudaMemcpyDeviceToHost, s));
+        decltype(w->sums) h;
+        GAHHG_CUDA_TRY(cudaMemcpyAsync(&h, &w->sums, sizeof h, cudaMemcpyDeviceToHost, s));
         GAHHG_CUDA_TRY(cudaStreamSynchronize(s));
+        b.sums = h.level;
+        const unsigned long long pairs = lvl ? (unsigned long long)h.level.pairs : h.l0.pairs;
+        if (pairs > (unsigned long long)INT_MAX) {
+            set_error("%s%llu list entries on level %d exceed 2^31 (fewer top cells are needed)", prefix.c_str(), pairs,
+                      lvl);
+            return GAHHG_ERR_CAPACITY;
+        }
+        return GAHHG_OK;
+    }
+
+    // ... under the budgets (`nodes`: in all, this level's included).  Bounded
+    // refinement: a polygon whose edges fill an area densely (not a curve)
+    // would need cells below the edge spacing everywhere.  Past the budget the
+    // remaining cells stay leaves with more edges: the labels are the same,
+    // the crossing loops longer.  (The budgets hold for the whole set.)
+    gahhg_status scan(int lvl, long long nodes)
+    {
+        GAHHG_TRY(scan_once(lvl, lvl >= MAX_LEVEL));
+        const LevelSums& c = lv[lvl].sums;
+        if (c.refined > 0 && (nodes + (long long)c.refined * FAN * FAN > NODE_BUDGET || 4 * c.pairs > PAIR_BUDGET))
+            return scan_once(lvl, true);
         return GAHHG_OK;
     }
 
@@ -2249,9 +2286,9 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
     GAHHG_TRY(emask.alloc(ne, s));
     GAHHG_TRY(boxes.alloc(ne, s));
     GAHHG_TRY(items.alloc(ne, s));
-    k_l0_edges<<<blocks_for(ne), TPB, 0, s>>>(v0, boxes.ptr, items.ptr, emask.ptr, lv[0].cnt.ptr, state.ptr, &w->l0);
+    k_l0_edges<<<blocks_for(ne), TPB, 0, s>>>(v0, boxes.ptr, items.ptr, emask.ptr, lv[0].cnt.ptr, state.ptr, &w->sums.l0);
     L0Totals tot{};
-    GAHHG_CUDA_TRY(cudaMemcpyAsync(&tot, &w->l0, sizeof tot, cudaMemcpyDeviceToHost, s));
+    GAHHG_CUDA_TRY(cudaMemcpyAsync(&tot, &w->sums.l0, sizeof tot, cudaMemcpyDeviceToHost, s));
     GAHHG_CUDA_TRY(cudaStreamSynchronize(s));
     if (tot.items > (unsigned long long)INT_MAX) {
         set_error("%s%llu level-0 candidate work items exceed 2^31 (fewer top cells are needed)", prefix.c_str(),
@@ -2265,10 +2302,10 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
         // the count pass's hits per item, so the fill pass does not test again
         if (tot.items <= L0_MASK_ITEMS) GAHHG_TRY(hits.alloc(tot.items, s));
         k_l0_items<0><<<sms * 8, TPB, 0, s>>>(v0, boxes.ptr, item_off.ptr, (int)tot.items, lv[0].cnt.ptr, state.ptr,
-                                              nullptr, nullptr, nullptr, hits.ptr);
+                                              nullptr, nullptr, nullptr, hits.ptr, &w->sums.l0);
     }
     phase("l0 count");
-    GAHHG_TRY(scan(0, false));
+    GAHHG_TRY(scan(0, n0));
     {
         LevelBuf& l0 = lv[0];
         DevArray<int> cursor, mid, longs;
@@ -2277,7 +2314,7 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
         k_l0_fill<<<blocks_for(ne), TPB, 0, s>>>(v0, boxes.ptr, emask.ptr, l0.off.ptr, cursor.ptr, l0.list.ptr);
         if (tot.items)
             k_l0_items<1><<<sms * 8, TPB, 0, s>>>(v0, boxes.ptr, item_off.ptr, (int)tot.items, l0.cnt.ptr, state.ptr,
-                                                  l0.off.ptr, cursor.ptr, l0.list.ptr, hits.ptr);
+                                                  l0.off.ptr, cursor.ptr, l0.list.ptr, hits.ptr, nullptr);
         GAHHG_CUDA_TRY(cudaMemsetAsync(w->sort, 0, sizeof w->sort, s));
         GAHHG_TRY(mid.alloc((size_t)l0.sums.pairs / (SORT_THREAD + 1) + 1, s));
         GAHHG_TRY(longs.alloc((size_t)l0.sums.pairs / (SORT_WARP + 1) + 1, s));
@@ -2363,8 +2400,8 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
         leaf_total += b.sums.leaves;
         rec_total += b.sums.recs;
         if (dbg)
-            fprintf(stderr, "lattice level %d: %d cells, %d edge entries, %d split, %d leaves of %d entries\n", lvl,
-                    b.nn, b.sums.pairs, nref, b.sums.leaves, b.sums.recs);
+            fprintf(stderr, "lattice level %d: %d cells, %lld edge entries, %d split, %d leaves of %lld entries\n",
+                    lvl, b.nn, b.sums.pairs, nref, b.sums.leaves, b.sums.recs);
         if (rec_total >= 0xFFFFFFFFll || leaf_total >= (long long)INDEX_MASK) {
             set_error("%stoo many leaves or edge records", prefix.c_str());
             return GAHHG_ERR_CAPACITY;
@@ -2395,15 +2432,7 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
         k_child_pairs<<<(c.nn + PAIR_TPB - 1) / PAIR_TPB, PAIR_TPB, 0, s>>>(a, v);
         k_child_pairs_long<<<sms * 2, TPB, 0, s>>>(a, v);
         GAHHG_CUDA_TRY(cudaGetLastError());
-        GAHHG_TRY(scan(lvl + 1, lvl + 1 >= MAX_LEVEL));
-        // Bounded refinement: a polygon whose edges fill an area densely (not
-        // a curve) would need cells below the edge spacing everywhere.  Past
-        // the budget the remaining cells stay leaves with more edges: the
-        // labels are the same, the crossing loops longer.  (The budget holds
-        // for the whole set.)
-        if (c.sums.refined > 0 &&
-            (gnext + (long long)c.sums.refined * FAN * FAN > NODE_BUDGET || 4LL * c.sums.pairs > PAIR_BUDGET))
-            GAHHG_TRY(scan(lvl + 1, true));
+        GAHHG_TRY(scan(lvl + 1, gnext));
     }
     const int nlev = (int)lv.size();
     L->nnodes = gnext;
