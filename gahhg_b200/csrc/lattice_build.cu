@@ -333,14 +333,30 @@ __device__ bool reference_points(const D3& a, const D3& b, double* xi, double* x
 constexpr int ORIGIN_PTS = 6;  // xo, xi, up to three hubs, the center
 struct OriginArcs {
     double pt[ORIGIN_PTS][3];
-    int np;    // points in use (0: edge 0 gives no reference point)
+    int np;    // points in use (0: the edge gives no reference point)
     int edge;  // the edge crossed by arc 0, within the polygon
 };
 struct OriginHits {
     int par[ORIGIN_PTS - 1];
     int cnt0, last0;  // crossings of arc 0
-    int coincident;   // an edge end coincides with a point of the path
+    int on0;          // an edge end coincides with an end of arc 0
+    int coincident;   // ... with another point of the path
 };
+__device__ __forceinline__ OriginHits no_hits()
+{
+    OriginHits h;
+    for (int k = 0; k < ORIGIN_PTS - 1; k++) h.par[k] = 0;
+    h.cnt0 = 0;
+    h.last0 = -1;
+    h.on0 = 0;
+    h.coincident = 0;
+    return h;
+}
+// Arc 0 crosses its own edge and no other, and meets no vertex.
+__device__ __forceinline__ bool arc0_serves(const OriginArcs& a, const OriginHits& h)
+{
+    return a.np > 0 && !h.on0 && h.par[0] == 1 && h.cnt0 == 1 && h.last0 == a.edge;
+}
 
 __device__ int origin_path(const double* xin, const double* center, double (*pt)[3])
 {
@@ -367,16 +383,18 @@ __device__ int origin_path(const double* xin, const double* center, double (*pt)
     return np + 1;
 }
 
+// Polygons 0 .. np of the arrays: the arcs from outer edge `edge` of each.
 __global__ void k_origin_setup(const double2* __restrict__ ends, const PolyGeo* __restrict__ pg,
-                               const long long* __restrict__ ebase, int np, OriginArcs* arcs, OriginHits* hits)
+                               const long long* __restrict__ ebase, int np, int edge, OriginArcs* arcs,
+                               OriginHits* hits)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np) return;
     OriginArcs a;
     a.np = 0;
-    a.edge = 0;
+    a.edge = edge;
     D3 A, B;
-    load_edge(ends, ebase[p], A, B);
+    load_edge(ends, ebase[p] + edge, A, B);
     double xi[3], xo[3];
     if (reference_points(A, B, xi, xo)) {
         const NodeCap c00 = node_cap(pg[p].g, 0, 0, 0);
@@ -384,23 +402,18 @@ __global__ void k_origin_setup(const double2* __restrict__ ends, const PolyGeo* 
         a.np = 1 + origin_path(xi, c00.R, a.pt + 1);
     }
     arcs[p] = a;
-    OriginHits h;
-    for (int k = 0; k < ORIGIN_PTS - 1; k++) h.par[k] = 0;
-    h.cnt0 = 0;
-    h.last0 = -1;
-    h.coincident = 0;
-    hits[p] = h;
+    hits[p] = no_hits();
 }
 
-// Every edge against its polygon's arcs (one pass over the edges; the arcs of
-// one polygon are the same for a whole warp, mostly).
-__global__ void __launch_bounds__(TPB) k_origin_cross(const double2* __restrict__ ends, long long ne,
+// Edges [e0, e1) against their polygons' arcs (one pass over the edges; the
+// arcs of one polygon are the same for a whole warp, mostly).
+__global__ void __launch_bounds__(TPB) k_origin_cross(const double2* __restrict__ ends, long long e0, long long e1,
                                                       const int* __restrict__ epoly,
                                                       const long long* __restrict__ ebase,
                                                       const OriginArcs* __restrict__ arcs, OriginHits* hits)
 {
-    const long long e = (long long)blockIdx.x * TPB + threadIdx.x;
-    if (e >= ne) return;
+    const long long e = e0 + (long long)blockIdx.x * TPB + threadIdx.x;
+    if (e >= e1) return;
     const int p = poly_of(epoly, e);
     const OriginArcs& a = arcs[p];
     const int np = a.np;
@@ -413,8 +426,9 @@ __global__ void __launch_bounds__(TPB) k_origin_cross(const double2* __restrict_
         const double P[3] = {a.pt[k][0], a.pt[k][1], a.pt[k][2]};
         const double Q[3] = {a.pt[k + 1][0], a.pt[k + 1][1], a.pt[k + 1][2]};
         if (exact::same(A, P) || exact::same(B, P) || exact::same(A, Q) || exact::same(B, Q)) {
-            hits[p].coincident = 1;
-            return;
+            if (k == 0) hits[p].on0 = 1;
+            else hits[p].coincident = 1;
+            continue;
         }
         if (!exact::crossing(P, Q, A, B)) continue;
         atomicXor(&hits[p].par[k], 1);
@@ -425,123 +439,88 @@ __global__ void __launch_bounds__(TPB) k_origin_cross(const double2* __restrict_
     }
 }
 
-// Parity, count and last index of the edges [e0, e1) crossing arc P -> Q,
-// summed over the block; coincident is set when an edge end coincides with P
-// or Q.  Every thread of the block calls.
-__device__ void block_arc_parity(const double2* ends, long long e0, long long e1, const double* P, const double* Q,
-                                 int& parity, int& ncross, int& last, bool& coincident)
+// origin[p] = the label of polygon p's first level-0 center from the
+// crossings found, -1 when a hub or the center coincides with a vertex,
+// ORIGIN_OPEN (counted in `open`) when the edge gave no reference point.
+constexpr int ORIGIN_OPEN = -2;
+__global__ void k_origin(const OriginArcs* __restrict__ arcs, const OriginHits* __restrict__ hits, int np, int* origin,
+                         int* open)
 {
-    __shared__ int s_par, s_cnt, s_last, s_co;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_par = 0;
-        s_cnt = 0;
-        s_last = -1;
-        s_co = 0;
-    }
-    __syncthreads();
-    int par = 0, cnt = 0, lst = -1, co = 0;
-    for (long long e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-        D3 a, b;
-        load_edge(ends, e, a, b);
-        const double A[3] = {a.x, a.y, a.z}, B[3] = {b.x, b.y, b.z};
-        if (exact::same(A, B)) continue;
-        if (exact::same(A, P) || exact::same(B, P) || exact::same(A, Q) || exact::same(B, Q)) {
-            co = 1;
-            continue;
-        }
-        if (exact::crossing(P, Q, A, B)) {
-            par ^= 1;
-            cnt++;
-            lst = max(lst, (int)(e - e0));
-        }
-    }
-    if (par) atomicXor(&s_par, 1);
-    if (cnt) atomicAdd(&s_cnt, cnt);
-    if (lst >= 0) atomicMax(&s_last, lst);
-    if (co) s_co = 1;
-    __syncthreads();
-    parity = s_par;
-    ncross = s_cnt;
-    last = s_last;
-    coincident = s_co != 0;
-    __syncthreads();
-}
-
-// One block per polygon: the label of its first level-0 center from the
-// crossings found, or, where the polygon's first edge gave no reference
-// point, from the next outer edge that does (one block's passes over the
-// polygon's edges).  origin[p] = the label, 0 when no outer edge gives a
-// reference point, -1 when a hub or the center coincides with a vertex.
-constexpr int ORIGIN_TPB = 512;
-__global__ void __launch_bounds__(ORIGIN_TPB) k_origin(const double2* __restrict__ ends,
-                                                       const PolyGeo* __restrict__ pg,
-                                                       const long long* __restrict__ ebase,
-                                                       const int* __restrict__ nouter,
-                                                       const OriginArcs* __restrict__ arcs,
-                                                       const OriginHits* __restrict__ hits, int* origin)
-{
-    const int p = blockIdx.x;
-    {
-        const int n = arcs[p].np;
-        const OriginHits& h = hits[p];
-        if (n > 0 && !h.coincident && h.par[0] == 1 && h.cnt0 == 1 && h.last0 == arcs[p].edge) {
-            if (threadIdx.x == 0) {
-                int par = 0;
-                for (int k = 1; k + 1 < n; k++) par ^= h.par[k];
-                origin[p] = par ? CELL_OUT : CELL_IN;
-            }
-            return;
-        }
-    }
-    const long long e0 = ebase[p], e1 = ebase[p + 1];
-    __shared__ double s_xi[3], s_xo[3];
-    __shared__ int s_ok;
-    bool found = false;
-    double xin[3] = {0.0, 0.0, 0.0};
-    for (int e = 0; e < nouter[p] && !found; e++) {
-        __syncthreads();  // every thread has read the previous candidate's s_ok
-        if (threadIdx.x == 0) {
-            D3 a, b;
-            load_edge(ends, e0 + e, a, b);
-            double xi[3], xo[3];
-            s_ok = reference_points(a, b, xi, xo) ? 1 : 0;
-            if (s_ok)
-                for (int k = 0; k < 3; k++) {
-                    s_xi[k] = xi[k];
-                    s_xo[k] = xo[k];
-                }
-        }
-        __syncthreads();
-        if (!s_ok) continue;  // the same in every thread
-        const double xo[3] = {s_xo[0], s_xo[1], s_xo[2]}, xi[3] = {s_xi[0], s_xi[1], s_xi[2]};
-        int par, nc, le;
-        bool co;
-        block_arc_parity(ends, e0, e1, xo, xi, par, nc, le, co);
-        if (!co && par == 1 && nc == 1 && le == e) {
-            found = true;
-            for (int k = 0; k < 3; k++) xin[k] = xi[k];
-        }
-    }
-    if (!found) {
-        if (threadIdx.x == 0) origin[p] = 0;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= np) return;
+    const OriginHits& h = hits[p];
+    if (!arc0_serves(arcs[p], h)) {
+        origin[p] = ORIGIN_OPEN;
+        atomicAdd(open, 1);
         return;
     }
-    const NodeCap c00 = node_cap(pg[p].g, 0, 0, 0);
-    double path[ORIGIN_PTS - 1][3];
-    const int n = origin_path(xin, c00.R, path);
-    int label = CELL_IN;
-    for (int k = 0; k + 1 < n; k++) {
-        int par, nc, le;
-        bool co;
-        block_arc_parity(ends, e0, e1, path[k], path[k + 1], par, nc, le, co);
-        if (co) {
-            if (threadIdx.x == 0) origin[p] = -1;
-            return;
-        }
-        if (par) label = 3 - label;
+    int par = 0;
+    for (int k = 1; k + 1 < arcs[p].np; k++) par ^= h.par[k];
+    origin[p] = h.coincident ? -1 : par ? CELL_OUT : CELL_IN;
+}
+
+// A polygon whose first edge gives no reference point (of no length, or with
+// other edges closer than a thousandth of its own length) takes the first
+// outer edge that does.  ORIGIN_CANDS edges are tried at a time, by a pass of
+// the whole grid over the polygon's edges: a comb of 160,000 edges, none of
+// which serves before the last one, was held up 29 s when one block tried one
+// edge after the other, 4.2 s by a grid and a round trip for each.
+constexpr int ORIGIN_CANDS = 64;
+__global__ void __launch_bounds__(ORIGIN_CANDS) k_origin_cands(const double2* __restrict__ ends, long long e0, int first,
+                                                              int nouter, OriginArcs* cands, OriginHits* hits)
+{
+    const int k = threadIdx.x;
+    OriginArcs a;
+    a.np = 0;
+    a.edge = first + k;
+    if (a.edge < nouter) {
+        D3 A, B;
+        load_edge(ends, e0 + a.edge, A, B);
+        if (reference_points(A, B, a.pt[1], a.pt[0])) a.np = 2;
     }
-    if (threadIdx.x == 0) origin[p] = label;
+    cands[k] = a;
+    hits[k] = no_hits();
+}
+
+__global__ void __launch_bounds__(TPB) k_origin_try(const double2* __restrict__ ends, long long e0, long long e1,
+                                                    const OriginArcs* __restrict__ cands, OriginHits* hits)
+{
+    __shared__ double s_pt[ORIGIN_CANDS][2][3];
+    __shared__ int s_np[ORIGIN_CANDS];
+    for (int t = threadIdx.x; t < ORIGIN_CANDS; t += TPB) {
+        s_np[t] = cands[t].np;
+        for (int j = 0; j < 6; j++) s_pt[t][j / 3][j % 3] = cands[t].np ? cands[t].pt[j / 3][j % 3] : 0.0;
+    }
+    __syncthreads();
+    const long long e = e0 + (long long)blockIdx.x * TPB + threadIdx.x;
+    if (e >= e1) return;
+    D3 a3, b3;
+    load_edge(ends, e, a3, b3);
+    const double A[3] = {a3.x, a3.y, a3.z}, B[3] = {b3.x, b3.y, b3.z};
+    if (exact::same(A, B)) return;
+    for (int k = 0; k < ORIGIN_CANDS; k++) {
+        if (!s_np[k]) continue;
+        const double *P = s_pt[k][0], *Q = s_pt[k][1];
+        if (exact::same(A, P) || exact::same(B, P) || exact::same(A, Q) || exact::same(B, Q)) {
+            hits[k].on0 = 1;
+        } else if (exact::crossing(P, Q, A, B)) {
+            atomicXor(&hits[k].par[0], 1);
+            atomicAdd(&hits[k].cnt0, 1);
+            atomicMax(&hits[k].last0, (int)(e - e0));
+        }
+    }
+}
+
+// *pick = the first candidate's edge that serves, -1 when none does.
+__global__ void __launch_bounds__(ORIGIN_CANDS) k_origin_pick(const OriginArcs* __restrict__ cands,
+                                                             const OriginHits* __restrict__ hits, int* pick)
+{
+    __shared__ int s_first;
+    if (threadIdx.x == 0) s_first = INT_MAX;
+    __syncthreads();
+    if (arc0_serves(cands[threadIdx.x], hits[threadIdx.x])) atomicMin(&s_first, cands[threadIdx.x].edge);
+    __syncthreads();
+    if (threadIdx.x == 0) *pick = s_first == INT_MAX ? -1 : s_first;
 }
 
 // ------------------------------------------------- level 0: edges -> cells --
@@ -1994,7 +1973,9 @@ struct BuildWords {
     struct {
         L0Totals l0;
         LevelSums level;
+        int open;  // polygons without the label of their first center
     } sums;
+    int pick;
     int bad[4];      // [0] coincidences, [1] unused, [2] long lists
     int sort[4];     // middling lists, next, long lists, next
     DeviceErrors err;
@@ -2075,6 +2056,8 @@ struct Builder {
         return GAHHG_OK;
     }
 
+    gahhg_status retry_origins(const std::vector<long long>& ebase, const long long* d_ebase,
+                               const std::vector<int>& nouter, OriginArcs* arcs, OriginHits* hits, int* origin);
     gahhg_status set_edges(Polygon* const* polys, const std::vector<long long>& ebase, const long long* d_ebase,
                            long long ne, int device);
     gahhg_status run(Grid* g, Polygon* const* polys, int count, const int* top_cells, const int* leaf_edges,
@@ -2137,6 +2120,43 @@ gahhg_status Builder::set_edges(Polygon* const* polys, const std::vector<long lo
     return GAHHG_OK;
 }
 
+// The first centers' labels of the polygons left open by k_origin: 0 where no
+// outer edge gives a reference point.
+gahhg_status Builder::retry_origins(const std::vector<long long>& ebase, const long long* d_ebase,
+                                    const std::vector<int>& nouter, OriginArcs* arcs, OriginHits* hits, int* origin)
+{
+    std::vector<int> h(np);
+    GAHHG_CUDA_TRY(cudaMemcpyAsync(h.data(), origin, sizeof(int) * np, cudaMemcpyDeviceToHost, s));
+    GAHHG_CUDA_TRY(cudaStreamSynchronize(s));
+    DevArray<OriginArcs> cands;
+    DevArray<OriginHits> chits;
+    GAHHG_TRY(cands.alloc(ORIGIN_CANDS, s));
+    GAHHG_TRY(chits.alloc(ORIGIN_CANDS, s));
+    const double2* ends = L->ends.ptr;
+    for (int p = 0; p < np; p++) {
+        if (h[p] != ORIGIN_OPEN) continue;
+        const long long e0 = ebase[p], e1 = ebase[p + 1];
+        int pick = -1;
+        for (int first = 0; first < nouter[p] && pick < 0; first += ORIGIN_CANDS) {
+            k_origin_cands<<<1, ORIGIN_CANDS, 0, s>>>(ends, e0, first, nouter[p], cands.ptr, chits.ptr);
+            k_origin_try<<<blocks_for(e1 - e0), TPB, 0, s>>>(ends, e0, e1, cands.ptr, chits.ptr);
+            k_origin_pick<<<1, ORIGIN_CANDS, 0, s>>>(cands.ptr, chits.ptr, &w->pick);
+            GAHHG_CUDA_TRY(cudaMemcpyAsync(&pick, &w->pick, sizeof pick, cudaMemcpyDeviceToHost, s));
+            GAHHG_CUDA_TRY(cudaStreamSynchronize(s));
+        }
+        if (pick < 0) {
+            GAHHG_CUDA_TRY(cudaMemsetAsync(origin + p, 0, sizeof(int), s));
+            continue;
+        }
+        k_origin_setup<<<1, TPB, 0, s>>>(ends, d_pg.ptr + p, d_ebase + p, 1, pick, arcs + p, hits + p);
+        k_origin_cross<<<blocks_for(e1 - e0), TPB, 0, s>>>(ends, e0, e1, np > 1 ? epoly.ptr : nullptr, d_ebase, arcs,
+                                                           hits);
+        k_origin<<<1, TPB, 0, s>>>(arcs + p, hits + p, 1, origin + p, &w->sums.open);
+        GAHHG_CUDA_TRY(cudaGetLastError());
+    }
+    return GAHHG_OK;
+}
+
 gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* top_cells, const int* leaf_edges,
                           const D3* d_pv, const int* d_pe)
 {
@@ -2164,9 +2184,7 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
     L->count = np;
     L->nedges = ne;
     DevArray<long long> d_ebase;
-    DevArray<int> d_nouter;
     GAHHG_TRY(upload(d_ebase, ebase, s));
-    GAHHG_TRY(upload(d_nouter, nouter, s));
     GAHHG_TRY(L->ends.alloc(3 * (size_t)ne, s));
     const double2* ends = L->ends.ptr;
     if (d_pv) {
@@ -2250,16 +2268,14 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
 
     // ---- exact label of every polygon's first level-0 center
     DevArray<int> origin;
+    DevArray<OriginArcs> arcs;
+    DevArray<OriginHits> ohits;
     GAHHG_TRY(origin.alloc(np, s));
-    {
-        DevArray<OriginArcs> arcs;
-        DevArray<OriginHits> hits;
-        GAHHG_TRY(arcs.alloc(np, s));
-        GAHHG_TRY(hits.alloc(np, s));
-        k_origin_setup<<<blocks_for(np), TPB, 0, s>>>(ends, d_pg.ptr, d_ebase.ptr, np, arcs.ptr, hits.ptr);
-        k_origin_cross<<<blocks_for(ne), TPB, 0, s>>>(ends, ne, ep, d_ebase.ptr, arcs.ptr, hits.ptr);
-        k_origin<<<np, ORIGIN_TPB, 0, s>>>(ends, d_pg.ptr, d_ebase.ptr, d_nouter.ptr, arcs.ptr, hits.ptr, origin.ptr);
-    }
+    GAHHG_TRY(arcs.alloc(np, s));
+    GAHHG_TRY(ohits.alloc(np, s));
+    k_origin_setup<<<blocks_for(np), TPB, 0, s>>>(ends, d_pg.ptr, d_ebase.ptr, np, 0, arcs.ptr, ohits.ptr);
+    k_origin_cross<<<blocks_for(ne), TPB, 0, s>>>(ends, 0, ne, ep, d_ebase.ptr, arcs.ptr, ohits.ptr);
+    k_origin<<<blocks_for(np), TPB, 0, s>>>(arcs.ptr, ohits.ptr, np, origin.ptr, &w->sums.open);
     phase("origin");
 
     // ---- level 0: candidate boxes, pair tests, counts
@@ -2287,9 +2303,11 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
     GAHHG_TRY(boxes.alloc(ne, s));
     GAHHG_TRY(items.alloc(ne, s));
     k_l0_edges<<<blocks_for(ne), TPB, 0, s>>>(v0, boxes.ptr, items.ptr, emask.ptr, lv[0].cnt.ptr, state.ptr, &w->sums.l0);
-    L0Totals tot{};
-    GAHHG_CUDA_TRY(cudaMemcpyAsync(&tot, &w->sums.l0, sizeof tot, cudaMemcpyDeviceToHost, s));
+    decltype(w->sums) first;
+    GAHHG_CUDA_TRY(cudaMemcpyAsync(&first, &w->sums, sizeof first, cudaMemcpyDeviceToHost, s));
     GAHHG_CUDA_TRY(cudaStreamSynchronize(s));
+    const L0Totals tot = first.l0;
+    if (first.open) GAHHG_TRY(retry_origins(ebase, d_ebase.ptr, nouter, arcs.ptr, ohits.ptr, origin.ptr));
     if (tot.items > (unsigned long long)INT_MAX) {
         set_error("%s%llu level-0 candidate work items exceed 2^31 (fewer top cells are needed)", prefix.c_str(),
                   tot.items);
