@@ -16,24 +16,11 @@
 // each wait is still bounded (spin_limit polls): when it runs out, the tile
 // sums the late tile's inputs itself and goes on looking back, so the result
 // stays exact, and the event is counted in DeviceErrors (scan fallbacks).
-#include "gahhg_internal.h"
+#include "scan_state.h"
 
 namespace gahhg {
 
 namespace {
-
-constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 8;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
-
-struct ScanState {
-    unsigned long long* status;
-    unsigned int* counter;
-    cudaStream_t stream;
-    size_t max_tiles;
-    unsigned int tile_base;
-    unsigned int epoch;
-};
 
 __device__ __forceinline__ unsigned long long load_status(const unsigned long long* p)
 {
@@ -135,47 +122,6 @@ k_scan_exclusive(const int* __restrict__ in, int* __restrict__ out, int n, int* 
 }
 
 }  // namespace
-
-// Status and counter come from the library's pool, ordered on the stream that
-// the scans run on (cudaMalloc and cudaFree took 100 us each, and a batch or a
-// hierarchy build makes a state).
-void scan_state_destroy(void* state)
-{
-    ScanState* st = (ScanState*)state;
-    if (!st) return;
-    if (st->status) cudaFreeAsync(st->status, st->stream);
-    if (st->counter) cudaFreeAsync(st->counter, st->stream);
-    delete st;
-}
-
-gahhg_status scan_state_reserve(void** state, size_t max_n, cudaStream_t s)
-{
-    const size_t need = (max_n + SCAN_TILE - 1) / SCAN_TILE + 1;
-    ScanState* st = (ScanState*)*state;
-    if (st && st->max_tiles >= need) return GAHHG_OK;
-    int dev = 0;
-    GAHHG_CUDA_TRY(cudaGetDevice(&dev));
-    if (!st) {
-        st = new ScanState();
-        st->status = nullptr;
-        st->counter = nullptr;
-        st->stream = s;
-        st->max_tiles = 0;
-        st->epoch = 1;
-        st->tile_base = 0;
-        *state = st;
-        GAHHG_TRY(pool_alloc((void**)&st->counter, sizeof(unsigned int), dev, s));
-        GAHHG_CUDA_TRY(cudaMemsetAsync(st->counter, 0, sizeof(unsigned int), s));
-    }
-    // growing: the new array starts cleared and the epoch sequence continues
-    if (st->status) cudaFreeAsync(st->status, s);
-    st->status = nullptr;
-    st->max_tiles = 0;
-    GAHHG_TRY(pool_alloc((void**)&st->status, 2 * need * sizeof(unsigned long long), dev, s));
-    GAHHG_CUDA_TRY(cudaMemsetAsync(st->status, 0, 2 * need * sizeof(unsigned long long), s));
-    st->max_tiles = 2 * need;
-    return GAHHG_OK;
-}
 
 gahhg_status scan_exclusive(const int* d_in, int* d_out, int n, int* d_total, void* state, DeviceErrors* err,
                             cudaStream_t s)
