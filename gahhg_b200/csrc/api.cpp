@@ -173,6 +173,13 @@ Grid::~Grid()
     }
 }
 
+// An index's memory goes back to the pool in the order of its own streams,
+// which know nothing of the streams that queries were issued on.
+void wait_for_queries(const std::atomic<bool>& unwaited)
+{
+    if (unwaited.load() && cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
+}
+
 static void fill_stats(Grid* g)
 {
     gahhg_stats& s = g->stats;
@@ -414,6 +421,7 @@ void gahhg_grid_free(gahhg_grid* G)
 {
     if (!G) return;
     cudaSetDevice(G->g.device);
+    wait_for_queries(G->g.unwaited);
     delete G;
 }
 
@@ -451,7 +459,10 @@ gahhg_status gahhg_query_device(gahhg_grid* G, const double* d_lonlat, size_t n,
     if (!G || (n && (!d_lonlat || !d_labels))) return GAHHG_ERR_ARG;
     Grid* g = &G->g;
     cudaStream_t s = (cudaStream_t)stream;
-    if (!sync) return run_query(g, d_lonlat, n, d_labels, precision, s, nullptr);
+    if (!sync) {
+        g->unwaited.store(true, std::memory_order_relaxed);
+        return run_query(g, d_lonlat, n, d_labels, precision, s, nullptr);
+    }
     uint64_t* d_cnt = nullptr;
     GAHHG_TRY(pool_alloc((void**)&d_cnt, 4 * sizeof(uint64_t), g->device, s));
     GAHHG_CUDA_TRY(cudaMemsetAsync(d_cnt, 0, 4 * sizeof(uint64_t), s));
@@ -475,7 +486,10 @@ gahhg_status gahhg_query_device(gahhg_grid* G, const double* d_lonlat, size_t n,
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaFreeAsync(d_cnt, s);
-    if (st != GAHHG_OK) return st;
+    if (st != GAHHG_OK) {
+        g->unwaited.store(true, std::memory_order_relaxed);  // (part of it may have been launched)
+        return st;
+    }
     g->stats.query_s = ms * 1e-3;
     g->stats.query_points = (long long)n;
     g->stats.esc_fp64 = (long long)cnt[0];
@@ -507,6 +521,7 @@ gahhg_status gahhg_query_device_noalloc(gahhg_grid* G, const double* d_lonlat, s
         return GAHHG_ERR_ARG;
     }
     GAHHG_CUDA_TRY(cudaSetDevice(g->device));
+    g->unwaited.store(true, std::memory_order_relaxed);
     return lattice_query_noalloc(g, d_lonlat, n, d_labels, precision, (cudaStream_t)stream);
 }
 

@@ -45,10 +45,12 @@ struct gahhg_batch {
     int g_nchunks = 0;
     long long g_qcap = 0;
     cudaStream_t owner_stream = nullptr;  // stream for workspace allocations
+    std::atomic<bool> unwaited{false};    // a query was issued that its call did not wait for
 
     ~gahhg_batch()
     {
         cudaSetDevice(device);
+        wait_for_queries(unwaited);
         if (exec) cudaGraphExecDestroy(exec);
         g_chunks.release();
         g_queue.release();
@@ -358,6 +360,7 @@ gahhg_status gahhg_batch_query_device(gahhg_batch* b, const double* d_lonlat, co
         GAHHG_CUDA_TRY(cudaMemsetAsync(d_stats, 0, 4 * sizeof(uint64_t), s));
     }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
+    if (!sync) b->unwaited.store(true, std::memory_order_relaxed);
     if (sync) {
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
@@ -383,6 +386,7 @@ gahhg_status gahhg_batch_query_device(gahhg_batch* b, const double* d_lonlat, co
             b->stats.in_count = (long long)c[3];
         }
     }
+    if (st != GAHHG_OK) b->unwaited.store(true, std::memory_order_relaxed);  // (part of it may have been launched)
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     cudaFreeAsync(d_chunks, s);
@@ -456,6 +460,7 @@ gahhg_status gahhg_batch_query_graph(gahhg_batch* b, const double* d_lonlat, con
         b->g_precision = precision;
         b->g_offsets.assign(offsets, offsets + b->count + 1);
     }
+    b->unwaited.store(true, std::memory_order_relaxed);
     GAHHG_CUDA_TRY(cudaGraphLaunch(b->exec, s));
     return GAHHG_OK;
 }

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -216,11 +217,14 @@ struct Grid {
     // semantics built on first need: report, export, depth, FP64 reference query)
     bool hierarchy = false;
     std::mutex hierarchy_mu;
+    // a query was issued that its call did not wait for: gahhg_grid_free does
+    std::atomic<bool> unwaited{false};
 
     Grid();
     ~Grid();
 };
 
+void wait_for_queries(const std::atomic<bool>& unwaited);  // on the current device
 gahhg_status grid_build(Grid* g);
 gahhg_status grid_classify(Grid* g);
 gahhg_status grid_query_ref(Grid* g, const double* d_lonlat, size_t n, uint8_t* d_labels, cudaStream_t s,

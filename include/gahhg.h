@@ -137,6 +137,8 @@ void gahhg_points_free(gahhg_points* p);
 gahhg_status gahhg_build(const gahhg_polygon* poly, const gahhg_build_opts* opts, gahhg_grid** out);
 /* GPISP::classifyAHHG (source/GPISPAHHG.cu:2018-2059). */
 gahhg_status gahhg_classify(gahhg_grid* g);
+/* Waits for the device's work first when a query was issued without `sync`
+ * (or by gahhg_query_device_noalloc): queries in flight complete. */
 void gahhg_grid_free(gahhg_grid* g);
 
 /* ---- query -------------------------------------------------------------- */
@@ -226,6 +228,7 @@ gahhg_status gahhg_batch_query_device(gahhg_batch* b, const double* d_lonlat, co
 gahhg_status gahhg_batch_query_graph(gahhg_batch* b, const double* d_lonlat, const int64_t* offsets,
                                      uint8_t* d_labels, int precision, void* stream);
 gahhg_status gahhg_batch_stats_get(const gahhg_batch* b, gahhg_batch_stats* s);
+/* As gahhg_grid_free: waits for queries that their calls did not wait for. */
 void gahhg_batch_free(gahhg_batch* b);
 
 /* ---- serving: a request loop over resident indexes (no counterpart in the
