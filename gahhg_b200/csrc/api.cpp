@@ -180,6 +180,13 @@ void wait_for_queries(const std::atomic<bool>& unwaited)
     if (unwaited.load() && cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
 }
 
+gahhg_status check_points_aligned(const double* d_lonlat)
+{
+    if (((uintptr_t)d_lonlat & 15u) == 0) return GAHHG_OK;
+    set_error("queries read lon/lat in 16-byte units: the device buffer must be 16-byte aligned");
+    return GAHHG_ERR_ARG;
+}
+
 static void fill_stats(Grid* g)
 {
     gahhg_stats& s = g->stats;
@@ -435,6 +442,7 @@ static gahhg_status run_query(Grid* g, const double* d_lonlat, size_t n, uint8_t
     if (precision == GAHHG_QUERY_AUTO)
         precision = g->lattice ? GAHHG_QUERY_FP32_FILTER : GAHHG_QUERY_REFERENCE_FP64;
     if (precision == GAHHG_QUERY_REFERENCE_FP64) {
+        if (n) GAHHG_TRY(check_points_aligned(d_lonlat));
         GAHHG_TRY(ensure_hierarchy(g));
         return grid_query_ref(g, d_lonlat, n, d_labels, s, d_counters);
     }
@@ -443,10 +451,7 @@ static gahhg_status run_query(Grid* g, const double* d_lonlat, size_t n, uint8_t
             set_error("exact precision needs a grid built with GAHHG_SEMANTICS_EXACT");
             return GAHHG_ERR_STATE;
         }
-        if ((uintptr_t)d_lonlat & 15u) {
-            set_error("exact queries read lon/lat in 16-byte units: the device buffer must be 16-byte aligned");
-            return GAHHG_ERR_ARG;
-        }
+        GAHHG_TRY(check_points_aligned(d_lonlat));
         return lattice_query(g, d_lonlat, n, d_labels, precision, s, d_counters);
     }
     set_error("unknown precision %d", precision);

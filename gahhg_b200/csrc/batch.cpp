@@ -338,6 +338,7 @@ gahhg_status gahhg_batch_query_device(gahhg_batch* b, const double* d_lonlat, co
         set_error("batches answer with exact labels (FP32 or FP64 filter)");
         return GAHHG_ERR_ARG;
     }
+    if (offsets[b->count]) GAHHG_TRY(check_points_aligned(d_lonlat));
     GAHHG_CUDA_TRY(cudaSetDevice(b->device));
     cudaStream_t s = (cudaStream_t)stream;
     const long long total = offsets[b->count];
@@ -406,6 +407,7 @@ gahhg_status gahhg_batch_query_graph(gahhg_batch* b, const double* d_lonlat, con
         set_error("batches answer with exact labels (FP32 or FP64 filter)");
         return GAHHG_ERR_ARG;
     }
+    if (offsets[b->count]) GAHHG_TRY(check_points_aligned(d_lonlat));
     GAHHG_CUDA_TRY(cudaSetDevice(b->device));
     cudaStream_t s = (cudaStream_t)stream;
     const bool same = b->exec && b->g_lonlat == d_lonlat && b->g_labels == d_labels && b->g_precision == precision &&

@@ -224,6 +224,7 @@ struct Grid {
     ~Grid();
 };
 
+gahhg_status check_points_aligned(const double* d_lonlat);  // to 16 bytes, as every query kernel reads points
 void wait_for_queries(const std::atomic<bool>& unwaited);  // on the current device
 gahhg_status grid_build(Grid* g);
 gahhg_status grid_classify(Grid* g);

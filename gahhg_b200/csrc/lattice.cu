@@ -2224,10 +2224,7 @@ gahhg_status lattice_query_noalloc(Grid* g, const double* d_lonlat, size_t n, ui
                   NOALLOC_MAX_POINTS);
         return GAHHG_ERR_CAPACITY;
     }
-    if ((uintptr_t)d_lonlat & 15u) {
-        set_error("exact queries read lon/lat in 16-byte units: the device buffer must be 16-byte aligned");
-        return GAHHG_ERR_ARG;
-    }
+    GAHHG_TRY(check_points_aligned(d_lonlat));
     if (n == 0) return GAHHG_OK;
     query_inline(make_view(g), (const double2*)d_lonlat, (int)n, d_labels, precision, nullptr, sm_count(g->device), s);
     GAHHG_CUDA_TRY(cudaGetLastError());

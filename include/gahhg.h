@@ -144,9 +144,8 @@ void gahhg_grid_free(gahhg_grid* g);
 /* ---- query -------------------------------------------------------------- */
 
 /* GPISP::test / kernel_PISP (source/GPISPAHHG.cu:2062-2085, 1422-1504).
- * Device pointers: lonlat (2 doubles per point; 16-byte aligned for the
- * exact precisions, which read it in 16-byte units, else GAHHG_ERR_ARG),
- * labels (1 byte per point).
+ * Device pointers: lonlat (2 doubles per point; 16-byte aligned, since points
+ * are read in 16-byte units, else GAHHG_ERR_ARG), labels (1 byte per point).
  * Asynchronous on `stream`; statistics are updated when `sync` is non-zero. */
 gahhg_status gahhg_query_device(gahhg_grid* g, const double* d_lonlat, size_t n, uint8_t* d_labels,
                                 int precision, void* stream, int sync);
@@ -215,8 +214,9 @@ gahhg_status gahhg_batch_shape_info(int shape, int* points_per_thread, int* bloc
 gahhg_status gahhg_batch_set_shape(gahhg_batch* b, int shape);
 /* Labels for all polygons at once.  d_lonlat holds the points polygon after
  * polygon: polygon p owns points [offsets[p], offsets[p+1]) (host array of
- * count+1 entries, offsets[0] = 0, fewer than 2^32 points in all).  Exact
- * labels (GAHHG_QUERY_AUTO, _FP32_FILTER, _FP64_FILTER).  Scratch comes from
+ * count+1 entries, offsets[0] = 0, fewer than 2^32 points in all), 16-byte
+ * aligned, else GAHHG_ERR_ARG.  Exact labels (GAHHG_QUERY_AUTO,
+ * _FP32_FILTER, _FP64_FILTER).  Scratch comes from
  * the library's stream-ordered pool; with sync != 0 the call waits and
  * records statistics. */
 gahhg_status gahhg_batch_query_device(gahhg_batch* b, const double* d_lonlat, const int64_t* offsets,
