@@ -26,10 +26,11 @@
 //
 // Builds.  Build workers (low-priority streams) take queued builds in order
 // once their estimated footprint fits in the HBM budget, evicting least
-// recently queried unpinned polygons first when asked to.  The estimate
-// (index bytes per edge with a margin and the build's own working memory, both
-// learnt from finished builds) is replaced by the measured footprint when the build finishes.  Queries to a polygon that
-// is still building are held and released when it is ready.
+// recently queried unpinned polygons first when asked to.  The estimate (index
+// bytes per edge with a margin and, beside other polygons, the build's working
+// memory, both learnt from finished builds: charge_locked) is replaced by the
+// measured footprint when the build finishes.  Queries to a polygon that is
+// still building are held and released when it is ready.
 //
 // A polygon's reference count covers its submitted but unfinished queries,
 // so an evicted polygon is freed only after the last of them completes.
@@ -89,7 +90,9 @@ struct SrvPoly {
     int top = 0, leaf = 0;
     bool pinned = false;
     int refs = 0;         // submitted queries not yet completed
-    long long est = 0;    // admission estimate (while queued or building)
+    long long est = 0;    // admission estimate (while queued)
+    long long scratch = 0;  // ... of the build's working memory
+    long long charged = 0;  // committed for it while it builds
     long long bytes = 0;  // measured device bytes (when ready)
     double last_use = 0.0;
     int swords = 0;
@@ -263,11 +266,18 @@ struct gahhg_server {
 
     long long estimate(long long edges) const
     {
-        // lattice (256 KB floor, 1.5x margin) + polygon copy (24 B vertex + 8 B
-        // edge) + what a build holds beside its index while it runs
-        return std::max<long long>(256 << 10, (long long)(1.5 * bytes_per_edge * (double)edges)) + edges * 32 +
-               (long long)(scratch_per_edge * (double)edges);
+        // lattice (256 KB floor, 1.5x margin) + polygon copy (24 B vertex + 8 B edge)
+        return std::max<long long>(256 << 10, (long long)(1.5 * bytes_per_edge * (double)edges)) + edges * 32;
     }
+
+    // What the build of P takes of the budget now: its index, and beside other
+    // polygons its working memory (the levels' arrays, as large as the index),
+    // up to what the others hold.  A polygon that would have the budget to
+    // itself is admitted by its index alone, before the working memory is
+    // learnt and after: charged in full it was refused a budget in which the
+    // first build of the same polygon had been admitted.  (The pool maps 4 GB
+    // beyond the budget.)
+    long long charge_locked(const SrvPoly& P) const { return P.est + std::min(P.scratch, committed); }
 
     // ------------------------------------------------------------- queries --
     void dispatch_loop()
@@ -522,10 +532,10 @@ struct gahhg_server {
         while (!build_queue.empty()) {
             const int id = build_queue.front();
             SrvPoly& P = polys[id];
-            const long long need = P.est;
-            if (committed + need <= o.hbm_budget) {
+            if (committed + charge_locked(P) <= o.hbm_budget) {
                 build_queue.pop_front();
-                committed += need;
+                P.charged = charge_locked(P);
+                committed += P.charged;
                 P.state = GAHHG_POLY_BUILDING;
                 builds_running++;
                 return id;
@@ -540,10 +550,10 @@ struct gahhg_server {
                 std::sort(cand.begin(), cand.end(),
                           [&](int a, int b) { return polys[a].last_use < polys[b].last_use; });
                 for (int i : cand) {
-                    if (committed + need <= o.hbm_budget) break;
+                    if (committed + charge_locked(P) <= o.hbm_budget) break;
                     free_poly_locked(i);
                 }
-                if (committed + need <= o.hbm_budget) continue;
+                if (committed + charge_locked(P) <= o.hbm_budget) continue;
             }
             // wait only while something under way can release memory
             bool can_free = builds_running > 0;
@@ -552,10 +562,10 @@ struct gahhg_server {
                 if (Q.state == GAHHG_POLY_EVICTING) can_free = true;
                 if (o.evict_lru && Q.state == GAHHG_POLY_READY && !Q.pinned && Q.refs > 0) can_free = true;
             }
-            if (need <= o.hbm_budget && can_free) return -1;
+            if (P.est <= o.hbm_budget && can_free) return -1;
             build_queue.pop_front();
-            set_error("build of %lld estimated bytes does not fit in the HBM budget (%lld of %lld committed)", need,
-                      committed, o.hbm_budget);
+            set_error("build of %lld estimated bytes does not fit in the HBM budget (%lld of %lld committed)",
+                      charge_locked(P), committed, o.hbm_budget);
             fail_build_locked(id, GAHHG_ERR_CAPACITY);
         }
         return -1;
@@ -631,7 +641,7 @@ struct gahhg_server {
             }
             lk.lock();
             builds_running--;
-            committed -= P.est;
+            committed -= P.charged;
             if (st != GAHHG_OK) {
                 set_error("%s", msg.c_str());
                 fail_build_locked(id, st);
@@ -862,6 +872,7 @@ gahhg_status gahhg_server_submit_build(gahhg_server* s, const gahhg_polygon* pol
     P.leaf = leaf_edges;
     P.pinned = (flags & GAHHG_SERVE_PINNED) != 0;
     P.est = s->estimate(edges);
+    P.scratch = (long long)(s->scratch_per_edge * (double)edges);
     P.last_use = now_seconds();
     Req* r = new Req();
     r->build = true;
