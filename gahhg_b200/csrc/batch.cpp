@@ -34,7 +34,8 @@ struct gahhg_batch {
     gahhg_batch_stats stats{};
     // graph replay state
     cudaGraphExec_t exec = nullptr;
-    cudaStream_t graph_stream = nullptr;
+    cudaEvent_t replayed = nullptr;  // after the last replay: its workspace is rewritten behind it
+    bool replays = false;            // the event was recorded
     const double* g_lonlat = nullptr;
     uint8_t* g_labels = nullptr;
     int g_precision = -1;
@@ -52,6 +53,7 @@ struct gahhg_batch {
         cudaSetDevice(device);
         wait_for_queries(unwaited);
         if (exec) cudaGraphExecDestroy(exec);
+        if (replayed) cudaEventDestroy(replayed);
         g_chunks.release();
         g_queue.release();
         g_counters.release();
@@ -421,6 +423,8 @@ gahhg_status gahhg_batch_query_graph(gahhg_batch* b, const double* d_lonlat, con
         }
         if (!b->owner_stream) GAHHG_CUDA_TRY(cudaStreamCreateWithFlags(&b->owner_stream, cudaStreamNonBlocking));
         cudaStream_t ws = b->owner_stream;
+        if (!b->replayed) GAHHG_CUDA_TRY(cudaEventCreateWithFlags(&b->replayed, cudaEventDisableTiming));
+        if (b->replays) GAHHG_CUDA_TRY(cudaStreamWaitEvent(ws, b->replayed, 0));
         const long long total = offsets[b->count];
         std::vector<uint8_t> chunks;
         batch_make_chunks((const long long*)offsets, b->count, b->chunk_points, b->swords.data(), nullptr, chunks,
@@ -464,6 +468,13 @@ gahhg_status gahhg_batch_query_graph(gahhg_batch* b, const double* d_lonlat, con
     }
     b->unwaited.store(true, std::memory_order_relaxed);
     GAHHG_CUDA_TRY(cudaGraphLaunch(b->exec, s));
+    // (a replay that becomes part of the caller's own graph runs when that does)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GAHHG_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+    if (cap == cudaStreamCaptureStatusNone) {
+        GAHHG_CUDA_TRY(cudaEventRecord(b->replayed, s));
+        b->replays = true;
+    }
     return GAHHG_OK;
 }
 

@@ -224,7 +224,8 @@ gahhg_status gahhg_batch_query_device(gahhg_batch* b, const double* d_lonlat, co
 /* The same query as a CUDA graph: the first call with a given set of
  * pointers, offsets and precision captures the launch sequence (with its own
  * persistent scratch); later calls with the same arguments only launch the
- * graph on `stream`.  Replays of one batch's graph must not overlap. */
+ * graph on `stream`.  Replays of one batch's graph must not overlap; a call
+ * that captures again waits for the replay before it. */
 gahhg_status gahhg_batch_query_graph(gahhg_batch* b, const double* d_lonlat, const int64_t* offsets,
                                      uint8_t* d_labels, int precision, void* stream);
 gahhg_status gahhg_batch_stats_get(const gahhg_batch* b, gahhg_batch_stats* s);
