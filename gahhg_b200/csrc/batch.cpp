@@ -370,7 +370,7 @@ gahhg_status gahhg_batch_query_device(gahhg_batch* b, const double* d_lonlat, co
         cudaEventRecord(e0, s);
     }
     gahhg_status st = batch_query_launch(b->views.ptr, d_chunks, nchunks, d_lonlat, d_labels, precision, queue,
-                                         qcap, counters, d_stats, s, b->device, true, b->shape);
+                                         qcap, total, counters, d_stats, s, b->device, true, b->shape);
     if (sync && st == GAHHG_OK) {
         cudaEventRecord(e1, s);
         uint64_t c[4] = {0, 0, 0, 0};
@@ -444,7 +444,7 @@ gahhg_status gahhg_batch_query_graph(gahhg_batch* b, const double* d_lonlat, con
             st = GAHHG_ERR_CUDA;
         } else {
             st = batch_query_launch(b->views.ptr, b->g_chunks.ptr, b->g_nchunks, d_lonlat, d_labels, precision,
-                                    b->g_queue.ptr, b->g_qcap, b->g_counters.ptr, nullptr, cs, b->device, true,
+                                    b->g_queue.ptr, b->g_qcap, total, b->g_counters.ptr, nullptr, cs, b->device, true,
                                     b->shape);
             if (cudaStreamEndCapture(cs, &graph) != cudaSuccess) st = GAHHG_ERR_CUDA;
         }

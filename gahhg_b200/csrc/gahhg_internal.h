@@ -266,7 +266,7 @@ size_t batch_queue_words(long long queue_cap, long long nchunks);
 // indexes the pass-1 launch shapes (batch_shape_info).
 gahhg_status batch_query_launch(const void* d_views, const void* d_chunks, int nchunks, const double* d_lonlat,
                                 uint8_t* d_labels, int precision, uint32_t* queue, long long queue_cap,
-                                unsigned int* counters, uint64_t* d_stats, cudaStream_t s, int device,
+                                long long points, unsigned int* counters, uint64_t* d_stats, cudaStream_t s, int device,
                                 bool zero_counters = true, int shape = 0);
 int batch_shape_count();
 bool batch_shape_info(int shape, int* points_per_thread, int* blocks_per_sm);

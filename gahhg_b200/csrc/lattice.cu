@@ -1038,25 +1038,76 @@ __device__ __forceinline__ void locate_chunk(const QueryView& Q, const uint32_t*
     }
 }
 
+// Prefix sums of the chunks' queue counts, by one block of THREADS threads:
+// pre[c] entries come before chunk c's, pre[nchunks] in all.  And zeros in tier
+// 2's counters, which nothing has touched yet.
+constexpr int CS_ITEMS = 8;
+template <int THREADS>
+__device__ __forceinline__ void chunk_prefix(const unsigned int* ccount, int nchunks, unsigned int* pre,
+                                             unsigned int* t2cnt)
+{
+    constexpr int WARPS = THREADS / 32;
+    __shared__ unsigned int s_w[WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < QUEUE_PARTS) t2cnt[threadIdx.x * COUNTER_STRIDE] = 0;
+    unsigned int before = 0;
+    for (int base = 0; base < nchunks; base += THREADS * CS_ITEMS) {
+        const int b0 = base + threadIdx.x * CS_ITEMS;
+        unsigned int c[CS_ITEMS], run = 0;
+#pragma unroll
+        for (int k = 0; k < CS_ITEMS; k++) {
+            c[k] = b0 + k < nchunks ? __ldcg(ccount + b0 + k) : 0u;
+            run += c[k];
+        }
+        unsigned int x = run;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_w[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            unsigned int z = lane < WARPS ? s_w[lane] : 0u;
+            for (int o = 1; o < WARPS; o <<= 1) {
+                const unsigned int y = __shfl_up_sync(0xffffffffu, z, o);
+                if (lane >= o) z += y;
+            }
+            if (lane < WARPS) s_w[lane] = z;
+        }
+        __syncthreads();
+        unsigned int at = before + (warp ? s_w[warp - 1] : 0u) + x - run;
+#pragma unroll
+        for (int k = 0; k < CS_ITEMS; k++) {
+            if (b0 + k < nchunks) pre[b0 + k] = at;
+            at += c[k];
+        }
+        before += s_w[WARPS - 1];
+        __syncthreads();  // s_w is rewritten
+    }
+    if (threadIdx.x == 0) pre[nchunks] = before;
+}
+
 // Pass 1 over a batch: a persistent grid takes chunks in order from an atomic
 // counter (polygons of very different sizes balance themselves; the next
 // chunk's number is on its way while a chunk is worked on), copies the chunk's
 // view and polygon summary to shared memory and runs the tile loop on it.  A
 // chunk's points in leaves are queued from the chunk's own first place,
-// counted in shared memory: no global atomic (see QUEUE_PARTS).
+// counted in shared memory: no global atomic (see QUEUE_PARTS).  With `pre` the
+// block that ends last makes the prefix sums of those counts (see SCAN_FOLD).
 template <bool STATS, int UNROLL, int BLOCKS>
 __global__ void __launch_bounds__(TPB, BLOCKS) k_batch_locate(const QueryView* __restrict__ views,
                                                      const BatchChunk* __restrict__ chunks, int nchunks,
                                                      unsigned int* next_chunk, const double2* __restrict__ ll,
                                                      uint8_t* __restrict__ out, uint32_t* __restrict__ queue,
-                                                     uint32_t* __restrict__ leafq, unsigned int* __restrict__ ccount,
+                                                     uint32_t* __restrict__ leafq, unsigned int* ccount,
+                                                     unsigned int* pre, unsigned int* t2cnt, unsigned int* ended,
                                                      unsigned long long* ctr, int poll_limit)
 {
     __shared__ __align__(16) uint32_t s_sum[SUMMARY_WORDS_MAX];  // receives the bulk copies
     __shared__ __align__(16) uint32_t s_view[sizeof(QueryView) / 4];
     __shared__ uint32_t s_mixed[TPB / 32][32 * (B_DESCENTS + UNROLL)];
     __shared__ __align__(8) uint64_t s_bar;
-    __shared__ int s_chunk, s_late;
+    __shared__ int s_chunk, s_late, s_last;
     __shared__ unsigned int s_queued;
     static_assert(sizeof(QueryView) % 4 == 0 && sizeof(QueryView) / 4 <= TPB, "a word of the view per thread");
     if (threadIdx.x == 0) {
@@ -1108,55 +1159,26 @@ __global__ void __launch_bounds__(TPB, BLOCKS) k_batch_locate(const QueryView* _
         if (threadIdx.x == 0) atomicAdd(&g_tma_timeouts, 1u);
         mbar_wait(&s_bar, phase ^ 1u);  // the copy in flight ends before the block does (bounded)
     }
+    if (pre) {
+        if (threadIdx.x == 0) {
+            __threadfence();  // this block's counts (thread 0 wrote them) come before its end
+            s_last = atomicAdd(ended, 1u) == gridDim.x - 1;
+            __threadfence();
+        }
+        __syncthreads();
+        if (s_last) chunk_prefix<TPB>(ccount, nchunks, pre, t2cnt);
+    }
     allow_dependents();
     if (STATS && ctr) count_inside(inside, ctr + 3);
 }
 
-// Prefix sums of the chunks' queue counts, by one block: pre[c] entries come
-// before chunk c's, pre[nchunks] in all.
-constexpr int CS_TPB = 1024, CS_ITEMS = 8;
+// The same by a launch of its own, and the tier 2 counters.
+constexpr int CS_TPB = 1024;
 __global__ void __launch_bounds__(CS_TPB) k_chunk_scan(const unsigned int* __restrict__ ccount, int nchunks,
-                                                      unsigned int* __restrict__ pre)
+                                                      unsigned int* __restrict__ pre, unsigned int* __restrict__ t2cnt)
 {
-    __shared__ unsigned int s_w[CS_TPB / 32];
     wait_for_predecessor();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned int before = 0;
-    for (int base = 0; base < nchunks; base += CS_TPB * CS_ITEMS) {
-        const int b0 = base + threadIdx.x * CS_ITEMS;
-        unsigned int c[CS_ITEMS], run = 0;
-#pragma unroll
-        for (int k = 0; k < CS_ITEMS; k++) {
-            c[k] = b0 + k < nchunks ? ccount[b0 + k] : 0u;
-            run += c[k];
-        }
-        unsigned int x = run;
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) s_w[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            const unsigned int v = s_w[lane];
-            unsigned int z = v;
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned int y = __shfl_up_sync(0xffffffffu, z, o);
-                if (lane >= o) z += y;
-            }
-            s_w[lane] = z;
-        }
-        __syncthreads();
-        unsigned int at = before + (warp ? s_w[warp - 1] : 0u) + x - run;
-#pragma unroll
-        for (int k = 0; k < CS_ITEMS; k++) {
-            if (b0 + k < nchunks) pre[b0 + k] = at;
-            at += c[k];
-        }
-        before += s_w[CS_TPB / 32 - 1];
-        __syncthreads();  // s_w is rewritten
-    }
-    if (threadIdx.x == 0) pre[nchunks] = before;
+    chunk_prefix<CS_TPB>(ccount, nchunks, pre, t2cnt);
     allow_dependents();
 }
 
@@ -1988,14 +2010,22 @@ PartQueue tier2_parts(long long points, unsigned int* cnt)
     return PartQueue{cnt, QUEUE_PARTS, (unsigned int)(points / 2 / QUEUE_PARTS + 1024)};
 }
 
+// A tier's blocks: what the chip holds, or a thread for each of `points`.
+int tier_grid(int resident, long long points, int tpb)
+{
+    return (int)std::min<long long>(resident, std::max(1LL, (points + tpb - 1) / tpb));
+}
+
 template <class VS>
-void tier2_launch(const VS& vs, const double2* ll, uint8_t* out, const Tiers& T, int precision,
+void tier2_launch(const VS& vs, const double2* ll, uint8_t* out, const Tiers& T, int precision, long long points,
                   unsigned long long* ctr, int sms, cudaStream_t s)
 {
     if (precision == GAHHG_QUERY_FP64_FILTER)
-        launch_dependent_tpb(k_leaf_t2<VS, true>, sms * T2_ALL_BLOCKS, T2_TPB, s, vs, ll, out, T, ctr);
+        launch_dependent_tpb(k_leaf_t2<VS, true>, tier_grid(sms * T2_ALL_BLOCKS, points, T2_TPB), T2_TPB, s, vs, ll, out,
+                             T, ctr);
     else
-        launch_dependent_tpb(k_leaf_t2<VS, false>, sms * T2_BLOCKS, T2_TPB, s, vs, ll, out, T, ctr);
+        launch_dependent_tpb(k_leaf_t2<VS, false>, tier_grid(sms * T2_BLOCKS, points, T2_TPB), T2_TPB, s, vs, ll, out, T,
+                             ctr);
 }
 
 }  // namespace
@@ -2196,7 +2226,7 @@ gahhg_status lattice_query(Grid* g, const double* d_lonlat, size_t n, uint8_t* d
             launch_dependent(k_leaf_t1s, sms * T1S_BLOCKS, s, Q, ll, out, T, ctr, polls);
         else if (!fp64)
             launch_dependent(k_leaf_t1<OneView>, sms * T1_BLOCKS, s, OneView{Q}, ll, out, T, ctr);
-        tier2_launch(OneView{Q}, ll, out, T, precision, ctr, sms, s);
+        tier2_launch(OneView{Q}, ll, out, T, precision, m, ctr, sms, s);
         if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) {
             set_error("query launch: %s", cudaGetErrorString(e));
             st = GAHHG_ERR_CUDA;
@@ -2289,22 +2319,22 @@ void batch_make_chunks(const long long* offsets, int nseg, int chunk_points, con
 template <int I>
 static void batch_locate_launch(int shape, int grid, cudaStream_t s, const QueryView* views, const BatchChunk* chunks,
                                 int nchunks, unsigned int* next_chunk, const double2* ll, uint8_t* out,
-                                uint32_t* queue, uint32_t* leafq, unsigned int* qcount, unsigned long long* ctr,
-                                int polls)
+                                uint32_t* queue, uint32_t* leafq, unsigned int* ccount, unsigned int* pre,
+                                unsigned int* t2cnt, unsigned int* ended, unsigned long long* ctr, int polls)
 {
     if constexpr (I < BATCH_NSHAPES) {
         if (shape != I) {
             batch_locate_launch<I + 1>(shape, grid, s, views, chunks, nchunks, next_chunk, ll, out, queue, leafq,
-                                       qcount, ctr, polls);
+                                       ccount, pre, t2cnt, ended, ctr, polls);
             return;
         }
         constexpr int U = BATCH_SHAPES[I].unroll, B = BATCH_SHAPES[I].blocks;
         if (ctr)
             k_batch_locate<true, U, B><<<grid, TPB, 0, s>>>(views, chunks, nchunks, next_chunk, ll, out, queue, leafq,
-                                                            qcount, ctr, polls);
+                                                            ccount, pre, t2cnt, ended, ctr, polls);
         else
             k_batch_locate<false, U, B><<<grid, TPB, 0, s>>>(views, chunks, nchunks, next_chunk, ll, out, queue,
-                                                             leafq, qcount, ctr, polls);
+                                                             leafq, ccount, pre, t2cnt, ended, ctr, polls);
     }
 }
 
@@ -2327,12 +2357,21 @@ size_t batch_queue_words(long long queue_cap, long long nchunks)
            2 * (size_t)nchunks + 1;
 }
 
-// counters: [1] next chunk, [2] overflow flag.  The queue holds
-// batch_queue_words(queue_cap, nchunks) words.  Everything is enqueued on `s` (no
+// At most this many chunk counts are scanned by the last block of pass 1, one
+// tile of its threads; more by a launch of their own with four times the
+// threads.  (us of a replay, last block | launch: 100 chunks 14.4 | 15.9, 512
+// 18.4 | 18.4, 2,000 28.3 | 28.2, 8,000 52.7 | 50.8.  With the launch alone, the
+// tiers at full grids and tier 2's counters cleared by a memset, batches of a
+// few hundred points took 16-18 us where they take 12-16.)
+constexpr int SCAN_FOLD = TPB * CS_ITEMS;
+
+// counters: [1] next chunk, [2] overflow flag, [3] blocks that ended.  The
+// queue holds batch_queue_words(queue_cap, nchunks) words; the chunks hold
+// `points` points, queue_cap at most.  Everything is enqueued on `s` (no
 // allocation, no host synchronisation), so it can be captured in a graph.
 gahhg_status batch_query_launch(const void* d_views, const void* d_chunks, int nchunks, const double* d_lonlat,
                                 uint8_t* d_labels, int precision, uint32_t* queue, long long queue_cap,
-                                unsigned int* counters, uint64_t* d_stats, cudaStream_t s, int device,
+                                long long points, unsigned int* counters, uint64_t* d_stats, cudaStream_t s, int device,
                                 bool zero_counters, int shape)
 {
     if (nchunks == 0) return GAHHG_OK;
@@ -2345,7 +2384,6 @@ gahhg_status batch_query_launch(const void* d_views, const void* d_chunks, int n
     Tiers T;
     T.p2 = tier2_parts(queue_cap, queue);
     const size_t cap2 = (size_t)T.p2.parts * T.p2.cap;
-    if (!fp64) GAHHG_CUDA_TRY(cudaMemsetAsync(T.p2.cnt, 0, sizeof(unsigned int) * QUEUE_PARTS * COUNTER_STRIDE, s));
     uint32_t* q1 = queue + QUEUE_PARTS * COUNTER_STRIDE;
     T.q1 = q1;
     T.over = counters + 2;
@@ -2359,13 +2397,15 @@ gahhg_status batch_query_launch(const void* d_views, const void* d_chunks, int n
     if (shape < 0 || shape >= BATCH_NSHAPES) shape = 0;
     const int grid = std::min(nchunks, sms * BATCH_SHAPES[shape].blocks);  // persistent: every block resident
     const double2* ll = (const double2*)d_lonlat;
+    unsigned int* pre = ccount + nchunks;
+    const bool fold = nchunks <= SCAN_FOLD;
     batch_locate_launch<0>(shape, grid, s, views, chunks, nchunks, counters + 1, ll, d_labels, q1, q1 + queue_cap, ccount,
-                           ctr, polls);
-    launch_dependent_tpb(k_chunk_scan, 1, CS_TPB, s, (const unsigned int*)ccount, nchunks, ccount + nchunks);
+                           fold ? pre : nullptr, T.p2.cnt, counters + 3, ctr, polls);
+    if (!fold) launch_dependent_tpb(k_chunk_scan, 1, CS_TPB, s, (const unsigned int*)ccount, nchunks, pre, T.p2.cnt);
     const ChunkViews vs{views, chunks, nchunks};
     if (!fp64)
-        launch_dependent(k_leaf_t1<ChunkViews>, sms * T1_BLOCKS, s, vs, ll, d_labels, T, ctr);
-    tier2_launch(vs, ll, d_labels, T, precision, ctr, sms, s);
+        launch_dependent(k_leaf_t1<ChunkViews>, tier_grid(sms * T1_BLOCKS, points, TPB), s, vs, ll, d_labels, T, ctr);
+    tier2_launch(vs, ll, d_labels, T, precision, points, ctr, sms, s);
     GAHHG_CUDA_TRY(cudaGetLastError());
     return GAHHG_OK;
 }

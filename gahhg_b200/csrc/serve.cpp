@@ -439,7 +439,7 @@ struct gahhg_server {
         // labels end where the header starts, so one copy brings both back
         uint8_t* d_labels = sl->d + lcap - (size_t)sl->points;
         GAHHG_TRY(batch_query_launch(d_views, din + HDR_BYTES, nchunks, (const double*)(din + pts_off), d_labels,
-                                     o.precision, sl->d_queue, o.slot_points, (unsigned int*)din,
+                                     o.precision, sl->d_queue, o.slot_points, sl->points, (unsigned int*)din,
                                      (uint64_t*)(din + 32), sl->s,
                                      o.device, false));
         GAHHG_CUDA_TRY(cudaMemcpyAsync(sl->h + lcap - (size_t)sl->points, d_labels, (size_t)sl->points + HDR_BYTES,
