@@ -2275,19 +2275,28 @@ gahhg_status lattice_staging_fallbacks(int device, unsigned long long* out)
     return GAHHG_OK;
 }
 
-// Chunks of at most `chunk_points` points, segment after segment.
-// A segment's chunks hold at least 2 points per word of its summary, so
-// staging the summary costs at most two bytes per point, from L2.  (16 points
-// per word made chunks of 65,536 points, fewer than the blocks of the grid:
-// the SMs stood idle 43 % of the pass, 150 us where 2 per word take 85; 1 and
-// 4 per word 87 and 91.)
+// Points of a chunk of a segment whose summary has `swords` words: what the
+// caller asked for, but 16 points per word at least as long as that makes
+// chunks of 4,096 points or less, and 2 per word in any case, so that staging
+// the summary costs at most two bytes per point, from L2.  (16 per word for
+// every summary made chunks of 65,536 points, fewer than the blocks of the grid:
+// the SMs stood idle 43 % of the pass, 150 us where 2 per word take 85; 1 and 4
+// per word 87 and 91.  2 per word for small summaries too made chunks of 256
+// points where a caller asks for that: 16.4M points in 16 polygons of 20 edges
+// 387 us, 152 with 16.)
+static long long chunk_step(int chunk_points, int swords)
+{
+    return std::max<long long>(chunk_points, std::max(2LL * swords, std::min(16LL * swords, 4096LL)));
+}
+
+// Chunks of a segment's step of points, segment after segment.
 void batch_write_chunks(const long long* offsets, int nseg, int chunk_points, const int* swords, const int* seg_view,
                         void* out, int* nchunks)
 {
     BatchChunk* v = (BatchChunk*)out;
     int n = 0;
     for (int p = 0; p < nseg; p++) {
-        const long long step = std::max<long long>(chunk_points, 2LL * (swords ? swords[p] : 0));
+        const long long step = chunk_step(chunk_points, swords ? swords[p] : 0);
         for (long long a = offsets[p]; a < offsets[p + 1]; a += step) {
             BatchChunk c;
             c.view = seg_view ? seg_view[p] : p;
