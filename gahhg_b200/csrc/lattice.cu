@@ -1279,15 +1279,11 @@ struct OneView {
     __device__ __forceinline__ void fetch(const Tiers& T, const Source& S, unsigned int t0, uint32_t& i, uint32_t& w,
                                           int&) const
     {
-        const unsigned int at = S.E.place(t0);
-        if (t0 + (threadIdx.x & 31) >= S.E.total) return;
-        if (S.ordered) {  // (an ordered queue has one part)
-            i = T.spts[at * T.sstride];
-            w = T.sleaf[at * T.sstride];
-        } else {
-            i = T.q1[at];
-            w = T.l1[at];
-        }
+        const unsigned int t = t0 + (threadIdx.x & 31);
+        const unsigned int at = S.ordered ? t * T.sstride : S.E.place(t0);
+        if (t >= S.E.total) return;
+        i = S.ordered ? T.spts[at] : T.q1[at];
+        w = S.ordered ? T.sleaf[at] : T.l1[at];
     }
 };
 
@@ -1473,13 +1469,13 @@ __global__ void __launch_bounds__(TPB, T1S_BLOCKS) k_leaf_t1s(const __grid_const
     }
     __syncthreads();
     wait_for_predecessor();
-    // (an ordered queue has one part: entries are at t * st)
-    const unsigned int m = *T.p1.cnt;
-    const bool ordered = *(const volatile unsigned int*)T.sorted == 1u;
-    const uint32_t* src = ordered ? T.spts : T.q1;
-    const uint32_t* src_leaf = ordered ? T.sleaf : T.l1;
-    const unsigned int st = ordered ? (unsigned int)T.sstride : 1u;
-    const bool sorted = src_leaf != T.l1;
+    PartEntries E;
+    E.begin(T.p1);
+    const unsigned int m = E.total;
+    const bool sorted = *(const volatile unsigned int*)T.sorted == 1u;
+    const uint32_t* src = sorted ? T.spts : T.q1;
+    const uint32_t* src_leaf = sorted ? T.sleaf : T.l1;
+    const unsigned int st = (unsigned int)T.sstride;  // (sorted: entries are at t * st)
     QueryCounts c;
     uint32_t phase = 0;  // parity of the barrier's current phase
     // Thread 0 works a tile ahead so that a tile's copy goes out as the tile
@@ -1553,9 +1549,11 @@ __global__ void __launch_bounds__(TPB, T1S_BLOCKS) k_leaf_t1s(const __grid_const
         bool defer = false;
         uint32_t i = 0, w = 0, mask = 0;
         PointCtx P{0.0, 0.0};
+        unsigned int at = t * st;
+        if (!sorted && (t & ~31u) < m) at = E.place(t & ~31u);
         if (t < m) {
-            i = src[t * st];
-            w = point_leaf(Q, ll[i], P, src_leaf[t * st]);
+            i = src[at];
+            w = point_leaf(Q, ll[i], P, src_leaf[at]);
         }
         __syncthreads();
         const int nl = s_nl;
@@ -1761,20 +1759,24 @@ __device__ __forceinline__ unsigned int smem_rank(unsigned int* cnt, int b)
     return base + __popc(same & ((1u << lane) - 1u));
 }
 
-__global__ void __launch_bounds__(P_TPB) k_part_count(const uint32_t* __restrict__ l1,
-                                                      const unsigned int* __restrict__ qcount, PartScratch S)
+__global__ void __launch_bounds__(P_TPB) k_part_count(const uint32_t* __restrict__ l1, PartQueue Q, PartScratch S)
 {
     __shared__ unsigned int s_cnt[PART_MAX];
     wait_for_predecessor();
-    const unsigned int m = *qcount;
+    PartEntries E;
+    E.begin(Q);
+    const unsigned int m = E.total, lane = threadIdx.x & 31;
     if (m < PART_MIN_QUEUE) {
         allow_dependents();
         return;
     }
     for (int k = threadIdx.x; k < S.np; k += P_TPB) s_cnt[k] = 0;
     __syncthreads();
-    for (unsigned int t = blockIdx.x * P_TPB + threadIdx.x; t < m; t += gridDim.x * P_TPB)
-        smem_rank(s_cnt, part_of(l1[t], S.np, S.scale));
+    for (unsigned int t0 = blockIdx.x * P_TPB + (threadIdx.x & ~31u); t0 < m; t0 += gridDim.x * P_TPB) {
+        const unsigned int at = E.place(t0);
+        if (t0 + lane < m) smem_rank(s_cnt, part_of(l1[at], S.np, S.scale));
+        __syncwarp();
+    }
     __syncthreads();
     allow_dependents();
     for (int k = threadIdx.x; k < S.np; k += P_TPB)
@@ -1782,12 +1784,13 @@ __global__ void __launch_bounds__(P_TPB) k_part_count(const uint32_t* __restrict
 }
 
 __global__ void __launch_bounds__(P_TPB) k_part_scatter(const uint32_t* __restrict__ queue,
-                                                        const uint32_t* __restrict__ l1,
-                                                        const unsigned int* __restrict__ qcount, PartScratch S)
+                                                        const uint32_t* __restrict__ l1, PartQueue Q, PartScratch S)
 {
     __shared__ unsigned int s_start[PART_MAX], s_cnt[PART_MAX], s_base[PART_MAX];
     wait_for_predecessor();
-    const unsigned int m = *qcount;
+    PartEntries E;
+    E.begin(Q);
+    const unsigned int m = E.total;
     if (m < PART_MIN_QUEUE) {
         allow_dependents();
         return;
@@ -1810,9 +1813,10 @@ __global__ void __launch_bounds__(P_TPB) k_part_scatter(const uint32_t* __restri
         int b[P_ITEMS];
 #pragma unroll
         for (int k = 0; k < P_ITEMS; k++) {
-            const unsigned int t = base + k * P_TPB + threadIdx.x;
-            q[k] = t < m ? queue[t] : 0u;
-            w[k] = t < m ? l1[t] : 0u;
+            const unsigned int t = base + k * P_TPB + threadIdx.x, t0 = t & ~31u;
+            const unsigned int at = t0 < m ? E.place(t0) : 0u;
+            q[k] = t < m ? queue[at] : 0u;
+            w[k] = t < m ? l1[at] : 0u;
             b[k] = part_of(w[k], S.np, S.scale);
         }
 #pragma unroll
@@ -1877,15 +1881,25 @@ __device__ __forceinline__ int leaf_bucket(uint32_t w, int nb)
     return (w & KIND_MASK) == KIND_LEAF ? (int)min(w & INDEX_MASK, (uint32_t)(nb - 1)) : nb - 1;
 }
 
-__global__ void __launch_bounds__(LS_TPB) k_ls_count(const uint32_t* __restrict__ l1,
-                                                     const unsigned int* __restrict__ qcount, LeafSortScratch S)
+__global__ void __launch_bounds__(LS_TPB) k_ls_count(const uint32_t* __restrict__ l1, PartQueue Q, LeafSortScratch S)
 {
     wait_for_predecessor();
-    const unsigned int m = *qcount;
+    PartEntries E;
+    E.begin(Q);
+    const unsigned int m = E.total;
     if (m >= PART_MIN_QUEUE)
-        for (unsigned int t = blockIdx.x * LS_TPB + threadIdx.x; t < m; t += gridDim.x * LS_TPB)
-            S.rank[t] = atomicAdd(S.cnt + leaf_bucket(l1[t], S.nb), 1u);
+        for (unsigned int t0 = blockIdx.x * LS_TPB + (threadIdx.x & ~31u); t0 < m; t0 += gridDim.x * LS_TPB) {
+            const unsigned int at = E.place(t0), t = t0 + (threadIdx.x & 31);
+            if (t < m) S.rank[t] = atomicAdd(S.cnt + leaf_bucket(l1[at], S.nb), 1u);
+        }
     allow_dependents();
+}
+
+__device__ __forceinline__ bool long_queue(const PartQueue& Q)
+{
+    PartEntries E;
+    E.begin(Q);
+    return E.total >= PART_MIN_QUEUE;
 }
 
 // Block-wide sum of one value per thread (every thread gets it).
@@ -1901,11 +1915,11 @@ __device__ __forceinline__ unsigned int ls_block_sum(unsigned int v, unsigned in
     return t;
 }
 
-__global__ void __launch_bounds__(LS_TPB) k_ls_tile_sums(const unsigned int* __restrict__ qcount, LeafSortScratch S)
+__global__ void __launch_bounds__(LS_TPB) k_ls_tile_sums(PartQueue Q, LeafSortScratch S)
 {
     __shared__ unsigned int s_w[LS_TPB / 32];
     wait_for_predecessor();
-    if (*qcount >= PART_MIN_QUEUE) {
+    if (long_queue(Q)) {
         for (int tile = blockIdx.x; tile < S.tiles; tile += gridDim.x) {
             unsigned int v = 0;
             const int b0 = tile * LS_TILE;
@@ -1918,12 +1932,12 @@ __global__ void __launch_bounds__(LS_TPB) k_ls_tile_sums(const unsigned int* __r
     allow_dependents();
 }
 
-__global__ void __launch_bounds__(LS_TPB) k_ls_scan(const unsigned int* __restrict__ qcount, LeafSortScratch S)
+__global__ void __launch_bounds__(LS_TPB) k_ls_scan(PartQueue Q, LeafSortScratch S)
 {
     __shared__ unsigned int s_w[LS_TPB / 32];
     __shared__ unsigned int s_wx[LS_TPB / 32];
     wait_for_predecessor();
-    if (*qcount >= PART_MIN_QUEUE) {
+    if (long_queue(Q)) {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         for (int tile = blockIdx.x; tile < S.tiles; tile += gridDim.x) {
             unsigned int before = 0;
@@ -1961,17 +1975,21 @@ __global__ void __launch_bounds__(LS_TPB) k_ls_scan(const unsigned int* __restri
 }
 
 __global__ void __launch_bounds__(LS_TPB) k_ls_scatter(const uint32_t* __restrict__ queue,
-                                                       const uint32_t* __restrict__ l1,
-                                                       const unsigned int* __restrict__ qcount, LeafSortScratch S)
+                                                       const uint32_t* __restrict__ l1, PartQueue Q, LeafSortScratch S)
 {
     wait_for_predecessor();
-    const unsigned int m = *qcount;
+    PartEntries E;
+    E.begin(Q);
+    const unsigned int m = E.total;
     if (m >= PART_MIN_QUEUE) {
-        for (unsigned int t = blockIdx.x * LS_TPB + threadIdx.x; t < m; t += gridDim.x * LS_TPB) {
-            const uint32_t w = l1[t];
-            const unsigned int at = S.start[leaf_bucket(w, S.nb)] + S.rank[t];
-            if (at < m) {  // counts and entries agree; never write past the queue
-                S.sent[at] = make_uint2(queue[t], w);
+        for (unsigned int t0 = blockIdx.x * LS_TPB + (threadIdx.x & ~31u); t0 < m; t0 += gridDim.x * LS_TPB) {
+            const unsigned int from = E.place(t0), t = t0 + (threadIdx.x & 31);
+            if (t < m) {
+                const uint32_t w = l1[from];
+                const unsigned int at = S.start[leaf_bucket(w, S.nb)] + S.rank[t];
+                if (at < m) {  // counts and entries agree; never write past the queue
+                    S.sent[at] = make_uint2(queue[from], w);
+                }
             }
         }
     }
@@ -2122,11 +2140,10 @@ gahhg_status lattice_query(Grid* g, const double* d_lonlat, size_t n, uint8_t* d
     }
     const long long ptiles = (chunk + TPB * LOC_UNROLL - 1) / (TPB * LOC_UNROLL);
     const int lgrid = (int)std::min<long long>(ptiles, sms * 8LL);
-    const int parts = ordered ? 1 : std::min(QUEUE_PARTS, lgrid);
+    const int parts = std::min(QUEUE_PARTS, lgrid);
     // room for the points of a part's blocks (the last chunk's grid is never larger)
-    const long long part_cap = ordered ? chunk
-                                       : (long long)((lgrid + parts - 1) / parts) * ((ptiles + lgrid - 1) / lgrid) *
-                                             (TPB * LOC_UNROLL);
+    const long long part_cap =
+        (long long)((lgrid + parts - 1) / parts) * ((ptiles + lgrid - 1) / lgrid) * (TPB * LOC_UNROLL);
     if (part_cap * parts > 0xFFFFFFFFll) {
         set_error("query queue of %lld places", part_cap * parts);
         return GAHHG_ERR_CAPACITY;
@@ -2197,9 +2214,8 @@ gahhg_status lattice_query(Grid* g, const double* d_lonlat, size_t n, uint8_t* d
                 W.sleaf = W.spts + chunk;
                 W.np = Q.nparts;
                 W.scale = Q.part_scale;
-                launch_dependent_tpb(k_part_count, sms * 4, P_TPB, s, (const uint32_t*)T.l1, (const unsigned int*)qc, W);
-                launch_dependent_tpb(k_part_scatter, sms * 4, P_TPB, s, (const uint32_t*)queue, (const uint32_t*)T.l1,
-                                     (const unsigned int*)qc, W);
+                launch_dependent_tpb(k_part_count, sms * 4, P_TPB, s, T.l1, T.p1, W);
+                launch_dependent_tpb(k_part_scatter, sms * 4, P_TPB, s, T.q1, T.l1, T.p1, W);
                 T.spts = W.spts;
                 T.sleaf = W.sleaf;
             } else {
@@ -2212,11 +2228,10 @@ gahhg_status lattice_query(Grid* g, const double* d_lonlat, size_t n, uint8_t* d
                 LS.rank = mem + lr;
                 LS.nb = nb;
                 LS.tiles = tiles;
-                const uint32_t* l1p = T.l1;
-                launch_dependent_tpb(k_ls_count, sms * 8, LS_TPB, s, l1p, (const unsigned int*)qc, LS);
-                launch_dependent_tpb(k_ls_tile_sums, std::min(tiles, sms * 8), LS_TPB, s, (const unsigned int*)qc, LS);
-                launch_dependent_tpb(k_ls_scan, std::min(tiles, sms * 8), LS_TPB, s, (const unsigned int*)qc, LS);
-                launch_dependent_tpb(k_ls_scatter, sms * 8, LS_TPB, s, (const uint32_t*)queue, l1p, (const unsigned int*)qc, LS);
+                launch_dependent_tpb(k_ls_count, sms * 8, LS_TPB, s, T.l1, T.p1, LS);
+                launch_dependent_tpb(k_ls_tile_sums, std::min(tiles, sms * 8), LS_TPB, s, T.p1, LS);
+                launch_dependent_tpb(k_ls_scan, std::min(tiles, sms * 8), LS_TPB, s, T.p1, LS);
+                launch_dependent_tpb(k_ls_scatter, sms * 8, LS_TPB, s, T.q1, T.l1, T.p1, LS);
                 T.spts = (const uint32_t*)LS.sent;
                 T.sleaf = T.spts + 1;
                 T.sstride = 2;
