@@ -141,13 +141,15 @@ __host__ __device__ inline NodeCap node_cap(const Geo& g, int lvl, long long ix,
 }
 
 // The cap's thresholds: squared chord of its radius r and the bound on the
-// sine of the distance from its center to a great circle that meets it.
+// sine of the distance from its center to a great circle that meets it.  (A
+// cell wider than a hemisphere has a cap that every great circle meets, and
+// none wider than the sphere.)
 __host__ __device__ inline double cap_chord2(double r)
 {
-    const double chord = 2.0 * sin(0.5 * r) * (1.0 + 1e-9) + 1e-12;
+    const double chord = r < 3.1 ? 2.0 * sin(0.5 * r) * (1.0 + 1e-9) + 1e-12 : 2.1;
     return chord * chord;
 }
-__host__ __device__ inline double cap_sin_bound(double r) { return sin(r) * (1.0 + 1e-9) + 1e-12; }
+__host__ __device__ inline double cap_sin_bound(double r) { return r < 1.5 ? sin(r) * (1.0 + 1e-9) + 1e-12 : 2.0; }
 
 // edge_hits_cap with the cap's thresholds and the edge's normal N = A x B,
 // nn = |N|, computed once by the caller.
