@@ -162,9 +162,10 @@ __global__ void k_ring_edges(const D3* __restrict__ pv, const long long* __restr
 // ----------------------------------------------------------------- domain --
 //
 // Longitude/latitude domain of a polygon's edges: per edge its latitude range
-// and the 0.1-degree longitude bins it touches (long edges by their
-// great-circle box, short ones by their ends' latitude and longitude, padded
-// by 1e-4 degrees).  Min, max and OR do not depend on the order of the edges.
+// and the 0.1-degree longitude bins it touches (edges whose great circle rises
+// above their ends by their great-circle box, the others by their ends'
+// latitude and longitude, padded by 1e-4 degrees).  Min, max and OR do not
+// depend on the order of the edges.
 constexpr int DOMAIN_BIN_WORDS = (3600 + 31) / 32;
 struct DomainOut {
     unsigned long long latmin, latmax;  // order-preserving keys of the doubles
@@ -221,10 +222,12 @@ __global__ void __launch_bounds__(TPB) k_domain_scan(const double2* __restrict__
                     double la0, la1, lo0, lo1;
                     bool fl = false;
                     const double dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
-                    if (dx * dx + dy * dy + dz * dz > 1e-4) {
-                        arc_box(a, b, la0, la1, lo0, lo1, fl);  // long edge: its great circle may bulge
+                    const double sy = fmax(fabs(a.y), fabs(b.y));
+                    // its great circle passes the higher end by c^2 / 8 tan(lat)
+                    if ((dx * dx + dy * dy + dz * dz) * sy > 8e-6 * sqrt(fmax(1.0 - sy * sy, 0.0))) {
+                        arc_box(a, b, la0, la1, lo0, lo1, fl);
                     } else {
-                        // short edge: its ends (the bulge is below 1e-4 deg, far inside the one-cell padding)
+                        // ... by less than 1e-6 rad: its ends and 1e-4 deg
                         const double ta = lat_of(a), tb = lat_of(b);
                         double oa = lon_of(a), ob = lon_of(b);
                         la0 = fmin(ta, tb) - 1e-4;
