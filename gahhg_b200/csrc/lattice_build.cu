@@ -19,7 +19,8 @@
 // Every step runs once for all polygons of the build (concatenated edges and
 // nodes, a polygon table for the per-polygon geometry), so launches and host
 // round trips scale with levels, not with polygons: two round trips before
-// the levels, one per level and one at the end.  A polygon's index does not
+// the levels, one per level and one at the end (and one for every 64 edges tried
+// where a polygon's first edges give no reference point).  A polygon's index does not
 // depend on what it was built with, up to numbering (node words hold child
 // indices relative to the polygon's first top node; leaves, records and edge
 // ids count over the whole set).
@@ -29,7 +30,8 @@
 // neighbour parities 2336, list sorts 1709, leaf records 1048, 21 scans 738,
 // level-0 labels 404.  With the lists and the labels' crossings taken in the
 // cells' projection planes, children's lists filtered in order and one scan
-// per level, the whole build is 2.8 ms where it was 17-19.
+// per level, the whole build is 1.7 ms of kernels in 2.1 ms where it was 14 in
+// 17-19.
 #include <cfloat>
 #include <climits>
 #include <cstdio>
@@ -1708,7 +1710,7 @@ __global__ void __launch_bounds__(TPB) k_leaf_records(const double2* __restrict_
         L.sb = (float)sb;
         L.cb = (float)cb;
     }
-    if (n > 65535) atomicAdd(bad + 2, 1);
+    if (n > 65535) atomicAdd(bad + 1, 1);
     local_frame::Basis fb;
     local_frame::basis_at(c.lonc, c.latc, fb);
     LeafAux X;
@@ -1979,7 +1981,7 @@ struct BuildWords {
         int open;  // polygons without the label of their first center
     } sums;
     int pick;
-    int bad[4];      // [0] coincidences, [1] unused, [2] long lists
+    int bad[2];      // [0] coincidences, [1] leaves of more than 65,535 edges
     int sort[4];     // middling lists, next, long lists, next
     DeviceErrors err;
 };
@@ -2036,14 +2038,11 @@ struct Builder {
         GAHHG_CUDA_TRY(cudaMemcpyAsync(&h, &w->sums, sizeof h, cudaMemcpyDeviceToHost, s));
         GAHHG_CUDA_TRY(cudaStreamSynchronize(s));
         b.sums = h.level;
-        const unsigned long long pairs = lvl ? (unsigned long long)h.level.pairs : h.l0.pairs;
-        if (pairs > (unsigned long long)INT_MAX) {
-            set_error("%s%llu list entries on level %d exceed 2^31 (fewer top cells are needed)", prefix.c_str(), pairs,
-                      lvl);
-            return GAHHG_ERR_CAPACITY;
-        }
+        if (lvl == 0) b.sums.pairs = (long long)h.l0.pairs;
         return GAHHG_OK;
     }
+    // A level's entries have 32-bit places, and below the top the budget.
+    bool too_long(int lvl) const { return lv[lvl].sums.pairs > (lvl ? PAIR_BUDGET : (long long)INT_MAX); }
 
     // ... under the budgets (`nodes`: in all, this level's included).  Bounded
     // refinement: a polygon whose edges fill an area densely (not a curve)
@@ -2054,7 +2053,8 @@ struct Builder {
     {
         GAHHG_TRY(scan_once(lvl, lvl >= MAX_LEVEL));
         const LevelSums& c = lv[lvl].sums;
-        if (c.refined > 0 && (nodes + (long long)c.refined * FAN * FAN > NODE_BUDGET || 4 * c.pairs > PAIR_BUDGET))
+        if (!too_long(lvl) && c.refined > 0 &&
+            (nodes + (long long)c.refined * FAN * FAN > NODE_BUDGET || 4 * c.pairs > PAIR_BUDGET))
             return scan_once(lvl, true);
         return GAHHG_OK;
     }
@@ -2070,8 +2070,8 @@ struct Builder {
 // The edges of a set whose vertices are on the host: one copy for all
 // polygons, gathered by the copy team into its page-locked slots or, small
 // sets, into one array.  (Two copies from pageable memory for each of 82
-// polygons of 1.1M edges in all took 4.6 ms of a build of 6.6, which takes 3.8
-// now.)
+// polygons of 1.1M edges in all took 4.6 ms of a build of 6.6; without them 3.8
+// there.)
 gahhg_status Builder::set_edges(Polygon* const* polys, const std::vector<long long>& ebase, const long long* d_ebase,
                                 long long ne, int device)
 {
@@ -2327,6 +2327,11 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
     }
     phase("l0 count");
     GAHHG_TRY(scan(0, n0));
+    if (too_long(0)) {
+        set_error("%s%lld list entries on level 0 exceed 2^31 (fewer top cells are needed)", prefix.c_str(),
+                  lv[0].sums.pairs);
+        return GAHHG_ERR_CAPACITY;
+    }
     {
         LevelBuf& l0 = lv[0];
         DevArray<int> cursor, mid, longs;
@@ -2400,6 +2405,27 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
     long long gnext = n0, leaf_total = 0, rec_total = 0;
     std::vector<int> leaf_base;
     std::vector<long long> rec_base;
+    // node words, refined nodes and leaves of a level whose labels are known
+    auto encode = [&](int lvl) -> gahhg_status {
+        LevelBuf& b = lv[lvl];
+        leaf_base.push_back((int)leaf_total);
+        rec_base.push_back(rec_total);
+        leaf_total += b.sums.leaves;
+        rec_total += b.sums.recs;
+        if (dbg)
+            fprintf(stderr, "lattice level %d: %d cells, %lld edge entries, %d split, %d leaves of %lld entries\n",
+                    lvl, b.nn, b.sums.pairs, b.sums.refined, b.sums.leaves, b.sums.recs);
+        if (rec_total >= 0xFFFFFFFFll || leaf_total >= (long long)INDEX_MASK) {
+            set_error("%stoo many leaves or edge records", prefix.c_str());
+            return GAHHG_ERR_CAPACITY;
+        }
+        GAHHG_TRY(b.words.alloc(b.nn, s));
+        GAHHG_TRY(b.rnode.alloc(b.sums.refined, s));
+        GAHHG_TRY(b.lnode.alloc(b.sums.leaves, s));
+        k_encode<<<blocks_for(b.nn), TPB, 0, s>>>(view(lvl), d_pg.ptr, (int)gnext, leaf_base[lvl], b.words.ptr,
+                                                  b.rnode.ptr, b.lnode.ptr);
+        return GAHHG_OK;
+    };
     for (int lvl = 0;; lvl++) {
         LevelBuf& b = lv[lvl];
         if (lvl > 0) {
@@ -2415,24 +2441,8 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
             k_child_exact<<<blocks_for(b.nn), TPB, 0, s>>>(ends, uv, d_pg.ptr, up.rnode.ptr, b.nn, b.ixy.ptr, b.cnt.ptr,
                                                            b.off.ptr, b.list.ptr, b.cpar.ptr, b.label.ptr, bad);
         }
+        GAHHG_TRY(encode(lvl));
         const int nref = b.sums.refined;
-        leaf_base.push_back((int)leaf_total);
-        rec_base.push_back(rec_total);
-        leaf_total += b.sums.leaves;
-        rec_total += b.sums.recs;
-        if (dbg)
-            fprintf(stderr, "lattice level %d: %d cells, %lld edge entries, %d split, %d leaves of %lld entries\n",
-                    lvl, b.nn, b.sums.pairs, nref, b.sums.leaves, b.sums.recs);
-        if (rec_total >= 0xFFFFFFFFll || leaf_total >= (long long)INDEX_MASK) {
-            set_error("%stoo many leaves or edge records", prefix.c_str());
-            return GAHHG_ERR_CAPACITY;
-        }
-        GAHHG_TRY(b.words.alloc(b.nn, s));
-        GAHHG_TRY(b.rnode.alloc(nref, s));
-        GAHHG_TRY(b.lnode.alloc(b.sums.leaves, s));
-        const LevelView v = view(lvl);
-        k_encode<<<blocks_for(b.nn), TPB, 0, s>>>(v, d_pg.ptr, (int)gnext, leaf_base[lvl], b.words.ptr, b.rnode.ptr,
-                                                  b.lnode.ptr);
         if (nref == 0) break;
         // the children: rectangles, pair tests, counts
         lv.emplace_back();
@@ -2450,10 +2460,24 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
         GAHHG_CUDA_TRY(cudaMemsetAsync(w->sort, 0, sizeof w->sort, s));
         const PairArgs a{ends, d_pg.ptr, b.rnode.ptr, nref, c.ixy.ptr, c.poly.ptr, b.hit.ptr, c.cnt.ptr,
                          c.cpar.ptr, longs.ptr, w->sort};
-        k_child_pairs<<<(c.nn + PAIR_TPB - 1) / PAIR_TPB, PAIR_TPB, 0, s>>>(a, v);
-        k_child_pairs_long<<<sms * 2, TPB, 0, s>>>(a, v);
+        k_child_pairs<<<(c.nn + PAIR_TPB - 1) / PAIR_TPB, PAIR_TPB, 0, s>>>(a, view(lvl));
+        k_child_pairs_long<<<sms * 2, TPB, 0, s>>>(a, view(lvl));
         GAHHG_CUDA_TRY(cudaGetLastError());
         GAHHG_TRY(scan(lvl + 1, gnext));
+        if (too_long(lvl + 1)) {
+            // edges closer to one another than the cells' margin: every child
+            // lists nearly all of them, however small (8 entries and more for
+            // one).  This level's cells stay leaves, as past the budgets.
+            gnext -= c.nn;
+            lv.pop_back();
+            leaf_total = leaf_base.back();
+            rec_total = rec_base.back();
+            leaf_base.pop_back();
+            rec_base.pop_back();
+            GAHHG_TRY(scan_once(lvl, true));
+            GAHHG_TRY(encode(lvl));
+            break;
+        }
     }
     const int nlev = (int)lv.size();
     L->nnodes = gnext;
@@ -2524,9 +2548,9 @@ gahhg_status Builder::run(Grid* g, Polygon* const* polys, int count, const int* 
     // a scan whose look-back ran out of time summed the late tile's counts
     // itself: its result is exact, the event is only counted
     g->stats.scan_fallbacks = hw.err.scan_lookback_timeout;
-    if (hw.bad[0] || hw.bad[2]) {
+    if (hw.bad[0] || hw.bad[1]) {
         set_error("%s%d center/vertex coincidences, %d oversize leaves",
-                  prefix.empty() ? "exact index: " : prefix.c_str(), hw.bad[0], hw.bad[2]);
+                  prefix.empty() ? "exact index: " : prefix.c_str(), hw.bad[0], hw.bad[1]);
         return GAHHG_ERR_DEVICE;
     }
     // ---- every polygon's query view
