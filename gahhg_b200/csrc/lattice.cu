@@ -13,10 +13,11 @@
 //   - in a leaf counts crossings of arc(R, q) with the leaf's edges:
 //       s2 = orient(A,B,q) = q.(A x B), s3 = orient(R,q,A) = q.(A x R),
 //       s4 = orient(R,q,B) = q.(B x R), s1 = orient(A,B,R) stored exactly;
-//     each sign is first taken in FP32 (q from __sincosf, vectors rounded to
-//     FP32) against a forward error bound, then in FP64 on the canonical q,
-//     then exactly (exact_pred.cuh).  Labels are therefore those of the exact
-//     oracle; the FP32 stage only decides when its bound proves the sign.
+//     each sign is first taken in FP32 (in the leaf's tangent frame, from the
+//     angle differences to R: local_frame.cuh) against a forward error bound,
+//     then in FP64 on the canonical q, then exactly (exact_pred.cuh).  Labels
+//     are therefore those of the exact oracle; the FP32 stage only decides when
+//     its bound proves the sign.
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -116,8 +117,9 @@ __device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontro
 // mbarrier in bytes; no multicast) issued by one thread, instead of a load
 // per word by every thread.  Both addresses are 16-byte aligned (pool
 // allocations are 256-byte aligned, the shared arrays are declared so) and
-// the size is rounded up to 16 bytes (the summary's allocation holds at least
-// 1,024 words).  Every wait is bounded; a wait that runs out is counted in
+// the size is rounded up to 16 bytes (in the index every summary starts at a
+// multiple of four words and the last one is padded to one, so the copy reads
+// no further).  Every wait is bounded; a wait that runs out is counted in
 // g_tma_timeouts and the block falls back to loading the summary itself into
 // memory no pending copy can write (see the kernels), so labels never depend
 // on a copy completing.
@@ -1442,12 +1444,13 @@ __global__ void __launch_bounds__(TPB, T1_BLOCKS) k_leaf_t1(const __grid_constan
 // global memory, so the late copy is never read), is counted once in
 // g_tma_timeouts, and before exiting the block waits (bounded again) for
 // that copy.  Both slices start on 16-byte boundaries (pool allocations are
-// 256-byte aligned; leaf records are 32 bytes, edge records 16) and their
-// sizes are multiples of 16 bytes.  Measured on 2e7 C2 points (9.1M queued):
-// 337 us against 283 us for k_leaf_t1 on the same leaf-ordered queue, whose
-// per-warp gathers leaf order already makes one request per warp and leaf;
-// the staging adds a block barrier and a wait per tile and copies every
-// leaf of the tile's range.  It is therefore an option (pass-2 order 3).
+// 256-byte aligned; leaf records are 64 bytes, edge records 16) and their
+// sizes are multiples of 16 bytes.  2e7 points, half of them near the
+// 1.1M-edge polygon's edges: 946 us a query, 896 with k_leaf_t1 on the same
+// leaf-ordered queue, whose per-warp gathers leaf order already makes one
+// request per warp and leaf; the staging adds a block barrier and a wait per
+// tile and copies every leaf of the tile's range.  It is therefore an option
+// (pass-2 order 3).
 constexpr int T1S_LEAVES = 256;  // 16 KB of leaf records per tile
 constexpr int T1S_RECS = 1024;   // 16 KB of edge records per tile
 constexpr int T1S_BLOCKS = 5;
@@ -1708,8 +1711,8 @@ __global__ void __launch_bounds__(T2_TPB, ALL ? T2_ALL_BLOCKS : T2_BLOCKS) k_lea
 //
 // Pass 1 queues points in input order, so on inputs without spatial order
 // (C2's near-edge points) the tiers' gathers of leaf and edge records sweep
-// the whole index, which is larger than L2 (350-400 MB on the C1 polygon):
-// nearly every record comes from DRAM, once per point.  Leaves are numbered
+// the whole index, which is larger than L2 (198 MB on the C1 polygon): over
+// half of the records come from DRAM.  Leaves are numbered
 // so that their records are contiguous, so a window of consecutive leaves is
 // a contiguous slice of the index.  Two launches put the queue in window
 // order (a counting sort with a few dozen bins, block-aggregated):
@@ -1721,8 +1724,10 @@ __global__ void __launch_bounds__(T2_TPB, ALL ? T2_ALL_BLOCKS : T2_BLOCKS) k_lea
 // The tiers' grid-stride loops then sweep the queue in order, so at any time
 // the grid works in one or two windows whose records stay in L2, and tier 1
 // writes the tier-2 queue in the same order.  Windows are sized at about
-// PART_BYTES of index; queues below PART_MIN_QUEUE entries keep pass-1 order
-// (both kernels return at once and the tiers read the pass-1 queue).
+// PART_BYTES of leaf and edge records; queues below PART_MIN_QUEUE entries
+// keep pass-1 order (both kernels return at once and the tiers read the pass-1
+// queue).  2e7 points, half of them near the 1.1M-edge polygon's edges, FP32
+// filter: 822 us where pass-1 order takes 666, leaf order (below) 896.
 constexpr int PART_MAX = 64;
 constexpr long long PART_BYTES = 24LL << 20;
 constexpr unsigned int PART_MIN_QUEUE = 1u << 18;
@@ -2052,7 +2057,9 @@ void tier2_launch(const VS& vs, const double2* ll, uint8_t* out, const Tiers& T,
 
 static const QueryView& make_view(const Grid* g) { return g->lattice->views[0]; }
 
-// Windows of about PART_BYTES of the records the tiers gather per leaf.
+// Windows of about PART_BYTES of the records the tiers gather per leaf, three
+// doubles of a leaf's aux line counted (the whole line: more windows, 855 us
+// where 825 were taken by 2e7 points near the 1.1M-edge polygon).
 void set_leaf_windows(QueryView& Q, long long nleaves, long long nrecs)
 {
     const long long tier_bytes = nrecs * (long long)(sizeof(float4) + sizeof(uint32_t)) +
@@ -2065,14 +2072,18 @@ void set_leaf_windows(QueryView& Q, long long nleaves, long long nrecs)
 // Points per pass.
 constexpr long long QUERY_CHUNK = 1LL << 27;
 // Queries of at most this many points run as one launch with every tier
-// inline (k_query).  us a call, one launch | passes of their own:
-//   points      uniform      near the edges   (1.1M-edge polygon, FP32 filter)
-//     32,000     7 | 19         13 | 27
-//    131,072     9 | 19         23 | 31
-//    524,288    11 | 19         58 | 59
-//  1,048,576    14 | 20        102 | 89
-//  2,097,152    19 | 23        178 | 157
-// The line is where the two gains are about equal.
+// inline (k_query).  us a call, one launch | passes of their own (FP32 filter;
+// uniform points, and half of them near an edge in random order):
+//              1.1M-edge polygon      100,000 edges          1,100 edges
+//   points     uniform     near      uniform     near      uniform     near
+//     32,000    6 | 16    10 | 23     6 | 16    10 | 23     6 | 15     9 | 22
+//    131,072    8 | 20    16 | 27     8 | 18    17 | 27     8 | 16    27 | 35
+//    524,288   10 | 18    35 | 41    10 | 18    32 | 36    12 | 20    43 | 47
+//    786,432   10 | 18    49 | 52    11 | 18    41 | 44    14 | 21    58 | 53
+//  1,048,576   12 | 20    61 | 59    12 | 19    51 | 51    16 | 21    64 | 66
+//  2,097,152   18 | 22   102 | 96    18 | 21    85 | 83    21 | 25   103 | 105
+// The line is where the near-edge points take the same either way; uniform
+// ones gain by one launch up to there and beyond.
 constexpr long long INLINE_MAX = 1LL << 20;
 // ... and of at most this many with a point per lane and the summary read in
 // place: less than a block per SM, so the query's time is one point's latency
