@@ -489,7 +489,8 @@ def run_c4(args, polys=None, seconds=None, pool_n=None, tune_budget=None):
                            "build_p99": round(float(np.percentile(build_lag, 99)) * 1e3, 4) if build_lag else None},
         "escalation": {"boundary_points": st["boundary_points"], "fp64_tests": st["esc_fp64"],
                        "exact_tests": st["esc_exact"]},
-        "gpu_launches": 4 * int(st["batches"]), "clocks": clk,
+        # per batch: pass 1 (which scans up to 2,048 chunk counts itself) and the two tiers
+        "gpu_launches": 3 * int(st["batches"]), "clocks": clk,
         "build_ms": {"resident_set_wall": round(resident_build_s * 1e3, 1), "resident_bytes": resident,
                      "generate_s": round(gen_s, 1), "autotune_s": round(tune_s, 1)},
         "tuning": tuning.as_dict(),
