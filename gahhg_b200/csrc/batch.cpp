@@ -468,13 +468,8 @@ gahhg_status gahhg_batch_query_graph(gahhg_batch* b, const double* d_lonlat, con
     }
     b->unwaited.store(true, std::memory_order_relaxed);
     GAHHG_CUDA_TRY(cudaGraphLaunch(b->exec, s));
-    // (a replay that becomes part of the caller's own graph runs when that does)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    GAHHG_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
-    if (cap == cudaStreamCaptureStatusNone) {
-        GAHHG_CUDA_TRY(cudaEventRecord(b->replayed, s));
-        b->replays = true;
-    }
+    GAHHG_CUDA_TRY(cudaEventRecord(b->replayed, s));
+    b->replays = true;
     return GAHHG_OK;
 }
 
